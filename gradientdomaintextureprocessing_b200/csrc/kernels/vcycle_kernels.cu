@@ -735,41 +735,171 @@ __device__ __forceinline__ void prefetch_l2_block(const void* p, long long bytes
 }
 
 // ----------------------------------------------------------------------------
-// Coarsest level: x = D Ainv^ D rhs with the scaled dense inverse (FP64).
+// Coarsest level: x = D Ainv^ D rhs with the scaled dense inverse (FP64): a
+// stream of the n x n inverse.  A block takes 2 R rows, a warp one part of the
+// j range (coarse_part's partition and order, so the same bits) of R rows and Q
+// channel groups: a value of the inverse is used for Q W channels, and a
+// right-hand side value, widened to FP64 once, for R rows.  What bounds it is
+// the loads in flight: a lane loads U of its j at once, before their updates.
 // ----------------------------------------------------------------------------
-template <typename T, int W>
-__global__ void __launch_bounds__(256) k_coarse_solve(int n, const double* __restrict__ ainv, const double* __restrict__ scale,
-                                                      const T* __restrict__ rhs, T* __restrict__ x, int KP, int G) {
-  // this block's two rows of the inverse (set-up data) start moving into L2
-  // while the previous launch finishes
-  {
-    const int r0 = blockIdx.x * 2;
-    if (r0 < n) prefetch_l2_block(ainv + (long long)r0 * n, (long long)min(2, n - r0) * n * sizeof(double));
-  }
+template <typename T, int W, int R, int Q, int U>
+__global__ void __launch_bounds__(256, Q == 1 ? 2 : 1) k_coarse_solve(int n, const double* __restrict__ ainv, const double* __restrict__ scale,
+                                                      const T* __restrict__ rhs, T* __restrict__ x, int KP) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rl = warp / kCoarseParts, p = warp % kCoarseParts;
+  const int b0 = blockIdx.x * 2 * R, row0 = b0 + rl * R;
+  // this block's rows of the inverse (set-up data) start moving into L2 while
+  // the previous launch finishes
+  if (b0 < n && blockIdx.y == 0) prefetch_l2_block(ainv + (long long)b0 * n, (long long)min(2 * R, n - b0) * n * sizeof(double));
   grid_dependency_wait();
   grid_launch_dependents();
-  // 2 rows per block, a warp per part of a row, parts added in order
-  __shared__ double part[2][kCoarseParts][4 * W];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rl = warp / kCoarseParts, p = warp % kCoarseParts, row = blockIdx.x * 2 + rl;
-  for (int q = 0; q < G; q++) {
-    const int off = q * W;
-    double acc[W];
-    if (row < n) coarse_part<T, W, LoadDefault>(n, ainv, scale, rhs, KP, off, row, p, lane, acc);
-    if (row < n && lane == 0)
+  __shared__ double part[2][R][kCoarseParts][Q * W];
+  const int c0 = blockIdx.y * Q * W;
+  const int len = ((n + kCoarseParts - 1) / kCoarseParts + 31) & ~31;
+  const int j0 = p * len, j1 = min(n, j0 + len);
+  double acc[R][Q * W];
 #pragma unroll
-      for (int c = 0; c < W; c++) part[rl][p][c] = acc[c];
-    __syncthreads();
-    if (threadIdx.x < 2 * W) {
-      const int r2 = threadIdx.x / W, c = threadIdx.x % W, rr = blockIdx.x * 2 + r2;
-      if (rr < n) {
-        double sum = 0;
-        for (int pp = 0; pp < kCoarseParts; pp++) sum += part[r2][pp][c];
-        x[(long long)rr * KP + off + c] = T(sum * scale[rr]);
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int c = 0; c < Q * W; c++) acc[r][c] = 0;
+  const double* arow[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) arow[r] = ainv + (long long)min(row0 + r, n - 1) * n;  // rows past n: computed, not stored
+  for (int j = j0 + lane; j < j1; j += 32 * U) {
+    double w[U][R], sc[U];
+    Vec<T, W> v[U][Q];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int ju = j + 32 * u;
+      if (ju < j1) {
+#pragma unroll
+        for (int r = 0; r < R; r++) w[u][r] = __ldg(arow[r] + ju);
+        sc[u] = scale[ju];
+#pragma unroll
+        for (int q = 0; q < Q; q++) v[u][q] = vload<T, W>(rhs + (long long)ju * KP + c0 + q * W);
       }
     }
-    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (j + 32 * u < j1) {
+#pragma unroll
+        for (int r = 0; r < R; r++) w[u][r] = w[u][r] * sc[u];
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+#pragma unroll
+          for (int c = 0; c < W; c++) {
+            const double d = double(v[u][q].v[c]);
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r][q * W + c] += w[u][r] * d;
+          }
+      }
   }
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int c = 0; c < Q * W; c++) {
+      double v = acc[r][c];
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
+      if (lane == 0) part[rl][r][p][c] = v;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * R * Q * W; i += blockDim.x) {
+    const int rr = i / (Q * W), c = i % (Q * W), row = b0 + rr;
+    if (row >= n) continue;
+    double sum = 0;
+    for (int pp = 0; pp < kCoarseParts; pp++) sum += part[rr / R][rr % R][pp][c];
+    x[(long long)row * KP + c0 + c] = T(sum * scale[row]);
+  }
+}
+
+// ----------------------------------------------------------------------------
+// Reduction of the per-block partial sums, in a fixed order: sum c is the sum
+// over a tree of 256 thread sums (thread t takes blocks t, t + 256, ...; the
+// tree adds t and t + 128, + 64, ... + 1).  Up to kSumWide sums are reduced side
+// by side, a block per kSumWide sums.
+// It is a chain of latencies over 1184 x 2K doubles, so the loads of a thread
+// are issued together, and what used to follow as launches of their own is done
+// here: the sums' copy for the host and the flexible-CG scalar.  One block for
+// all 2K sums took 57 us at K = 15 and 230 us at K = 64, the blocks here 12 us at
+// K = 64.  Reducing in the last block of the kernel that writes the partials
+// was measured slower (its fences and arrivals: the operator 77 -> 97 us at
+// 2048^2, against 7 us for this launch).
+// ----------------------------------------------------------------------------
+constexpr int kSumWide = 8;
+constexpr int kSumThreads = 256;
+
+// sums [c0, c0 + count) of 2K by a block of kSumThreads threads, into total[]
+// (shared) and `sums` / `host` (optional, mapped host memory)
+__device__ __forceinline__ void reduce_partials(const double* __restrict__ partials, int nBlocks, int K, int c0, int count, double* sums,
+                                                double* host, double (*sh)[kSumThreads], double* total) {
+  double s[kSumWide];
+#pragma unroll
+  for (int c = 0; c < kSumWide; c++) s[c] = 0;
+  constexpr int kAhead = 4;
+  for (int b = threadIdx.x; b < nBlocks; b += kAhead * kSumThreads) {
+    double v[kAhead][kSumWide];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+#pragma unroll
+      for (int c = 0; c < kSumWide; c++)
+        if (b + u * kSumThreads < nBlocks && c < count) v[u][c] = partials[(long long)(b + u * kSumThreads) * 2 * K + c0 + c];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+#pragma unroll
+      for (int c = 0; c < kSumWide; c++)
+        if (b + u * kSumThreads < nBlocks && c < count) s[c] += v[u][c];
+  }
+  // four sums at a time: 256 thread sums -> 32 in shared memory (+128, +64, +32),
+  // then one warp's shuffles (+16 ... +1)
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 0; h < kSumWide; h += 4) {
+    if (h >= count) break;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; c++) sh[c][threadIdx.x] = s[h + c];
+    __syncthreads();
+    if (w < 4) {
+      const double* a = sh[w];
+      double v = ((a[l] + a[l + 128]) + (a[l + 64] + a[l + 192])) + ((a[l + 32] + a[l + 160]) + (a[l + 96] + a[l + 224]));
+#pragma unroll
+      for (int d = 16; d >= 1; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+      if (l == 0 && h + w < count) {
+        total[h + w] = v;
+        sums[c0 + h + w] = v;
+        if (host) host[c0 + h + w] = v;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// beta = -alpha_old (z . q_old) / rho_old (0 on a (re)start, rho_old = 0); rho = z . r
+__device__ __forceinline__ void fcg_beta(int K, int c, double rho, double gamma, double* sc) {
+  const double rhoOld = sc[3 * K + c];
+  sc[K + c] = rhoOld != 0.0 ? -sc[c] * gamma / rhoOld : 0.0;
+  sc[2 * K + c] = rho;
+  sc[3 * K + c] = rho;
+}
+// alpha = rho / (p . A p), 0 for frozen right-hand sides
+__device__ __forceinline__ void fcg_alpha(int K, int c, double pq, const int* frozen, double* sc) {
+  sc[c] = (frozen && frozen[c]) || !(pq > 0) ? 0.0 : sc[2 * K + c] / pq;
+}
+
+// scalar: 1 beta and rho, 2 alpha (K <= kSumWide / 2: one block holds every sum)
+__global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* __restrict__ partials, int nBlocks, int K,
+                                                             double* __restrict__ sums, double* __restrict__ host, int scalar,
+                                                             double* __restrict__ sc, const int* __restrict__ frozen) {
+  grid_dependency_wait();
+  grid_launch_dependents();
+  __shared__ double sh[4][kSumThreads];
+  __shared__ double total[kSumWide];
+  const int c0 = blockIdx.x * kSumWide;
+  reduce_partials(partials, nBlocks, K, c0, min(kSumWide, 2 * K - c0), sums, host, sh, total);
+  const int c = threadIdx.x;
+  if (scalar == 1 && c < K) fcg_beta(K, c, total[c], total[K + c], sc);
+  if (scalar == 2 && c < K) fcg_alpha(K, c, total[c], frozen, sc);
 }
 
 // Per-block sums of two per-channel accumulators into partials[block][0..K) and
@@ -812,7 +942,7 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
                                                       const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
                                                       const double* __restrict__ b, const double* __restrict__ x,
                                                       double* __restrict__ out, int K, int G, int mode, double* __restrict__ partials,
-                                                      float* __restrict__ out32 = nullptr, int KP = 0) {
+                                                      float* __restrict__ out32, int KP) {
   grid_dependency_wait();
   grid_launch_dependents();
   // grid-stride over deep items (runs x 32 x G) then boundary items (rows x G);
@@ -876,65 +1006,15 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
   block_partials(rr, bb, G, K, partials);
 }
 
-// Small exchanges of the solve loops with the host, kept off the copy engines
-// (which a streaming solve keeps busy with whole vectors): the norms are
-// written into mapped pinned host memory, the per-right-hand-side flags come
-// in as a kernel argument.  One block each.
-__global__ void k_copy_f64(double* __restrict__ dst, const double* __restrict__ src, int n) {
-  grid_dependency_wait();
-  grid_launch_dependents();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
-}
+// The solve loops' per-right-hand-side flags come in as a kernel argument (and
+// the norms go out through mapped pinned host memory, SumTarget::host): small
+// exchanges kept off the copy engines, which a streaming solve keeps busy with
+// whole vectors.
 __global__ void k_set_flags(int* __restrict__ flags, unsigned long long mask, int k) {
   grid_dependency_wait();
   grid_launch_dependents();
   const int c = threadIdx.x;
   if (c < k) flags[c] = int((mask >> c) & 1ull);
-}
-
-// Sum of per-block partials in a fixed order (one block): sums[2K]; up to
-// kSumWide sums (K <= 4: the solve's right-hand sides) reduced side by side
-constexpr int kSumWide = 8;
-__global__ void k_sum_partials(const double* __restrict__ partials, int nBlocks, int K, double* __restrict__ sums) {
-  grid_dependency_wait();
-  grid_launch_dependents();
-  __shared__ double sh[256];
-  if (2 * K <= kSumWide) {
-    // every sum at once (one tree for all of them): per sum the same thread
-    // partials, in the same order, and the same tree as the loop below
-    __shared__ double shw[kSumWide][256];
-    double s[kSumWide];
-#pragma unroll
-    for (int c = 0; c < kSumWide; c++) s[c] = 0;
-    for (int b = threadIdx.x; b < nBlocks; b += blockDim.x)
-#pragma unroll
-      for (int c = 0; c < kSumWide; c++)
-        if (c < 2 * K) s[c] += partials[(long long)b * 2 * K + c];
-#pragma unroll
-    for (int c = 0; c < kSumWide; c++) shw[c][threadIdx.x] = s[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w)
-#pragma unroll
-        for (int c = 0; c < kSumWide; c++)
-          if (c < 2 * K) shw[c][threadIdx.x] += shw[c][threadIdx.x + w];
-      __syncthreads();
-    }
-    if ((int)threadIdx.x < 2 * K) sums[threadIdx.x] = shw[threadIdx.x][0];
-    return;
-  }
-  for (int c = 0; c < 2 * K; c++) {
-    double s = 0;
-    for (int b = threadIdx.x; b < nBlocks; b += blockDim.x) s += partials[(long long)b * 2 * K + c];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) sums[c] = sh[0];
-    __syncthreads();
-  }
 }
 
 // ----------------------------------------------------------------------------
@@ -968,16 +1048,12 @@ __global__ void __launch_bounds__(256) k_fcg_precond(long long n, int K, int KP,
   block_partials(a, b, G, K, partials);
 }
 
-// beta = -alpha_old (z . q_old) / rho_old (0 on a (re)start, rho_old = 0); rho = z . r
+// the scalars as launches of their own (more right-hand sides than one block sums)
 __global__ void k_fcg_beta(int K, const double* __restrict__ sums, double* __restrict__ sc) {
   grid_dependency_wait();
   grid_launch_dependents();
   const int c = threadIdx.x;
-  if (c >= K) return;
-  const double rho = sums[c], gamma = sums[K + c], rhoOld = sc[3 * K + c];
-  sc[K + c] = rhoOld != 0.0 ? -sc[c] * gamma / rhoOld : 0.0;
-  sc[2 * K + c] = rho;
-  sc[3 * K + c] = rho;
+  if (c < K) fcg_beta(K, c, sums[c], sums[K + c], sc);
 }
 
 // p = z + beta p
@@ -991,14 +1067,11 @@ __global__ void __launch_bounds__(256) k_fcg_direction(long long n, int K, const
   p[t] = z[t] + sc[K + c] * p[t];
 }
 
-// alpha = rho / (p . A p), 0 for frozen right-hand sides
 __global__ void k_fcg_alpha(int K, const double* __restrict__ sums, const int* __restrict__ frozen, double* __restrict__ sc) {
   grid_dependency_wait();
   grid_launch_dependents();
   const int c = threadIdx.x;
-  if (c >= K) return;
-  const double pq = sums[c];
-  sc[c] = (frozen && frozen[c]) || !(pq > 0) ? 0.0 : sc[2 * K + c] / pq;
+  if (c < K) fcg_alpha(K, c, sums[c], frozen, sc);
 }
 
 // x += alpha p, r -= alpha q, r packed into the next V-cycle's FP32 right-hand
@@ -1256,10 +1329,26 @@ void launch_boundary_solve(const BoundaryDev<T>& B, const T* rhs, T* x, int KP, 
   // product sits between the two launches
   if (B.nI > 0) launch(k_bs_back<T, W>, dim3(nblk((long long)B.nI * G * 8)), s, B, x, KP, G, B.nS > 0 ? 1 : 0);
 }
+// Rows per warp R and channel groups per warp Q.  One group: the fewest rows that
+// fit the blocks on one wave of two per SM, so that a small level's rows spread and
+// a large one reuses the right-hand side (n = 2316: 14.9 us with R = 4, 17.5 with
+// R = 2 in 1.3 waves, 21.8 with R = 8 and fewer loads in flight, 23.6 before, a
+// warp per part of one row; n = 1024, R = 2: 5.0 us, 5.8 before).  Several groups:
+// the inverse read once for up to 4 (n = 2219, 16 groups: 152 us with R = Q = 4,
+// 187 with R = 2 and twice the loads ahead, 423 before, a read per group).
 template <typename T, int W>
 void launch_coarse_solve(int n, const double* ainv, const double* scale, const T* rhs, T* x, int KP, cudaStream_t s) {
   if (n == 0) return;
-  launch(k_coarse_solve<T, W>, dim3((n + 1) / 2), s, n, ainv, scale, rhs, x, KP, KP / W);
+  const int G = KP / W;
+  auto go = [&](auto kernel, int R, int Q) { launch(kernel, dim3((n + 2 * R - 1) / (2 * R), G / Q), s, n, ainv, scale, rhs, x, KP); };
+  if constexpr (W > 1) {
+    if (G % 4 == 0) return go(k_coarse_solve<T, W, 4, 4, 1>, 4, 4);
+    if (G % 2 == 0) return go(k_coarse_solve<T, W, 2, 2, 4>, 2, 2);
+  }
+  constexpr int kWave = 2 * 148;
+  if (n <= 2 * kWave) return go(k_coarse_solve<T, W, 1, 1, 4>, 1, 1);
+  if (n <= 4 * kWave) return go(k_coarse_solve<T, W, 2, 1, 4>, 2, 1);
+  go(k_coarse_solve<T, W, 4, 1, 4>, 4, 1);
 }
 
 static inline int raw_groups(int K) { int G = 1; while (4 * G < K) G *= 2; return G; }
@@ -1282,61 +1371,66 @@ static int raw_blocks() {
     return std::min(kRawMaxBlocks, 8 * sms);
   });
 }
+// The 2K sums of a launch of `blocks` blocks; scalar: true when the reduction
+// evaluated it too (it holds every sum in one block)
+static bool launch_sums(const SumTarget& t, int blocks, int K, cudaStream_t s, int scalar = 0, double* sc = nullptr,
+                        const int* frozen = nullptr) {
+  const bool one = 2 * K <= kSumWide;
+  launch(k_sum_partials, dim3((2 * K + kSumWide - 1) / kSumWide), s, (const double*)t.partials, blocks, K, t.sums, t.host, one ? scalar : 0,
+         sc, frozen);
+  return one;
+}
 void launch_raw_operator(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
                          const double* bVal, const int* bGlobal, int nB, const double* b, const double* x, double* out, int K,
-                         int mode, double* partials, double* sums, cudaStream_t s) {
+                         int mode, const SumTarget& t, cudaStream_t s) {
   const int G = raw_groups(K);
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
   launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, G, mode,
-         partials, (float*)nullptr, 0);
-  if (partials && sums) launch(k_sum_partials, dim3(1), s, partials, blocks, K, sums);
+         t.partials, (float*)nullptr, 0);
+  if (t.partials && t.sums) launch_sums(t, blocks, K, s);
 }
 int raw_operator_blocks(int nRuns, int nB, int K) { return raw_blocks(); }
 void launch_raw_residual_f32(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr,
                              const int* bCol, const double* bVal, const int* bGlobal, int nB, const double* b, const double* x,
-                             float* rhs32, int K, int KP, double* partials, double* sums, cudaStream_t s, bool xZero) {
+                             float* rhs32, int K, int KP, const SumTarget& t, cudaStream_t s, bool xZero) {
   const int G = raw_groups(K);
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
   launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, (double*)nullptr, K,
-         G, xZero ? 3 : 0, partials, rhs32, KP);
-  if (partials && sums) launch(k_sum_partials, dim3(1), s, partials, blocks, K, sums);
+         G, xZero ? 3 : 0, t.partials, rhs32, KP);
+  launch_sums(t, blocks, K, s);
 }
 
 // ---- flexible CG steps (fixed grids: partial sums in a fixed order)
 static inline int fcg_blocks(long long n, int G) { return int(std::min<long long>(raw_blocks(), nblk(n * G))); }
-void launch_fcg_precond(long long n, int K, int KP, float* e, const double* r, const double* q, double* z, double* partials,
-                        double* sums, double* sc, cudaStream_t s) {
+void launch_fcg_precond(long long n, int K, int KP, float* e, const double* r, const double* q, double* z, const SumTarget& t,
+                        double* sc, cudaStream_t s) {
   const int G = raw_groups(K), blocks = fcg_blocks(n, G);
-  launch(k_fcg_precond, dim3(blocks), s, n, K, KP, G, e, r, q, z, partials);
-  launch(k_sum_partials, dim3(1), s, partials, blocks, K, sums);
-  launch(k_fcg_beta, dim3(1), s, K, (const double*)sums, sc);
+  launch(k_fcg_precond, dim3(blocks), s, n, K, KP, G, e, r, q, z, t.partials);
+  if (!launch_sums(t, blocks, K, s, 1, sc)) launch(k_fcg_beta, dim3(1), s, K, (const double*)t.sums, sc);
 }
 void launch_fcg_direction(long long n, int K, const double* z, const double* sc, double* p, cudaStream_t s) {
   launch(k_fcg_direction, dim3(nblk(n * K)), s, n, K, z, sc, p);
 }
-void launch_fcg_alpha(int K, const double* sums, const int* frozen, double* sc, cudaStream_t s) {
-  launch(k_fcg_alpha, dim3(1), s, K, sums, frozen, sc);
-}
 void launch_fcg_update(long long n, int K, int KP, const double* sc, const double* p, const double* q, double* x, double* r, float* rhs32,
-                       double* partials, double* sums, cudaStream_t s) {
+                       const SumTarget& t, cudaStream_t s) {
   const int G = raw_groups(K), blocks = fcg_blocks(n, G);
-  launch(k_fcg_update, dim3(blocks), s, n, K, KP, G, sc, p, q, x, r, rhs32, partials);
-  launch(k_sum_partials, dim3(1), s, partials, blocks, K, sums);
+  launch(k_fcg_update, dim3(blocks), s, n, K, KP, G, sc, p, q, x, r, rhs32, t.partials);
+  launch_sums(t, blocks, K, s);
 }
 void launch_raw_apply_dot(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
-                          const double* bVal, const int* bGlobal, int nB, const double* x, double* out, int K, double* partials,
-                          double* sums, cudaStream_t s) {
+                          const double* bVal, const int* bGlobal, int nB, const double* x, double* out, int K, const int* frozen,
+                          double* sc, const SumTarget& t, cudaStream_t s) {
   const int G = raw_groups(K);
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
   launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, (const double*)nullptr, x,
-         out, K, G, 2, partials, (float*)nullptr, 0);
-  launch(k_sum_partials, dim3(1), s, partials, blocks, K, sums);
+         out, K, G, 2, t.partials, (float*)nullptr, 0);
+  if (!launch_sums(t, blocks, K, s, 2, sc, frozen)) launch(k_fcg_alpha, dim3(1), s, K, (const double*)t.sums, frozen, sc);
 }
 
 void launch_axpby(double* out, double a, const double* x, double b, const double* y, long long n, cudaStream_t s) {
@@ -1346,7 +1440,6 @@ template <typename T>
 void launch_pack_rhs(const double* r, T* rhs, long long n, int K, int KP, cudaStream_t s) {
   launch(k_pack_rhs<T>, dim3(nblk(n * KP)), s, r, rhs, n, K, KP);
 }
-void launch_copy_f64(double* dst, const double* src, int n, cudaStream_t s) { launch(k_copy_f64, dim3(1), s, dst, src, n); }
 void launch_set_flags(int* flags, unsigned long long mask, int k, cudaStream_t s) {
   launch(k_set_flags, dim3(1), s, flags, mask, k);
 }

@@ -179,9 +179,15 @@ void launch_boundary_solve(const BoundaryDev<T>& B, const T* rhs, T* x, int KP, 
 template <typename T, int W>
 void launch_coarse_solve(int n, const double* ainv, const double* scale, const T* rhs, T* x, int KP, cudaStream_t s);
 
+// Where a launch's per-right-hand-side sums go: its blocks' partial sums
+// (raw_operator_blocks() x 2K), the 2K sums, optionally their copy in mapped host
+// memory
+struct SumTarget {
+  double *partials = nullptr, *sums = nullptr, *host = nullptr;
+};
 void launch_raw_operator(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
                          const double* bVal, const int* bGlobal, int nB, const double* b, const double* x, double* out, int K,
-                         int mode, double* partials, double* sums, cudaStream_t s);
+                         int mode, const SumTarget& t, cudaStream_t s);
 // Blocks of the FP64 operator's fixed grid on the current device (8 per SM, at
 // most kRawMaxBlocks): the partial-sum buffers hold this many blocks x 2K.
 constexpr int kRawMaxBlocks = 2048;
@@ -191,29 +197,25 @@ int raw_operator_blocks(int nRuns, int nB, int K);
 // same bits and norms)
 void launch_raw_residual_f32(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr,
                              const int* bCol, const double* bVal, const int* bGlobal, int nB, const double* b, const double* x,
-                             float* rhs32, int K, int KP, double* partials, double* sums, cudaStream_t s, bool xZero = false);
+                             float* rhs32, int K, int KP, const SumTarget& t, cudaStream_t s, bool xZero = false);
 template <typename T>
 void launch_pack_rhs(const double* r, T* rhs, long long n, int K, int KP, cudaStream_t s);
-// n doubles (n <= a few hundred) by one block, e.g. into mapped pinned host memory
-void launch_copy_f64(double* dst, const double* src, int n, cudaStream_t s);
 // flags[c] = bit c of mask, c < k <= 64
 void launch_set_flags(int* flags, unsigned long long mask, int k, cudaStream_t s);
 // Flexible preconditioned CG around the FP32 V-cycle (vcycle_kernels.cu).  sc: 4K
 // per-RHS scalars {alpha, beta, rho, rho_old}; sums: 2K.
 //   precond:   z = e (e cleared), rho = z.r, beta = -alpha_old (z.q_old) / rho_old
 //   direction: p = z + beta p
-//   apply_dot: q = A p, sums[0..K) = p.q
-//   alpha:     alpha = rho / p.q (0 where frozen)
+//   apply_dot: q = A p, sums[0..K) = p.q, alpha = rho / p.q (0 where frozen)
 //   update:    x += alpha p, r -= alpha q, rhs32 = r, sums[0..K) = r.r
-void launch_fcg_precond(long long n, int K, int KP, float* e, const double* r, const double* q, double* z, double* partials,
-                        double* sums, double* sc, cudaStream_t s);
+void launch_fcg_precond(long long n, int K, int KP, float* e, const double* r, const double* q, double* z, const SumTarget& t,
+                        double* sc, cudaStream_t s);
 void launch_fcg_direction(long long n, int K, const double* z, const double* sc, double* p, cudaStream_t s);
 void launch_raw_apply_dot(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
-                          const double* bVal, const int* bGlobal, int nB, const double* x, double* out, int K, double* partials,
-                          double* sums, cudaStream_t s);
-void launch_fcg_alpha(int K, const double* sums, const int* frozen, double* sc, cudaStream_t s);
+                          const double* bVal, const int* bGlobal, int nB, const double* x, double* out, int K, const int* frozen,
+                          double* sc, const SumTarget& t, cudaStream_t s);
 void launch_fcg_update(long long n, int K, int KP, const double* sc, const double* p, const double* q, double* x, double* r, float* rhs32,
-                       double* partials, double* sums, cudaStream_t s);
+                       const SumTarget& t, cudaStream_t s);
 // out = a x + b y over n doubles
 void launch_axpby(double* out, double a, const double* x, double b, const double* y, long long n, cudaStream_t s);
 // x += e (columns c with frozen[c] != 0 unchanged; frozen may be null), then e = 0

@@ -92,8 +92,11 @@ extern "C" int gdtp_residual_static(gdtp_system* s, const double* b_dev, const d
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // every block overwrites its own partials and the reduction overwrites the
   // totals, so the scratch needs no clearing between calls
+  dev::SumTarget sumTarget;
+  sumTarget.partials = partials;
+  sumTarget.sums = sums;
   dev::launch_raw_operator(op.runs, op.nRuns, op.coef, op.planeStride, op.bPtr, op.bCol, op.bVal, op.bGlobal, op.nB, b_dev, x_dev,
-                           r_dev, k, 0, partials, sums, st);
+                           r_dev, k, 0, sumTarget, st);
   double tot[2 * kStaticMaxRhs];
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(tot, sums, 2 * size_t(k) * sizeof(double), cudaMemcpyDeviceToHost, st);

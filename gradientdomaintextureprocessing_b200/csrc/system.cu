@@ -1448,14 +1448,9 @@ bool DeviceSystem::ensure_work(int kk) {
 }
 
 bool DeviceSystem::read_norms(int k, cudaStream_t s, const char* what) {
-  if (sumsMapped_) {
-    kernelLaunches += 1;
-    dev::launch_copy_f64(sumsMapped_, sums_, 2 * k, s);
-    if (!check(cudaGetLastError(), "norms to host")) return false;
-  } else if (!check(cudaMemcpyAsync(sumsHost_, sums_, 2 * size_t(k) * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h norms")) {
+  if (!sumsMapped_ && !check(cudaMemcpyAsync(sumsHost_, sums_, 2 * size_t(k) * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h norms"))
     return false;
-  }
-  return check(cudaStreamSynchronize(s), what);
+  return check(cudaGetLastError(), what) && check(cudaStreamSynchronize(s), what);
 }
 
 bool DeviceSystem::upload_flags(int k, cudaStream_t s) {
@@ -1470,7 +1465,7 @@ bool DeviceSystem::upload_flags(int k, cudaStream_t s) {
 bool DeviceSystem::raw_apply_dev(const RawOperator& op, const double* b, const double* x, double* out, int k, int mode,
                                  cudaStream_t s, double* sumsHost) {
   dev::launch_raw_operator(op.runs, op.nRuns, op.coef, op.planeStride, op.bPtr, op.bCol, op.bVal, op.bGlobal, op.nB, b, x, out, k,
-                           mode, partials_, sums_, s);
+                           mode, sum_target(true), s);
   if (!sumsHost) return check(cudaGetLastError(), "raw operator");
   return check(cudaMemcpyAsync(sumsHost, sums_, 2 * size_t(k) * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h norms") &&
          check(cudaStreamSynchronize(s), "raw operator");
@@ -1685,7 +1680,7 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
       dev::launch_add_correction<float>(X, D0.x, (long long)n, k, mg.KP, s, frozen_);
       // r = b - A x, written straight into the FP32 right-hand side of the next V-cycle
       dev::launch_raw_residual_f32(rawA_.runs, rawA_.nRuns, rawA_.coef, rawA_.planeStride, rawA_.bPtr, rawA_.bCol, rawA_.bVal,
-                                   rawA_.bGlobal, rawA_.nB, B, X, D0.b, k, mg.KP, partials_, sums_, s);
+                                   rawA_.bGlobal, rawA_.nB, B, X, D0.b, k, mg.KP, sum_target(true), s);
       profiling_ = false;
       if (!check(cudaStreamEndCapture(s, &g), "capture end")) return false;
       StepGraph sg;
@@ -1703,7 +1698,7 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
     if (!check(cudaMemsetAsync(mg.levels[0].x, 0, n * mg.KP * sizeof(float), s), "zero correction")) return false;
     kernelLaunches += 2;  // operator + norm reduction
     dev::launch_raw_residual_f32(rawA_.runs, rawA_.nRuns, rawA_.coef, rawA_.planeStride, rawA_.bPtr, rawA_.bCol, rawA_.bVal,
-                                 rawA_.bGlobal, rawA_.nB, B, X, mg.levels[0].b, k, mg.KP, partials_, sums_, s, zeroGuess);
+                                 rawA_.bGlobal, rawA_.nB, B, X, mg.levels[0].b, k, mg.KP, sum_target(true), s, zeroGuess);
     if (!read_norms(k, s, "initial residual")) return false;
     rep = SolveReport();
     rep.rel.assign(k, 0.0);
@@ -1911,7 +1906,7 @@ bool DeviceSystem::krylov_solve(Multigrid<float>& mg, const double* B, double* X
   auto true_residual = [&]() {
     kernelLaunches += 2;  // operator + norm reduction
     dev::launch_raw_operator(rawA_.runs, rawA_.nRuns, rawA_.coef, rawA_.planeStride, rawA_.bPtr, rawA_.bCol, rawA_.bVal, rawA_.bGlobal,
-                             rawA_.nB, B, X, r64_, k, 0, partials_, sums_, s);
+                             rawA_.nB, B, X, r64_, k, 0, sum_target(true), s);
     return fetch("residual");
   };
   // (re)start: p = q = 0, rho_old = 0, the V-cycle's right-hand side = r, e = 0
@@ -1940,12 +1935,11 @@ bool DeviceSystem::krylov_solve(Multigrid<float>& mg, const double* B, double* X
     if (!check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture")) return false;
     if (KP == 1) vcycle<float, 1>(mg, s, true); else vcycle<float, 4>(mg, s, true);
     profiling_ = false;
-    dev::launch_fcg_precond((long long)n, k, KP, D0.x, r64_, q_, z_, partials_, sums_, sc_, s);
+    dev::launch_fcg_precond((long long)n, k, KP, D0.x, r64_, q_, z_, sum_target(false), sc_, s);
     dev::launch_fcg_direction((long long)n, k, z_, sc_, p_, s);
     dev::launch_raw_apply_dot(rawA_.runs, rawA_.nRuns, rawA_.coef, rawA_.planeStride, rawA_.bPtr, rawA_.bCol, rawA_.bVal, rawA_.bGlobal,
-                              rawA_.nB, p_, q_, k, partials_, sums_, s);
-    dev::launch_fcg_alpha(k, sums_, frozen_, sc_, s);
-    dev::launch_fcg_update((long long)n, k, KP, sc_, p_, q_, X, r64_, D0.b, partials_, sums_, s);
+                              rawA_.nB, p_, q_, k, frozen_, sc_, sum_target(false), s);
+    dev::launch_fcg_update((long long)n, k, KP, sc_, p_, q_, X, r64_, D0.b, sum_target(true), s);
     if (!check(cudaStreamEndCapture(s, &g), "capture end")) return false;
     StepGraph sg;
     sg.kind = 1;

@@ -355,8 +355,16 @@ class DeviceSystem {
   int filterK_ = 0;
   double* sumsHost_ = nullptr;    // pinned, mapped
   double* sumsMapped_ = nullptr;  // its device address (null: norms come back by copy)
-  // the solve loops' small host exchanges, by kernel: norms sums_ -> sumsHost_
-  // (then waits for the stream), flags frozenHost_ -> frozen_
+  // where the stream's reductions go; toHost: also into sumsHost_ (mapped)
+  dev::SumTarget sum_target(bool toHost) const {
+    dev::SumTarget t;
+    t.partials = partials_;
+    t.sums = sums_;
+    if (toHost) t.host = sumsMapped_;
+    return t;
+  }
+  // the solve loops' small host exchanges: the norms of a launch that reduced
+  // into sum_target(true), once the stream is done; flags frozenHost_ -> frozen_
   bool read_norms(int k, cudaStream_t s, const char* what);
   bool upload_flags(int k, cudaStream_t s);
   // solve_stream: two slots of device b / x (n x k FP64), alternating between

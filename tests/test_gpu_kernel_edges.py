@@ -1,0 +1,88 @@
+"""Edges of the solve kernels' launch rules on the device: widths, level sizes
+and shapes where a kernel changes its variant or its last block is ragged.
+
+Tolerances: the FP32 V-cycle's arithmetic per right-hand side does not depend on
+how many are solved together nor on which kernel variant runs, so those
+comparisons are bitwise.  Norms are FP64 sums of n x 2 non-negative terms:
+relative error at most n 2^-53 (n <= 1e5 here), so 1e-11 with numpy's own.
+"""
+import numpy as np
+import pytest
+
+from conftest import golden_mesh, load_golden
+
+pytestmark = pytest.mark.gpu
+
+
+def make(name, levels=None, metric=False):
+    from gradientdomaintextureprocessing_b200.hierarchy import InitializeHierarchy
+    from gradientdomaintextureprocessing_b200.system import System
+    g = load_golden(name)
+    h = InitializeHierarchy(golden_mesh(g), levels=int(g["meta/size"][2]) if levels is None else levels)
+    s = System(h)
+    s.update(1e-3, 1.0)
+    return s
+
+
+@pytest.fixture(scope="module")
+def torus(built_lib):
+    return make("torus128")
+
+
+@pytest.fixture(scope="module")
+def ico(built_lib):
+    return make("ico256")
+
+
+def vectors(n, k, seed=0):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal((n, k)), rng.standard_normal((n, k))
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 33, 64])
+def test_norm_sums_at_every_width(torus, k):
+    b, x = vectors(torus.n, k)
+    r = b - torus.apply(x)
+    expect = np.sqrt((r * r).sum(0) / (b * b).sum(0))
+    np.testing.assert_allclose(torus.residual(b, x), expect, rtol=1e-11)
+    np.testing.assert_array_equal(torus.residual(b, x), torus.residual(b, x))
+
+
+@pytest.mark.parametrize("k", [1, 3, 5, 9, 13, 64])
+def test_reported_residual_is_the_solutions(torus, k):
+    b, _ = vectors(torus.n, k)
+    for krylov in (0, 1):
+        torus.set("krylov", krylov)
+        try:
+            x, rep = torus.solve(b, tol=1e-6, max_iters=200)
+        finally:
+            torus.set("krylov", 0)
+        np.testing.assert_allclose(rep["rel_residual_max"], torus.residual(b, x).max(), rtol=1e-11)
+
+
+@pytest.mark.parametrize("k", [2, 5, 9, 16, 40, 64])
+def test_vcycle_columns_do_not_depend_on_the_width(ico, k):
+    b, x = (v.astype(np.float32) for v in vectors(ico.n, k))
+    wide = ico.vcycle(x, b)
+    for c in (0, k // 2, k - 1):
+        np.testing.assert_array_equal(wide[:, c], ico.vcycle(x[:, c], b[:, c])[:, 0])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("max_coarse", [2600, 1000, 600, 300, 260])
+def test_coarsest_solve_at_every_size(torus, ico, max_coarse, precision):
+    """The coarsest level's rows per block follow its size; the coarse-level
+    cluster kernel solves it a row per warp, with the same bits."""
+    for s in (torus, ico):
+        b, _ = vectors(s.n, 3)
+        try:
+            s.set("max_coarse", max_coarse)
+            s.update(1e-3, 1.0)
+            got, rep = s.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)
+            s.set("cluster_texels", 1 << 30)
+            ref, _ = s.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)
+        finally:
+            s.set("cluster_texels", 0)
+            s.set("max_coarse", 2600)
+            s.update(1e-3, 1.0)
+        np.testing.assert_array_equal(got, ref)
