@@ -284,87 +284,6 @@ __global__ void __launch_bounds__(kGroupBlockMax, 1) k_gs_groups(const ColourRun
   }
 }
 
-// The chart smoother for FP32 vectors of one channel group whose colour passes
-// fit kGroupRegBlock threads: thread t owns item t of every colour (run t / 32,
-// texel t % 32) and loads its run, coefficients and (rhsEarly) right-hand side
-// for all four colours before the dependency wait, with independent loads;
-// the passes then read x from shared memory only.  REV: colours 3..0.  Same
-// updates, same order, same bits as k_gs_groups.
-constexpr int kGroupRegBlock = 512;
-template <int W, bool REV>
-__global__ void __launch_bounds__(kGroupRegBlock, 1) k_gs_groups_reg(const ColourRun* __restrict__ runs,
-                                                                   const int* __restrict__ groups, const float* __restrict__ coef,
-                                                                   int planeStride, const float* __restrict__ rhs,
-                                                                   float* __restrict__ x, int sweeps, int rhsEarly) {
-  constexpr int KP = W;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* xs = reinterpret_cast<float*>(smem_raw);
-  const int* g = groups + 10 * blockIdx.x;
-  const int lo = g[8], span = g[9];
-  const int t = threadIdx.x, m = t & 31;
-  bool act[4];
-  int pos[4], pp[4], pn[4];
-  float w[4][9];
-  Vec<float, W> bv[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    act[c] = false;
-    pos[c] = pp[c] = pn[c] = 0;
-    if (t < g[4 + c] * 32) {
-      const ColourRun R = runs[g[c] + (t >> 5)];
-      if (m < R.len) {
-        act[c] = true;
-        pos[c] = R.pos0 + 2 * m - lo;
-        pp[c] = R.prev0 + 2 * m - lo;
-        pn[c] = R.next0 + 2 * m - lo;
-        const float* cf = coef + R.coef0 + m;
-#pragma unroll
-        for (int k = 0; k < 9; k++) w[c][k] = cf[k * planeStride];
-        if (rhsEarly) bv[c] = vload<float, W>(rhs + (long long)(pos[c] + lo) * KP);
-      }
-    }
-  }
-  grid_dependency_wait();
-  grid_launch_dependents();
-  for (int i = t; i < span * KP; i += blockDim.x) xs[i] = x[(long long)lo * KP + i];
-  if (!rhsEarly)
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-      if (act[c]) bv[c] = vload<float, W>(rhs + (long long)(pos[c] + lo) * KP);
-  __syncthreads();
-  // the pass loop stays rolled (the per-colour arrays then live in local
-  // memory, L1-resident): unrolled, the compiled passes did not reproduce the
-  // launch path's bits
-  for (int sw = 0; sw < sweeps; sw++) {
-#pragma unroll 1
-    for (int cc = 0; cc < 4; cc++) {
-      const int c = REV ? 3 - cc : cc;
-      if (act[c]) {
-        Vec<float, W> acc;
-#pragma unroll
-        for (int k = 0; k < W; k++) acc.v[k] = 0;
-        axpy(acc, w[c][0], vload<float, W>(xs + (pp[c] - 1) * KP));
-        axpy(acc, w[c][1], vload<float, W>(xs + (pp[c]) * KP));
-        axpy(acc, w[c][2], vload<float, W>(xs + (pp[c] + 1) * KP));
-        axpy(acc, w[c][3], vload<float, W>(xs + (pos[c] - 1) * KP));
-        axpy(acc, w[c][5], vload<float, W>(xs + (pos[c] + 1) * KP));
-        axpy(acc, w[c][6], vload<float, W>(xs + (pn[c] - 1) * KP));
-        axpy(acc, w[c][7], vload<float, W>(xs + (pn[c]) * KP));
-        axpy(acc, w[c][8], vload<float, W>(xs + (pn[c] + 1) * KP));
-        Vec<float, W> out;
-#pragma unroll
-        for (int k = 0; k < W; k++) out.v[k] = bv[c].v[k] * w[c][4] - acc.v[k];
-        vstore<float, W>(xs + pos[c] * KP, out);
-      }
-      __syncthreads();
-    }
-  }
-  // write back this thread's deep texels (boundary texels of the span stay)
-#pragma unroll
-  for (int c = 0; c < 4; c++)
-    if (act[c]) vstore<float, W>(x + (long long)(pos[c] + lo) * KP, vload<float, W>(xs + pos[c] * KP));
-}
-
 // ----------------------------------------------------------------------------
 // Residual: deep rows by runs (all colours), boundary rows by CSR (global cols).
 // Blocks [0, deepBlocks) handle deep texels, the rest boundary rows.
@@ -1234,37 +1153,6 @@ bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cu
   if (D.nGroups == 0 || sweeps <= 0) return true;
   const size_t smem = gs_groups_smem<T, W>(D, KP);
   if (smem > kGroupSmemMax) return false;
-  if constexpr (std::is_same<T, float>::value) {
-    // one channel group, every colour pass of a chart within one block: the
-    // register-staged variant
-    if (KP == W && D.maxGroupColourRuns > 0 && D.maxGroupColourRuns * 32 <= kGroupRegBlock) {
-      auto kern = reverse ? k_gs_groups_reg<W, true> : k_gs_groups_reg<W, false>;
-      static std::atomic<int> regAttr[2][kMaxDevices];
-      static const bool regInit = [] {
-        for (auto& r : regAttr)
-          for (auto& a : r) a.store(kUnset);
-        return true;
-      }();
-      (void)regInit;
-      const int okReg = per_device_once(regAttr[reverse ? 1 : 0], [kern] {
-        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGroupSmemMax)) == cudaSuccess ? 1 : 0;
-      });
-      if (okReg) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(D.nGroups);
-        cfg.blockDim = dim3(std::max(128, D.maxGroupColourRuns * 32));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = g_programmatic ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, kern, D.runs, D.groups, (const float*)D.coef, D.planeStride, (const float*)D.b, D.x, sweeps,
-                                  rhsEarly ? 1 : 0) == cudaSuccess;
-      }
-    }
-  }
   static std::atomic<int> attr[kMaxDevices];
   static const bool init = [] {
     for (auto& a : attr) a.store(kUnset);

@@ -17,6 +17,26 @@ struct ColourRun;
 struct RowLine;
 struct RestrictRun;
 struct ProlongRun;
+// Cluster chart smoother (chart_cluster.cu): a pair of texels 2q, 2q + 1 of a
+// raster line.  pos: texel 2q, | 1 << kItemPairBit when 2q + 1 exists, | 1 <<
+// kItemOddBit when 2q is in an odd column, | 1 << kItemUpBit (kItemUpBit + 1) when
+// the CTA of the rows above (below) keeps a copy of this row; dist: distance to
+// the texel above (bits 0-15) and below (bits 16-31); c0, c1: coefficient indices
+// of 2q and 2q + 1.
+constexpr int kItemPairBit = 27, kItemOddBit = 28, kItemUpBit = 29;
+constexpr int kItemPosMask = (1 << kItemPairBit) - 1;
+struct __align__(16) ClusterItem {
+  int pos, dist, c0, c1;
+};
+// One CTA's rows of a chart: the texels [lo, lo + count) its updates touch (its
+// slab) and those of the CTAs above and below (count 0: none), its items of even
+// and odd rows.
+struct ClusterPart {
+  int lo, count, upLo, upCount, dnLo, dnCount;
+  int item0[2], nItems[2];
+};
+constexpr size_t kClusterSmemMax = 227 * 1024;
+constexpr int kClusterMaxThreads = 512;
 
 // Longest j chunk of a boundary dense product (its input vector is staged in
 // shared memory): subdomains hold at most this many rows, and the separator
@@ -93,6 +113,10 @@ struct LevelDev {
   const int* rowLineOf[2] = {nullptr, nullptr};
   int nRowBins[2] = {0, 0};
   int rowBlock = 0, rowSlots = 0;
+  // chart smoother on clusters (launch_gs_cluster): clusterSize parts per chart
+  const ClusterPart* clusterParts = nullptr;
+  const ClusterItem* clusterItems = nullptr;
+  int nClusterParts = 0, clusterSize = 0, clusterThreads = 0, clusterSlab = 0;
 };
 
 template <typename T, int W>
@@ -130,6 +154,13 @@ constexpr size_t kGroupSmemMax = 200 * 1024;
 // rhsEarly: the previous launch does not write the level's right-hand side
 template <typename T, int W>
 bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s, bool rhsEarly = false);
+// The same sweeps, same bits, on a cluster of CTAs per chart (chart_cluster.cu).
+// zeroStart: x = 0 on entry.  gs_cluster_available: the level has its layout, it
+// fits this device, and KP channels of it fill few enough waves.
+template <typename T, int W>
+bool gs_cluster_available(const LevelDev<T>& D, int KP);
+template <typename T, int W>
+bool launch_gs_cluster(const LevelDev<T>& D, int sweeps, bool reverse, bool zeroStart, int KP, cudaStream_t s, bool rhsEarly = false);
 // Fused smoothing round (tile_smoother.cu): tiles of kTileW x kTileH texels of
 // one chart, a CTA each, `sweeps` 4-colour sweeps in shared memory, x updated
 // in place.  Tiles are ordered by tile colour (tile column parity | tile row

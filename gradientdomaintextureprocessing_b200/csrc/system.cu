@@ -141,6 +141,111 @@ bool build_row_bins(const GridLevel& L, const DeepRuns& R, RowBins& out) {
   return true;
 }
 
+// The smallest cluster whose CTAs have at most kClusterThreadsGoal pairs per row
+// parity; the largest cluster when none does.  False (cluster smoother unused)
+// when the rows do not fit 8 CTAs or an index its packed field.
+static constexpr int kClusterThreadsGoal = 256;
+bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& out) {
+  out = ChartClusters();
+  const int nc = (int)L.charts.size();
+  if (nc == 0 || L.rasterLines.empty() || L.numTexels > dev::kItemPosMask) return false;
+  // rows of each chart (the lines of one row in texel order)
+  struct Row {
+    int cj, deep;
+    std::vector<int> lines;
+  };
+  std::vector<std::vector<Row>> rows(nc);
+  for (size_t li = 0; li < L.rasterLines.size(); li++) {
+    const Line& l = L.rasterLines[li];
+    const NodeInfo& n = L.nodes[l.start];
+    if (n.chart < 0 || n.chart >= nc || l.start - l.prev > 0xffff || l.next - l.start > 0xffff || l.prev >= l.start || l.next <= l.start)
+      return false;
+    std::vector<Row>& rc = rows[n.chart];
+    if (!rc.empty() && rc.back().cj > n.cj) return false;
+    if (rc.empty() || rc.back().cj != n.cj) rc.push_back({n.cj, 0, {}});
+    rc.back().lines.push_back((int)li);
+    rc.back().deep += l.end - l.start + 1;
+  }
+  for (int C = 1; C <= 8; C *= 2) {
+    ChartClusters cc;
+    cc.size = C;
+    int pairs = 0;
+    for (int c = 0; c < nc; c++) {
+      const std::vector<Row>& rc = rows[c];
+      if (rc.empty()) continue;
+      long long total = 0, done = 0;
+      for (const Row& r : rc) total += r.deep;
+      // rows [cut[p], cut[p + 1]) go to part p: at least one while rows remain
+      std::vector<int> cut(C + 1, (int)rc.size());
+      cut[0] = 0;
+      int at = 0;
+      for (int p = 0; p < C; p++) {
+        cut[p] = at;
+        const int from = at;
+        while (at < (int)rc.size() && (at == from || (done + rc[at].deep / 2) * C <= total * (p + 1))) done += rc[at++].deep;
+        if (p == C - 1)
+          while (at < (int)rc.size()) done += rc[at++].deep;
+      }
+      std::vector<dev::ClusterPart> parts(C);
+      for (int p = 0; p < C; p++) {
+        dev::ClusterPart& P = parts[p];
+        P = dev::ClusterPart();
+        if (cut[p] == cut[p + 1]) continue;
+        int lo = INT_MAX, hi = INT_MIN;
+        for (int r = cut[p]; r < cut[p + 1]; r++)
+          for (int li : rc[r].lines) {
+            const Line& l = L.rasterLines[li];
+            const int len = l.end - l.start + 1;
+            lo = std::min(lo, l.prev - 1);
+            hi = std::max(hi, l.next + len);
+          }
+        if (lo < 0 || hi >= L.numTexels) return false;
+        P.lo = lo;
+        P.count = hi - lo + 1;
+        cc.slab = std::max(cc.slab, P.count);
+      }
+      for (int p = 0; p < C; p++) {
+        dev::ClusterPart& P = parts[p];
+        const bool up = p > 0 && parts[p - 1].count > 0, dn = p + 1 < C && parts[p + 1].count > 0;
+        if (up) { P.upLo = parts[p - 1].lo; P.upCount = parts[p - 1].count; }
+        if (dn) { P.dnLo = parts[p + 1].lo; P.dnCount = parts[p + 1].count; }
+        for (int par = 0; par < 2; par++) {
+          P.item0[par] = (int)cc.items.size();
+          for (int r = cut[p]; r < cut[p + 1]; r++) {
+            if ((rc[r].cj & 1) != par) continue;
+            const bool pushUp = up && r == cut[p], pushDn = dn && r == cut[p + 1] - 1;
+            for (int li : rc[r].lines) {
+              const Line& l = L.rasterLines[li];
+              const int len = l.end - l.start + 1, odd = L.nodes[l.start].ci & 1;
+              const int cEven = R.lineCoef[2 * li], cOdd = R.lineCoef[2 * li + 1];
+              if ((cEven < 0 && len > odd) || (cOdd < 0 && len > 1 - odd)) return false;
+              for (int q = 0; 2 * q < len; q++) {
+                dev::ClusterItem it;
+                it.pos = (l.start + 2 * q) | (2 * q + 1 < len ? 1 << dev::kItemPairBit : 0) | (odd << dev::kItemOddBit) |
+                         ((pushUp ? 1 : 0) << dev::kItemUpBit) | ((pushDn ? 1 : 0) << (dev::kItemUpBit + 1));
+                it.dist = int(unsigned(l.start - l.prev) | (unsigned(l.next - l.start) << 16));
+                it.c0 = (odd ? cOdd : cEven) + q;
+                it.c1 = 2 * q + 1 < len ? (odd ? cEven : cOdd) + q : 0;
+                cc.items.push_back(it);
+              }
+            }
+          }
+          P.nItems[par] = (int)cc.items.size() - P.item0[par];
+          pairs = std::max(pairs, P.nItems[par]);
+        }
+        cc.parts.push_back(P);
+      }
+    }
+    cc.threads = std::max(32, (pairs + 31) / 32 * 32);
+    cc.slab = (cc.slab + 1) & ~1;  // the kernel may swap the entries of a pair (slab_slot)
+    if (cc.threads <= kClusterThreadsGoal || (C == 8 && cc.threads <= dev::kClusterMaxThreads)) {
+      out = std::move(cc);
+      return !out.parts.empty();
+    }
+  }
+  return false;
+}
+
 // Per chart and colour, the range of that colour's runs that lie in the chart:
 // grp[10 g + c] = first run, grp[10 g + 4 + c] = run count, then the chart's
 // texel span (first texel, count) that its updates touch.  Runs of a colour
@@ -884,6 +989,18 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
         D.rowSlots = RB.slots;
       }
     }
+    // charts dealt to clusters (all sweeps of a smoothing step in one launch)
+    {
+      ChartClusters CC;
+      if (build_chart_clusters(G, R, CC)) {
+        D.clusterParts = A.upload(CC.parts);
+        D.clusterItems = A.upload(CC.items);
+        D.nClusterParts = (int)CC.parts.size();
+        D.clusterSize = CC.size;
+        D.clusterThreads = CC.threads;
+        D.clusterSlab = CC.slab;
+      }
+    }
     // tiles of the fused smoother (FP32 levels it runs on; the tile_texels knob
     // drops the multigrids when it changes; host-built values only)
     if (!numeric && sizeof(T) == 4 && G.numDeep >= kTileBuildMin && knobs.tileTexels > 0 && G.numDeep >= knobs.tileTexels) {
@@ -1338,6 +1455,8 @@ void DeviceSystem::vcycle(Multigrid<T>& mg, cudaStream_t s, bool zeroStart) {
       // x = 0 on entry (a refinement step's correction, or a level entered
       // through the restriction) unless a boundary solve ran first
       tile_smooth(mg, D, knobs.tilePreSweeps, false, (l > 0 || zeroStart) && !knobs.preBoundary, s, false);
+    } else if (clustered(D, KP) && pre_sweeps(l) > 0) {
+      dev::launch_gs_cluster<T, W>(D, pre_sweeps(l), false, (l > 0 || zeroStart) && !knobs.preBoundary, KP, s);
     } else if (grouped(D, KP) && pre_sweeps(l) > 0) {
       dev::launch_gs_groups<T, W>(D, pre_sweeps(l), false, KP, s);
     } else {
@@ -1395,6 +1514,8 @@ void DeviceSystem::vcycle(Multigrid<T>& mg, cudaStream_t s, bool zeroStart) {
       // timed on level 0: the post-smoothing rounds (coefficients, rhs, x read
       // and written once each per round)
       tile_smooth(mg, D, knobs.tilePostSweeps, true, false, s, profiling_ && l == 0);
+    } else if (clustered(D, KP) && post_sweeps(l) > 0) {
+      dev::launch_gs_cluster<T, W>(D, post_sweeps(l), true, false, KP, s, true);
     } else if (grouped(D, KP) && post_sweeps(l) > 0) {
       // after the prolongation and the boundary solve, which leave the right-hand side alone
       dev::launch_gs_groups<T, W>(D, post_sweeps(l), true, KP, s, true);

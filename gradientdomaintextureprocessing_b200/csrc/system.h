@@ -78,6 +78,16 @@ struct RowBins {
 };
 bool build_row_bins(const GridLevel& L, const DeepRuns& R, RowBins& out);
 
+// Rows of every chart dealt to the CTAs of its cluster (dev::launch_gs_cluster):
+// `size` parts per chart; threads: the most items of one row parity in a part, in
+// warps; slab: the most texels a part touches
+struct ChartClusters {
+  std::vector<dev::ClusterPart> parts;
+  std::vector<dev::ClusterItem> items;
+  int size = 0, threads = 0, slab = 0;
+};
+bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& out);
+
 template <typename T>
 using LevelDev = dev::LevelDev<T>;
 
@@ -133,6 +143,8 @@ struct SolverKnobs {
                                         // step's sweeps split between them)
   int tileFinish = 0;                   // 1: one global colour sweep after each tiled smoothing step
   int deviceFactor = 1;                 // dense set-up inverses and products on the device (0: host)
+  int chartCluster = 1;                 // levels whose charts fit a thread-block cluster smooth all sweeps in
+                                        // one launch, a cluster per chart (0: off)
   int rowSweeps = 1;                    // FP32 colour sweeps of k <= 4 channels as two row-smoother launches
                                         // (0: four colour passes)
 };
@@ -217,6 +229,12 @@ class DeviceSystem {
   bool grouped(const dev::LevelDev<T>& D, int KP) const {
     return knobs.chartTexels > 0 && D.nGroups > 0 && D.maxGroupDeep <= knobs.chartTexels &&
            size_t(D.maxGroupSpan) * KP * sizeof(T) <= dev::kGroupSmemMax;
+  }
+  // the cluster chart smoother runs this level
+  template <typename T>
+  bool clustered(const dev::LevelDev<T>& D, int KP) const {
+    if (!knobs.chartCluster || D.clusterThreads == 0) return false;
+    return KP % 4 == 0 ? dev::gs_cluster_available<T, 4>(D, KP) : dev::gs_cluster_available<T, 1>(D, KP);
   }
   // the fused tile smoother runs this level (FP32 vectors of 1 or 4 channels)
   template <typename T>

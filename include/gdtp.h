@@ -251,6 +251,9 @@ int gdtp_residual_static(gdtp_system* s, const double* b_dev, const double* x_de
  * (levels whose largest chart has at most this many deep texels run all sweeps
  * of a smoothing step in one launch, one block per chart with the chart's
  * texels in shared memory; same results; default 1000, 0 = off),
+ * "chart_cluster" (0/1, default 1: levels whose charts fit a thread-block
+ * cluster each run all sweeps of a smoothing step in one launch, a cluster per
+ * chart; same results; takes precedence over "chart_texels"),
  * "trace_levels" (0/1: time every level's legs, arrays "profile.levels" and
  * "profile.cluster"), "krylov" (0/1, default 0: flexible preconditioned
  * conjugate gradients in FP64 around the FP32 V-cycle instead of plain

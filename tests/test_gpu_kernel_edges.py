@@ -86,3 +86,41 @@ def test_coarsest_solve_at_every_size(torus, ico, max_coarse, precision):
             s.set("max_coarse", 2600)
             s.update(1e-3, 1.0)
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.fixture(scope="module", params=[("torus", 256, 256), ("torus", 301, 277), ("icosphere", 512, 512), ("icosphere", 905, 643),
+                                        ("genus2", 643, 905)])
+def atlas(request, built_lib):
+    from gradientdomaintextureprocessing_b200 import meshgen
+    from gradientdomaintextureprocessing_b200.hierarchy import InitializeHierarchy
+    from gradientdomaintextureprocessing_b200.system import System
+    name, w, h = request.param
+    m = {"torus": lambda: meshgen.torus_atlas(w, h), "icosphere": lambda: meshgen.icosphere_atlas(w, h, subdiv=5),
+         "genus2": lambda: meshgen.genus2_atlas(w, h, nu=176, nv=72)}[name]()
+    s = System(InitializeHierarchy(m, w, h, levels=4))
+    s.update(1e-3, 1.0)
+    return s
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("k", [1, 3, 15])
+def test_cluster_chart_smoother_matches_the_launches(atlas, k, precision):
+    """All sweeps of a chart in one cluster launch: the bits of the row and colour launches."""
+    b, _ = vectors(atlas.n, k)
+    sweeps = {q: atlas.get(q) for q in ("coarse_pre_sweeps", "pre_sweeps", "post_sweeps")}
+    got = {}
+    for pre in (0, 2):
+        try:
+            atlas.set("coarse_pre_sweeps", pre)
+            atlas.set("pre_sweeps", 3 - pre)
+            atlas.set("post_sweeps", 1 + pre)
+            for on in (1, 0):
+                atlas.set("chart_cluster", on)
+                atlas.set("chart_texels", 0 if on == 0 else 1000)
+                got[on] = atlas.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+        finally:
+            atlas.set("chart_cluster", 1)
+            atlas.set("chart_texels", 1000)
+            for q, v in sweeps.items():
+                atlas.set(q, v)
+        np.testing.assert_array_equal(got[1], got[0])
