@@ -48,14 +48,6 @@ namespace gdtp {
 namespace dev {
 namespace {
 
-// acc += a v as fused multiply-adds, written out: left to contraction, the first
-// two terms (of a sum that starts at 0) may be fused the other way round
-template <typename T, int W>
-__device__ __forceinline__ void fma_to(Vec<T, W>& acc, T a, const Vec<T, W>& v) {
-#pragma unroll
-  for (int c = 0; c < W; c++) acc.v[c] = fma(a, v.v[c], acc.v[c]);
-}
-
 // Slab slot of texel i: threads of a line touch every other texel, so the lowest
 // bit is mixed with the one that would bring two of them onto one bank.  Texels 2j
 // and 2j + 1 may swap places, so a slab holds an even number of entries.

@@ -8,12 +8,16 @@
 //   boundary relax   IterativeSolvers.inl:414-430   x_B = BB^-1 (rhs_B - BD x)
 //   boundary residual IterativeSolvers.inl:549-555  r_B = rhs_B - BD x - BB x_B
 //   raw operator     IterativeSolvers.inl:881-950   y = A x (MultiplyBySystemMatrix_NoReciprocals)
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <type_traits>
 
 #include "vcycle.cuh"
 #include "vcycle_kernels.h"
 #include "vcycle_ops.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace gdtp {
 namespace dev {
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(kGroupBlockMax, 1) k_gs_groups(const ColourRun
                                                                T* __restrict__ x, int KP, int G, int sweeps, int reverse) {
   grid_dependency_wait();
   grid_launch_dependents();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(32) unsigned char smem_raw[];
   T* xs = reinterpret_cast<T*>(smem_raw);
   const int* g = groups + 10 * blockIdx.x;
   const int lo = g[8], span = g[9];
@@ -418,141 +422,205 @@ __global__ void __launch_bounds__(256) k_prolong_add(const ProlongRun* __restric
 //                       x_S = s xs
 //   k_bs_back:          x_I = s (y - W_p xs),  W_p = Inv_p A_{I_p,S} (m x t_p)
 // The sparse row sums run on 8 lanes per row (group8_sum in vcycle_ops.cuh).
-// The dense products are memory-bound streams of the symmetric inverses,
-// stored row-major with rows padded to a multiple of 4: lane l of a warp reads
-// rows 4l..4l+3 of matrix row j with one vector load, so a warp reads
-// contiguous memory.  A block takes 128 rows of one matrix and a chunk of its
-// j range (8 warps interleave j); the chunks of a row group (blockIdx.y) write
-// partial sums and the last block to finish adds them in chunk order, so the
-// result does not depend on scheduling.  Chunking keeps the dependent-load
-// chain of each warp short on the small coarse levels.
+// The dense products stream the symmetric inverses, stored row-major with rows
+// padded to a multiple of 4: lane l of a warp reads rows 4l..4l+3 of matrix row j
+// with one vector load, so a warp reads contiguous memory.  The j range of a row
+// group (128 rows of one matrix) is cut into nch chunks, which keeps the
+// dependent-load chain of each warp short on the small levels (8 warps interleave
+// a chunk's j); partial sums are added warps first, then chunks, in order, so the
+// result does not depend on scheduling.
 // ----------------------------------------------------------------------------
 
-template <typename T, int W>
-__global__ void __launch_bounds__(256, 3) k_bs_dense(BoundaryDev<T> B, int mode, const T* __restrict__ rhs, T* __restrict__ x, int KP,
-                                                  int G) {
-  __shared__ T red[8][32][4 * W];
-  __shared__ Vec<T, W> vin[kBoundaryChunkMax];
-  __shared__ int lastFlag;
+// Chunks of one row group share a cluster of up to kBsClusterMax CTAs: CTA r takes
+// chunks r, r + CS, ..., one per group of 8 warps (blockDim / 256 groups, then the
+// next round), and the chunks' partial sums meet in distributed shared memory,
+// where each CTA adds, in chunk order, the rows it writes.
+// What bounds it: on every level but the finest a product is a few MB behind a chain
+// of latencies, so what is set-up data (task, first matrix rows, couplings) is
+// loaded before the dependency wait, and the chunks' sums no longer go through
+// global memory, fences and an arrival counter (the last CTA then read them back: two
+// more trips).  Per refinement step with the early loads of k_bs_prep and k_bs_back:
+// 256^2 torus 134 -> 124 us, 1024^2 genus-2 (one channel) 153 -> 144, 1024^2
+// icosphere 334 -> 314, 2048^2 672 -> 653, 15 right-hand sides 490 -> 434.
+// Shared memory: vin [groups][Q][chunk], red [groups][8][128 W], part [chunks of the
+// CTA][Q][128 W] (one chunk: unused).
+constexpr int kBsClusterMax = 8;
+constexpr size_t kBsDenseSmemMax = 200 * 1024;
+// Threads a CTA is compiled for: with the couplings in registers the separator
+// product (mode 1) spills at the 64 registers of 1024 threads
+template <typename T>
+constexpr int bs_dense_threads(int Q, int mode) { return sizeof(T) == 4 && Q == 1 ? (mode == 0 ? 1024 : 768) : 512; }
+template <typename T, int W, int Q, int mode>
+__global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(BoundaryDev<T> B, int nch, int clen0, T* __restrict__ x,
+                                                                     int KP) {
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int CS = gridDim.y, rank = blockIdx.y, groups = blockDim.x >> 8, grp = threadIdx.x >> 8, tg = threadIdx.x & 255;
+  constexpr int kRowVals = 128 * W;  // values of one channel group of the task's rows
+  Vec<T, W>* vin = reinterpret_cast<Vec<T, W>*>(smem_raw) + size_t(grp) * Q * clen0;
+  T* redAll = reinterpret_cast<T*>(reinterpret_cast<Vec<T, W>*>(smem_raw) + size_t(groups) * Q * clen0);
+  T* red = redAll + size_t(grp) * 8 * kRowVals;
+  T* part = redAll + size_t(groups) * 8 * kRowVals;
   // the block's task, its matrix and its rows of it are set-up data: read (and
   // the rows prefetched into L2) before waiting for the previous launch
   const int4 task = (mode == 0 ? B.subTasks : B.schurTasks)[blockIdx.x];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rq = task.y + lane;
+  const int warp = tg >> 5, lane = tg & 31, rq = task.y + lane;
   const int r0 = mode == 0 ? B.subPtr[task.x] : 0;
   const int m = mode == 0 ? B.subPtr[task.x + 1] - r0 : B.nS, mp = (m + 3) & ~3;
   const T* M = mode == 0 ? B.inv + B.invOff[task.x] : B.sinv;
-  const int nch = gridDim.y, chunk = blockIdx.y;
-  const int clen = (m + nch - 1) / nch, j0 = min(m, chunk * clen), j1 = min(m, j0 + clen);
+  const int clen = (m + nch - 1) / nch;
+  const int c0 = blockIdx.z * Q * W;  // first channel
+  if (blockIdx.z == 0) {
+    // rows of this group's chunks, columns 4 task.y .. 4 task.y + 127 (clipped to the padded row)
+    const int col0 = 4 * task.y, cols = max(0, min(mp - col0, 128));
+    if (lane * 32 < cols * (int)sizeof(T))
+      for (int ch = rank + CS * grp; ch < nch; ch += CS * groups) {
+        const int j0 = min(m, ch * clen), j1 = min(m, j0 + clen);
+        for (int j = j0 + warp; j < j1; j += 8)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(M + (long long)j * mp + col0) + lane * 32));
+      }
+  }
+  // the first rows of this warp's first chunk into registers; mode 1: the first
+  // row's couplings
+  const bool active = 4 * rq < m;
+  constexpr int kPre = W == 1 ? 4 : sizeof(T) == 4 ? 2 : 1;
+  Quad<T> pre[kPre];
+  T aw[2];
+  int ac[2], ae0 = 0, ae1 = 0;
   {
-    // rows j0..j1 of columns 4 task.y .. 4 task.y + 127 (clipped to the padded row)
-    const int c0 = 4 * task.y, cols = max(0, min(mp - c0, 128));
-    if (cols > 0)
-      for (int j = j0 + warp; j < j1; j += 8)
-        if (lane * 32 < cols * (int)sizeof(T)) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(M + (long long)j * mp + c0) + lane * 32));
+    const int ch = rank + CS * grp, j0 = min(m, ch * clen), j1 = min(m, j0 + clen);
+    if (active)
+#pragma unroll
+      for (int u = 0; u < kPre; u++)
+        if (j0 + warp + 8 * u < j1) pre[u] = *reinterpret_cast<const Quad<T>*>(M + (long long)(j0 + warp + 8 * u) * mp + 4 * rq);
+    if (mode == 1 && j0 + (tg >> 3) < j1) {
+      ae0 = B.asiPtr[j0 + (tg >> 3)] + (tg & 7);
+      ae1 = B.asiPtr[j0 + (tg >> 3) + 1];
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        if (ae0 + 8 * u < ae1) {
+          aw[u] = B.asiVal[ae0 + 8 * u];
+          ac[u] = B.asiCol[ae0 + 8 * u];
+        }
+    }
   }
   grid_dependency_wait();
   grid_launch_dependents();
-  const bool active = 4 * rq < m;
-  T* part = mode == 0 ? B.subPart : B.schurPart;
-  for (int q = 0; q < G; q++) {
-    const int off = q * W;
-    // prologue: the chunk's input vector (mode 0: the scaled right-hand side
-    // from k_bs_prep; mode 1: minus the coupling to the interior solution)
+  const int rounds = (nch - rank + CS * groups - 1) / (CS * groups);  // the same for every group of the CTA
+  for (int rd = 0; rd < rounds; rd++) {
+    const int ch = rank + CS * (grp + groups * rd);
+    const bool has = ch < nch;
+    const int j0 = has ? min(m, ch * clen) : 0, j1 = has ? min(m, j0 + clen) : 0;
+    // the chunk's input vector (mode 0: the scaled right-hand side from k_bs_prep;
+    // mode 1: minus the coupling to the interior solution)
     if (mode == 0) {
-      for (int j = j0 + (int)threadIdx.x; j < j1; j += blockDim.x)
-        vin[j - j0] = vload<T, W>(B.rhat + (long long)(r0 + j) * KP + off);
-    } else {
-      const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3;
-      for (int jb = j0; jb < j1; jb += 32) {  // 32 groups of 8 lanes
-        const int j = jb + grp;
-        const Vec<T, W> v = bs_schur_input_group<T, W, LoadDefault>(B, j, j < j1, KP, off, lane8);
-        if (j < j1 && lane8 == 0) vin[j - j0] = v;
+      for (int i = tg; i < (j1 - j0) * Q; i += 256) {
+        const int j = Q == 1 ? i : i / Q, q = Q == 1 ? 0 : i - j * Q;
+        vin[q * clen0 + j] = vload<T, W>(B.rhat + (long long)(r0 + j0 + j) * KP + c0 + q * W);
       }
+    } else {
+      const int lane8 = tg & 7, row = tg >> 3;
+      for (int q = 0; q < Q; q++)
+        for (int jb = j0; jb < j1; jb += 32) {  // 32 groups of 8 lanes
+          const int j = jb + row;
+          Vec<T, W> v;
+          if (rd == 0 && jb == j0) {
+            // bs_schur_input_group's sums from the couplings loaded above
+            Vec<T, W> sum, y[2], r;
+#pragma unroll
+            for (int c = 0; c < W; c++) sum.v[c] = 0;
+            if (j < j1 && lane8 == 0) r = vload<T, W>(B.rhat + (long long)(B.nI + j) * KP + c0 + q * W);
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+              if (ae0 + 8 * u < ae1) y[u] = vload<T, W>(B.y + (long long)ac[u] * KP + c0 + q * W);
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+              if (ae0 + 8 * u < ae1) fma_to(sum, aw[u], y[u]);
+            for (int e = ae0 + 16; e < ae1; e += 8) fma_to(sum, B.asiVal[e], vload<T, W>(B.y + (long long)B.asiCol[e] * KP + c0 + q * W));
+            sum = group8_sum(sum);
+#pragma unroll
+            for (int c = 0; c < W; c++) v.v[c] = r.v[c] - sum.v[c];
+          } else {
+            v = bs_schur_input_group<T, W, LoadDefault>(B, j, j < j1, KP, c0 + q * W, lane8);
+          }
+          if (j < j1 && lane8 == 0) vin[q * clen0 + j - j0] = v;
+        }
     }
     __syncthreads();
-    T acc[4][W];
+    T acc[4][Q * W];
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-      for (int c = 0; c < W; c++) acc[a][c] = 0;
+      for (int c = 0; c < Q * W; c++) acc[a][c] = 0;
     if (active) {
-#pragma unroll 8
-      for (int j = j0 + warp; j < j1; j += 8) {
-        const Quad<T> mq = *reinterpret_cast<const Quad<T>*>(M + (long long)j * mp + 4 * rq);
-        const Vec<T, W> v = vin[j - j0];
+      auto add = [&](const Quad<T>& mq, int j) {
 #pragma unroll
-        for (int a = 0; a < 4; a++)
+        for (int q = 0; q < Q; q++) {
+          const Vec<T, W> v = vin[q * clen0 + j - j0];
 #pragma unroll
-          for (int c = 0; c < W; c++) acc[a][c] += mq.v[a] * v.v[c];
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < W; c++) acc[a][q * W + c] = fma(mq.v[a], v.v[c], acc[a][q * W + c]);
+        }
+      };
+      int j = j0 + warp;
+      if (rd == 0) {
+#pragma unroll
+        for (int u = 0; u < kPre; u++)
+          if (j + 8 * u < j1) add(pre[u], j + 8 * u);
+        j += 8 * kPre;
       }
+      constexpr int kAhead = sizeof(T) == 4 ? 4 : 6;
+#pragma unroll kAhead
+      for (; j < j1; j += 8) add(*reinterpret_cast<const Quad<T>*>(M + (long long)j * mp + 4 * rq), j);
     }
+    const int slot = grp + groups * rd;  // chunk ch = rank + CS slot
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int q = 0; q < Q; q++) {
+      if (q) __syncthreads();
 #pragma unroll
-      for (int c = 0; c < W; c++) red[warp][lane][a * W + c] = acc[a][c];
-    __syncthreads();
-    if (warp == 0 && active) {
+      for (int a = 0; a < 4; a++)
 #pragma unroll
-      for (int a = 0; a < 4; a++) {
-        const int row = 4 * rq + a;
-        if (row >= m) continue;
-        Vec<T, W> sum;
+        for (int c = 0; c < W; c++) red[warp * kRowVals + (4 * lane + a) * W + c] = acc[a][q * W + c];
+      __syncthreads();
+      for (int o = tg; o < kRowVals; o += 256) {
+        T v = 0;
 #pragma unroll
-        for (int c = 0; c < W; c++) {
-          T v = 0;
-          for (int w = 0; w < 8; w++) v += red[w][lane][a * W + c];
-          sum.v[c] = v;
-        }
-        if (nch > 1) {
-          vstore<T, W>(part + (((long long)blockIdx.x * nch + chunk) * 128 + 4 * lane + a) * KP + off, sum);
-        } else if (mode == 0) {
-          vstore<T, W>(B.y + (long long)(r0 + row) * KP + off, sum);
-        } else {
-          vstore<T, W>(B.xs + (long long)row * KP + off, sum);
-          const T sc = B.scale[B.nI + row];
-#pragma unroll
-          for (int c = 0; c < W; c++) sum.v[c] *= sc;
-          vstore<T, W>(x + (long long)B.posGlobal[B.nI + row] * KP + off, sum);
-        }
+        for (int w = 0; w < 8; w++) v += red[w * kRowVals + o];
+        if (has) part[(size_t(slot) * Q + q) * kRowVals + o] = v;
       }
     }
     __syncthreads();
   }
-  if (nch == 1) return;
-  // the last chunk of this row group to finish adds the partials in chunk order
-  __threadfence();
-  __syncthreads();
-  int* counter = (mode == 0 ? B.subCount : B.schurCount) + blockIdx.x;
-  if (threadIdx.x == 0) {
-    const int prev = atomicAdd(counter, 1);
-    lastFlag = prev == nch - 1;
-    if (lastFlag) *counter = 0;  // ready for the next launch
-  }
-  __syncthreads();
-  if (!lastFlag) return;
-  __threadfence();
-  for (int it = threadIdx.x; it < 128 * G; it += blockDim.x) {
-    const int rt = it / G, q = it - rt * G, row = 4 * task.y + rt, off = q * W;
+  // the chunks in order; CTA r writes every CS-th slice of the rows
+  if (CS > 1) cluster.sync();
+  for (int i = rank * blockDim.x + threadIdx.x; i < Q * kRowVals; i += CS * blockDim.x) {
+    const int q = i / kRowVals, o = i - q * kRowVals, rt = o / W, c = o - rt * W, row = 4 * task.y + rt;
     if (row >= m) continue;
-    Vec<T, W> sum;
-#pragma unroll
-    for (int c = 0; c < W; c++) sum.v[c] = 0;
-#pragma unroll 4
-    for (int ch = 0; ch < nch; ch++) {
-      const T* src = part + (((long long)blockIdx.x * nch + ch) * 128 + rt) * KP + off;
-#pragma unroll
-      for (int c = 0; c < W; c++) sum.v[c] += __ldcg(src + c);
-    }
-    if (mode == 0) {
-      vstore<T, W>(B.y + (long long)(r0 + row) * KP + off, sum);
+    T sum;
+    if (nch == 1) {
+      sum = part[i];
     } else {
-      vstore<T, W>(B.xs + (long long)row * KP + off, sum);
-      const T sc = B.scale[B.nI + row];
+      sum = 0;
+      for (int s = 0; s * CS < nch; s++) {
+        T v[kBsClusterMax];
 #pragma unroll
-      for (int c = 0; c < W; c++) sum.v[c] *= sc;
-      vstore<T, W>(x + (long long)B.posGlobal[B.nI + row] * KP + off, sum);
+        for (int r = 0; r < kBsClusterMax; r++)
+          if (r < CS && s * CS + r < nch) v[r] = cluster.map_shared_rank(part, r)[(size_t(s) * Q + q) * kRowVals + o];
+#pragma unroll
+        for (int r = 0; r < kBsClusterMax; r++)
+          if (r < CS && s * CS + r < nch) sum += v[r];
+      }
+    }
+    const int ch = c0 + q * W + c;
+    if (mode == 0) {
+      B.y[(long long)(r0 + row) * KP + ch] = sum;
+    } else {
+      B.xs[(long long)row * KP + ch] = sum;
+      x[(long long)B.posGlobal[B.nI + row] * KP + ch] = sum * B.scale[B.nI + row];
     }
   }
+  if (CS > 1) cluster.sync();  // the others may still read this CTA's partial sums
 }
 
 // x_I = s (y - W_p xs[touch_p]) for every interior position (W_p column-major,
@@ -587,14 +655,40 @@ __global__ void __launch_bounds__(256) k_bs_back(BoundaryDev<T> B, T* __restrict
       g = B.posGlobal[i];
     }
   }
+  // the first columns of this lane's part of the row (set-up data)
+  constexpr int kAhead = 4;
+  T w[kAhead];
+  int col[kAhead];
+#pragma unroll
+  for (int u = 0; u < kAhead; u++) {
+    const int e = e0 + lane8 + 8 * u;
+    if (e < e1) {
+      w[u] = Wp[(long long)(e - e0) * m];
+      col[u] = B.touch[e];
+    }
+  }
   grid_dependency_wait();
   grid_launch_dependents();
   if (valid && lane8 == 0 && !yEarly) yv = vload<T, W>(B.y + i * KP + off);
   Vec<T, W> acc;
 #pragma unroll
   for (int c = 0; c < W; c++) acc.v[c] = 0;
-  if (valid)
-    for (int e = e0 + lane8; e < e1; e += 8) axpy(acc, Wp[(long long)(e - e0) * m], vload<T, W>(B.xs + (long long)B.touch[e] * KP + off));
+  for (int e = e0 + lane8; e < e1; e += 8 * kAhead) {
+    Vec<T, W> v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+      if (e + 8 * u < e1) v[u] = vload<T, W>(B.xs + (long long)col[u] * KP + off);
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+      if (e + 8 * u < e1) {
+        fma_to(acc, w[u], v[u]);
+        const int en = e + 8 * (u + kAhead);
+        if (en < e1) {
+          w[u] = Wp[(long long)(en - e0) * m];
+          col[u] = B.touch[en];
+        }
+      }
+  }
   acc = group8_sum(acc);
   if (valid && lane8 == 0) {
 #pragma unroll
@@ -629,13 +723,30 @@ __global__ void __launch_bounds__(256) k_bs_prep(BoundaryDev<T> B, const T* __re
       if (rhsEarly) r = vload<T, W>(rhs + (long long)g * KP + off);
     }
   }
+  // this lane's first entries of the row (set-up data)
+  constexpr int kAhead = 2;
+  T w[kAhead];
+  int col[kAhead];
+#pragma unroll
+  for (int u = 0; u < kAhead; u++) {
+    const int e = e0 + lane8 + 8 * u;
+    if (e < e1) {
+      w[u] = B.bdVal[e];
+      col[u] = B.bdCol[e];
+    }
+  }
   grid_dependency_wait();
   grid_launch_dependents();
-  Vec<T, W> acc;
+  Vec<T, W> acc, v[kAhead];
 #pragma unroll
   for (int c = 0; c < W; c++) acc.v[c] = 0;
-  if (valid)
-    for (int e = e0 + lane8; e < e1; e += 8) axpy(acc, B.bdVal[e], vload<T, W>(x + (long long)B.bdCol[e] * KP + off));
+#pragma unroll
+  for (int u = 0; u < kAhead; u++)
+    if (e0 + lane8 + 8 * u < e1) v[u] = vload<T, W>(x + (long long)col[u] * KP + off);
+#pragma unroll
+  for (int u = 0; u < kAhead; u++)
+    if (e0 + lane8 + 8 * u < e1) fma_to(acc, w[u], v[u]);
+  for (int e = e0 + lane8 + 8 * kAhead; e < e1; e += 8) fma_to(acc, B.bdVal[e], vload<T, W>(x + (long long)B.bdCol[e] * KP + off));
   acc = group8_sum(acc);
   if (valid && lane8 == 0) {
     if (!rhsEarly) r = vload<T, W>(rhs + (long long)g * KP + off);
@@ -1206,13 +1317,61 @@ void launch_prolong_add(const ProlongRun* runs, int nRuns, const T* coarse, T* f
   const int G = KP / W;
   launch(k_prolong_add<T, W>, dim3(nblk((long long)nRuns * 32 * G)), s, runs, nRuns, coarse, fine, KP, G);
 }
+// One dense product of the boundary solve (mode 0: subdomains, 1: separator).
+// Channel groups per CTA: as many as the registers hold (a matrix value read once
+// for them); warp groups per CTA: one per chunk while the registers last.
+template <typename T, int W, int Q, int mode>
+static bool launch_bs_dense_q(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) {
+  const int nch = mode == 0 ? B.subChunks : B.schurChunks, tasks = mode == 0 ? B.nSubTasks : B.nSchurTasks;
+  const int CS = std::min(kBsClusterMax, nch), slots = (nch + CS - 1) / CS;
+  const int groups = std::min(bs_dense_threads<T>(Q, mode) / 256, slots);
+  const int clen = ((mode == 0 ? kBoundaryChunkMax : B.nS) + nch - 1) / nch;
+  const size_t smem = size_t(groups) * Q * clen * sizeof(Vec<T, W>) + size_t(groups) * 8 * 128 * W * sizeof(T) +
+                      size_t(slots) * Q * 128 * W * sizeof(T);
+  if (smem > kBsDenseSmemMax) return false;
+  static std::atomic<int> attr[kMaxDevices];
+  static const bool init = [] {
+    for (auto& a : attr) a.store(kUnset);
+    return true;
+  }();
+  (void)init;
+  if (!per_device_once(attr, [] {
+        return cudaFuncSetAttribute(k_bs_dense<T, W, Q, mode>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBsDenseSmemMax)) == cudaSuccess
+                   ? 1
+                   : 0;
+      }))
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(tasks), unsigned(CS), unsigned(KP / W / Q));
+  cfg.blockDim = dim3(unsigned(256 * groups));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {1, unsigned(CS), 1};
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = g_programmatic ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k_bs_dense<T, W, Q, mode>, B, nch, clen, x, KP) == cudaSuccess;
+}
+template <typename T, int W, int mode>
+static void launch_bs_dense(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) {
+  if constexpr (W > 1) {
+    const int G = KP / W;
+    if constexpr (sizeof(T) == 4)
+      if (G % 4 == 0 && launch_bs_dense_q<T, W, 4, mode>(B, x, KP, s)) return;
+    if (G % 2 == 0 && launch_bs_dense_q<T, W, 2, mode>(B, x, KP, s)) return;
+  }
+  launch_bs_dense_q<T, W, 1, mode>(B, x, KP, s);
+}
 template <typename T, int W>
 void launch_boundary_solve(const BoundaryDev<T>& B, const T* rhs, T* x, int KP, cudaStream_t s, bool rhsEarly) {
   if (B.nb == 0) return;
   const int G = KP / W;
   launch(k_bs_prep<T, W>, dim3(nblk((long long)B.nb * G * 8)), s, B, rhs, x, KP, G, rhsEarly ? 1 : 0);
-  if (B.nSubTasks > 0) launch(k_bs_dense<T, W>, dim3(B.nSubTasks, B.subChunks), s, B, 0, rhs, x, KP, G);
-  if (B.nS > 0) launch(k_bs_dense<T, W>, dim3(B.nSchurTasks, B.schurChunks), s, B, 1, rhs, x, KP, G);
+  if (B.nSubTasks > 0) launch_bs_dense<T, W, 0>(B, x, KP, s);
+  if (B.nS > 0) launch_bs_dense<T, W, 1>(B, x, KP, s);
   // y comes from the subdomain product: read early only when the separator
   // product sits between the two launches
   if (B.nI > 0) launch(k_bs_back<T, W>, dim3(nblk((long long)B.nI * G * 8)), s, B, x, KP, G, B.nS > 0 ? 1 : 0);

@@ -69,9 +69,8 @@ struct BoundaryDev {
   const int *touchPtr = nullptr, *touch = nullptr; // per subdomain: separator columns
   const long long* wOff = nullptr;
   const T* wt = nullptr;                // Inv_p A_{I_p,touch}, column-major m x t_p
-  T *y = nullptr, *xs = nullptr, *subPart = nullptr, *schurPart = nullptr;  // work
+  T *y = nullptr, *xs = nullptr;        // work
   T* rhat = nullptr;                    // scaled right-hand side s (rhs - BD x) per position (work)
-  int *subCount = nullptr, *schurCount = nullptr;                            // chunk arrival counters (zero between launches)
 };
 
 // One multigrid level on the device, value type T (plain pointers and counts;

@@ -77,6 +77,15 @@ __device__ __forceinline__ void axpy(Vec<T, W>& acc, T a, const Vec<T, W>& v) {
   for (int c = 0; c < W; c++) acc.v[c] += a * v.v[c];
 }
 
+// acc += a v as fused multiply-adds, written out: left to contraction, the first
+// two terms (of a sum that starts at 0) may be fused the other way round where the
+// compiler sees both
+template <typename T, int W>
+__device__ __forceinline__ void fma_to(Vec<T, W>& acc, T a, const Vec<T, W>& v) {
+#pragma unroll
+  for (int c = 0; c < W; c++) acc.v[c] = fma(a, v.v[c], acc.v[c]);
+}
+
 // Gauss-Seidel update of one colour-run texel: x = rhs*c4 - sum_{k!=4} c_k x_k
 // (IterativeSolvers.inl:449-463).  Items: runs x 32 x G.
 template <typename T, int W, typename LD>

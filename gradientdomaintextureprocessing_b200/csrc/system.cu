@@ -1097,8 +1097,6 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
       B.subTasks = A.upload(tasks);
       B.nSubTasks = (int)tasks.size();
       B.subChunks = chunks_for(B.nSubTasks, maxM, 1);
-      B.subPart = static_cast<T*>(A.alloc(size_t(std::max(1, B.nSubTasks)) * B.subChunks * 128 * KP * sizeof(T)));
-      B.subCount = A.zeros<int>(std::max(1, B.nSubTasks));
       // separator Schur complement inverse, same layout
       if (bs.nS > 0) {
         const int nS = bs.nS, nSp = (nS + 3) & ~3;
@@ -1115,8 +1113,6 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
         B.schurTasks = A.upload(st);
         B.nSchurTasks = (int)st.size();
         B.schurChunks = chunks_for(B.nSchurTasks, nS, (nS + dev::kBoundaryChunkMax - 1) / dev::kBoundaryChunkMax);
-        B.schurPart = static_cast<T*>(A.alloc(size_t(B.nSchurTasks) * B.schurChunks * 128 * KP * sizeof(T)));
-        B.schurCount = A.zeros<int>(B.nSchurTasks);
       }
       // back substitution: W_p column-major with its separator columns
       std::vector<long long> wOff(bs.wOff.begin(), bs.wOff.end());
@@ -1248,12 +1244,6 @@ bool DeviceSystem::derive_multigrid(const Multigrid<T>& base, Multigrid<T>& mg, 
     if (D.nTiles > 0) D.tileSync = A.zeros<int>(2 + size_t(D.nTiles));
     dev::BoundaryDev<T>& B = D.B;
     if (B.nb == 0) continue;
-    B.subPart = static_cast<T*>(A.alloc(size_t(std::max(1, B.nSubTasks)) * B.subChunks * 128 * KP * sizeof(T)));
-    B.subCount = A.zeros<int>(std::max(1, B.nSubTasks));
-    if (B.nS > 0) {
-      B.schurPart = static_cast<T*>(A.alloc(size_t(B.nSchurTasks) * B.schurChunks * 128 * KP * sizeof(T)));
-      B.schurCount = A.zeros<int>(B.nSchurTasks);
-    }
     B.y = static_cast<T*>(A.alloc(size_t(std::max(1, B.nI)) * KP * sizeof(T)));
     B.xs = static_cast<T*>(A.alloc(size_t(std::max(1, B.nS)) * KP * sizeof(T)));
     B.rhat = static_cast<T*>(A.alloc(size_t(std::max(1, B.nb)) * KP * sizeof(T)));

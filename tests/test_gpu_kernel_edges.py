@@ -124,3 +124,32 @@ def test_cluster_chart_smoother_matches_the_launches(atlas, k, precision):
             for q, v in sweeps.items():
                 atlas.set(q, v)
         np.testing.assert_array_equal(got[1], got[0])
+
+
+@pytest.mark.parametrize("k", [1, 3, 5, 16])
+@pytest.mark.parametrize("knobs", [{"bs_blocks_per_sm": 1}, {"bs_blocks_per_sm": 16}, {"max_block": 64}, {"max_block": 17},
+                                   {"dense_boundary_max": 8192}])
+def test_boundary_products_at_every_chunking(ico, k, knobs):
+    """Chunks per row group from 1 to the largest, ragged row groups, one whole
+    block: the boundary products of the launches against those of the coarse-level
+    cluster kernel (the same chunks, added in the same order)."""
+    b, _ = vectors(ico.n, k)
+    old = {q: ico.get(q) for q in knobs}
+    out = {}
+    try:
+        for q, v in knobs.items():
+            ico.set(q, v)
+        for precision in ("mixed", "fp64"):
+            ico.update(2e-3, 1.0)
+            ico.set("max_block", ico.get("max_block"))  # lays the boundary solver out for the knobs
+            for cluster in (0, 1 << 30):
+                ico.set("cluster_texels", cluster)
+                out[precision, cluster] = ico.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+    finally:
+        ico.set("cluster_texels", 0)
+        for q, v in old.items():
+            ico.set(q, v)
+        ico.set("max_block", ico.get("max_block"))
+        ico.update(1e-3, 1.0)
+    for precision in ("mixed", "fp64"):
+        np.testing.assert_array_equal(out[precision, 0], out[precision, 1 << 30])
