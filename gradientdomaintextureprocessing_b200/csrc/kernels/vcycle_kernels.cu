@@ -433,17 +433,22 @@ __global__ void __launch_bounds__(256) k_prolong_add(const ProlongRun* __restric
 
 // Chunks of one row group share a cluster of up to kBsClusterMax CTAs: CTA r takes
 // chunks r, r + CS, ..., one per group of 8 warps (blockDim / 256 groups, then the
-// next round), and the chunks' partial sums meet in distributed shared memory,
-// where each CTA adds, in chunk order, the rows it writes.
+// next round), and stores each partial sum into the shared memory of the CTA that
+// will write the row (distributed shared memory); after one cluster barrier every
+// CTA adds its rows' chunks, in order, from its own.
 // What bounds it: on every level but the finest a product is a few MB behind a chain
 // of latencies, so what is set-up data (task, first matrix rows, couplings) is
 // loaded before the dependency wait, and the chunks' sums no longer go through
 // global memory, fences and an arrival counter (the last CTA then read them back: two
 // more trips).  Per refinement step with the early loads of k_bs_prep and k_bs_back:
-// 256^2 torus 134 -> 124 us, 1024^2 genus-2 (one channel) 153 -> 144, 1024^2
-// icosphere 334 -> 314, 2048^2 672 -> 653, 15 right-hand sides 490 -> 434.
-// Shared memory: vin [groups][Q][chunk], red [groups][8][128 W], part [chunks of the
-// CTA][Q][128 W] (one chunk: unused).
+// 256^2 torus 134 -> 124 us, 1024^2 genus-2 (one channel) 153 -> 149, 1024^2
+// icosphere 334 -> 315, 2048^2 672 -> 655, 15 right-hand sides 490 -> 435.  Storing
+// the sums where they are added, instead of reading them there (a trip and a second
+// barrier), and accumulators without bank conflicts (16-way before): 120, 146, 310,
+// 653 and 414 us.
+// Shared memory: vin [groups][Q][chunk], red [groups][8][128 W], recv [chunks][values
+// this CTA writes].  A row group's values are numbered (row % 4, row / 4, channel), so
+// that a warp's accumulators go to shared memory without bank conflicts.
 constexpr int kBsClusterMax = 8;
 constexpr size_t kBsDenseSmemMax = 200 * 1024;
 // Threads a CTA is compiled for: with the couplings in registers the separator
@@ -460,7 +465,11 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
   Vec<T, W>* vin = reinterpret_cast<Vec<T, W>*>(smem_raw) + size_t(grp) * Q * clen0;
   T* redAll = reinterpret_cast<T*>(reinterpret_cast<Vec<T, W>*>(smem_raw) + size_t(groups) * Q * clen0);
   T* red = redAll + size_t(grp) * 8 * kRowVals;
-  T* part = redAll + size_t(groups) * 8 * kRowVals;
+  T* recv = redAll + size_t(groups) * 8 * kRowVals;
+  const int share = (Q * kRowVals + CS - 1) / CS;  // CTA r writes values [r share, (r + 1) share)
+  // the CTAs of the cluster are running once this barrier's wait returns (before
+  // the first remote store)
+  if (CS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   // the block's task, its matrix and its rows of it are set-up data: read (and
   // the rows prefetched into L2) before waiting for the previous launch
   const int4 task = (mode == 0 ? B.subTasks : B.schurTasks)[blockIdx.x];
@@ -485,8 +494,9 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
   const bool active = 4 * rq < m;
   constexpr int kPre = W == 1 ? 4 : sizeof(T) == 4 ? 2 : 1;
   Quad<T> pre[kPre];
-  T aw[2];
-  int ac[2], ae0 = 0, ae1 = 0;
+  constexpr int kPreA = W == 1 ? 4 : 3;
+  T aw[kPreA];
+  int ac[kPreA], ae0 = 0, ae1 = 0;
   {
     const int ch = rank + CS * grp, j0 = min(m, ch * clen), j1 = min(m, j0 + clen);
     if (active)
@@ -497,7 +507,7 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
       ae0 = B.asiPtr[j0 + (tg >> 3)] + (tg & 7);
       ae1 = B.asiPtr[j0 + (tg >> 3) + 1];
 #pragma unroll
-      for (int u = 0; u < 2; u++)
+      for (int u = 0; u < kPreA; u++)
         if (ae0 + 8 * u < ae1) {
           aw[u] = B.asiVal[ae0 + 8 * u];
           ac[u] = B.asiCol[ae0 + 8 * u];
@@ -526,17 +536,17 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
           Vec<T, W> v;
           if (rd == 0 && jb == j0) {
             // bs_schur_input_group's sums from the couplings loaded above
-            Vec<T, W> sum, y[2], r;
+            Vec<T, W> sum, y[kPreA], r;
 #pragma unroll
             for (int c = 0; c < W; c++) sum.v[c] = 0;
             if (j < j1 && lane8 == 0) r = vload<T, W>(B.rhat + (long long)(B.nI + j) * KP + c0 + q * W);
 #pragma unroll
-            for (int u = 0; u < 2; u++)
+            for (int u = 0; u < kPreA; u++)
               if (ae0 + 8 * u < ae1) y[u] = vload<T, W>(B.y + (long long)ac[u] * KP + c0 + q * W);
 #pragma unroll
-            for (int u = 0; u < 2; u++)
+            for (int u = 0; u < kPreA; u++)
               if (ae0 + 8 * u < ae1) fma_to(sum, aw[u], y[u]);
-            for (int e = ae0 + 16; e < ae1; e += 8) fma_to(sum, B.asiVal[e], vload<T, W>(B.y + (long long)B.asiCol[e] * KP + c0 + q * W));
+            for (int e = ae0 + 8 * kPreA; e < ae1; e += 8) fma_to(sum, B.asiVal[e], vload<T, W>(B.y + (long long)B.asiCol[e] * KP + c0 + q * W));
             sum = group8_sum(sum);
 #pragma unroll
             for (int c = 0; c < W; c++) v.v[c] = r.v[c] - sum.v[c];
@@ -574,43 +584,46 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
 #pragma unroll kAhead
       for (; j < j1; j += 8) add(*reinterpret_cast<const Quad<T>*>(M + (long long)j * mp + 4 * rq), j);
     }
-    const int slot = grp + groups * rd;  // chunk ch = rank + CS slot
+    if (CS > 1 && rd == 0) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       if (q) __syncthreads();
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int a = 0; a < 4; a++) {
+        Vec<T, W> v;
 #pragma unroll
-        for (int c = 0; c < W; c++) red[warp * kRowVals + (4 * lane + a) * W + c] = acc[a][q * W + c];
+        for (int c = 0; c < W; c++) v.v[c] = acc[a][q * W + c];
+        vstore<T, W>(red + warp * kRowVals + (a * 32 + lane) * W, v);
+      }
       __syncthreads();
       for (int o = tg; o < kRowVals; o += 256) {
         T v = 0;
 #pragma unroll
         for (int w = 0; w < 8; w++) v += red[w * kRowVals + o];
-        if (has) part[(size_t(slot) * Q + q) * kRowVals + o] = v;
+        if (has) {
+          const int i = q * kRowVals + o, r = i / share;
+          T* dst = CS > 1 ? cluster.map_shared_rank(recv, r) : recv;
+          dst[(size_t)ch * share + (i - r * share)] = v;
+        }
       }
     }
     __syncthreads();
   }
-  // the chunks in order; CTA r writes every CS-th slice of the rows
-  if (CS > 1) cluster.sync();
-  for (int i = rank * blockDim.x + threadIdx.x; i < Q * kRowVals; i += CS * blockDim.x) {
-    const int q = i / kRowVals, o = i - q * kRowVals, rt = o / W, c = o - rt * W, row = 4 * task.y + rt;
+  // the chunks of this CTA's values, in order
+  if (CS > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  for (int j = threadIdx.x; j < share; j += blockDim.x) {
+    const int i = rank * share + j;
+    if (i >= Q * kRowVals) break;
+    const int q = i / kRowVals, o = i - q * kRowVals, rw = o / W, c = o - rw * W, row = 4 * (task.y + (rw & 31)) + (rw >> 5);
     if (row >= m) continue;
-    T sum;
-    if (nch == 1) {
-      sum = part[i];
-    } else {
-      sum = 0;
-      for (int s = 0; s * CS < nch; s++) {
-        T v[kBsClusterMax];
-#pragma unroll
-        for (int r = 0; r < kBsClusterMax; r++)
-          if (r < CS && s * CS + r < nch) v[r] = cluster.map_shared_rank(part, r)[(size_t(s) * Q + q) * kRowVals + o];
-#pragma unroll
-        for (int r = 0; r < kBsClusterMax; r++)
-          if (r < CS && s * CS + r < nch) sum += v[r];
-      }
+    T sum = recv[j];
+    if (nch > 1) {
+      sum = T(0) + sum;
+#pragma unroll 4
+      for (int k = 1; k < nch; k++) sum += recv[(size_t)k * share + j];
     }
     const int ch = c0 + q * W + c;
     if (mode == 0) {
@@ -620,7 +633,6 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
       x[(long long)B.posGlobal[B.nI + row] * KP + ch] = sum * B.scale[B.nI + row];
     }
   }
-  if (CS > 1) cluster.sync();  // the others may still read this CTA's partial sums
 }
 
 // x_I = s (y - W_p xs[touch_p]) for every interior position (W_p column-major,
@@ -1327,7 +1339,7 @@ static bool launch_bs_dense_q(const BoundaryDev<T>& B, T* x, int KP, cudaStream_
   const int groups = std::min(bs_dense_threads<T>(Q, mode) / 256, slots);
   const int clen = ((mode == 0 ? kBoundaryChunkMax : B.nS) + nch - 1) / nch;
   const size_t smem = size_t(groups) * Q * clen * sizeof(Vec<T, W>) + size_t(groups) * 8 * 128 * W * sizeof(T) +
-                      size_t(slots) * Q * 128 * W * sizeof(T);
+                      size_t(nch) * ((Q * 128 * W + CS - 1) / CS) * sizeof(T);
   if (smem > kBsDenseSmemMax) return false;
   static std::atomic<int> attr[kMaxDevices];
   static const bool init = [] {
