@@ -41,7 +41,9 @@ struct ProlongRun {      // fine texels f0 + m, m < len, line position i0 + m
 };
 
 template <typename T, int W>
-struct Vec;
+struct Vec {
+  T v[W];
+};
 template <>
 struct Vec<float, 1> {
   float v[1];

@@ -299,10 +299,24 @@ __global__ void __launch_bounds__(256) k_residual(const ColourRun* __restrict__ 
                                                   const int* __restrict__ bGlobal, int nB, const T* __restrict__ rhs,
                                                   const T* __restrict__ x, T* __restrict__ res, int KP, int G, int rhsEarly) {
   if ((int)blockIdx.x >= deepBlocks) {
+    const long long t = (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x;
+    if (G > 1) {  // several channel groups: a thread per row and group (row8_lanes)
+      grid_dependency_wait();
+      grid_launch_dependents();
+      residual_boundary_item<T, W, LoadDefault>(bPtr, bCol, bVal, bGlobal, nB, rhs, x, res, KP, G, t);
+      return;
+    }
+    // residual_boundary_item's sum on 8 lanes, its first entries loaded before the wait
+    const long long row = t >> 3;
+    const int lane8 = int(t & 7), off = 0;
+    const bool valid = row < nB;
+    const int g = valid ? bGlobal[row] : 0;
+    OrderedRow8<T, W, 2> entries(bCol, bVal, valid ? bPtr[row] : 0, valid ? bPtr[row + 1] : 0, lane8);
     grid_dependency_wait();
     grid_launch_dependents();
-    residual_boundary_item<T, W, LoadDefault>(bPtr, bCol, bVal, bGlobal, nB, rhs, x, res, KP, G,
-                                              (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x);
+    Vec<T, W> acc = vload<T, W>(rhs + (long long)g * KP + off);
+    entries.add_to(acc, true, bCol, bVal, lane8, [&](int c) { return vload<T, W>(x + (long long)c * KP + off); });
+    if (valid && lane8 == 0) vstore<T, W>(res + (long long)g * KP + off, acc);
     return;
   }
   // deep items (residual_deep_item's arithmetic, same order): the run and its
@@ -362,13 +376,32 @@ __global__ void __launch_bounds__(256) k_restrict(const RestrictRun* __restrict_
   // not touch the coarse level)
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < coarseVals; i += (long long)gridDim.x * blockDim.x)
     coarseX[i] = T(0);
+  if ((int)blockIdx.x < deepBlocks) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    restrict_deep_item<T, W, LoadDefault>(runs, nRuns, res, coarseRhs, KP, G, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+    return;
+  }
+  const long long t = (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x;
+  if (G > 1) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    restrict_boundary_item<T, W, LoadDefault>(rPtr, rCol, rVal, rOut, nB, res, coarseRhs, KP, G, t);
+    return;
+  }
+  // restrict_boundary_item's sum on 8 lanes, its first entries loaded before the wait
+  const long long row = t >> 3;
+  const int lane8 = int(t & 7), off = 0;
+  const bool valid = row < nB;
+  const int o = valid ? rOut[row] : 0;
+  OrderedRow8<T, W, 2> entries(rCol, rVal, valid ? rPtr[row] : 0, valid ? rPtr[row + 1] : 0, lane8);
   grid_dependency_wait();
   grid_launch_dependents();
-  if ((int)blockIdx.x < deepBlocks)
-    restrict_deep_item<T, W, LoadDefault>(runs, nRuns, res, coarseRhs, KP, G, (long long)blockIdx.x * blockDim.x + threadIdx.x);
-  else
-    restrict_boundary_item<T, W, LoadDefault>(rPtr, rCol, rVal, rOut, nB, res, coarseRhs, KP, G,
-                                              (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x);
+  Vec<T, W> acc;
+#pragma unroll
+  for (int k = 0; k < W; k++) acc.v[k] = 0;
+  entries.add_to(acc, false, rCol, rVal, lane8, [&](int c) { return vload<T, W>(res + (long long)c * KP + off); });
+  if (valid && lane8 == 0) vstore<T, W>(coarseRhs + (long long)o * KP + off, acc);
 }
 
 // ----------------------------------------------------------------------------
@@ -979,23 +1012,66 @@ __device__ __forceinline__ void block_partials(double (&ra)[4], double (&rb)[4],
 // (group q of G = KP/4 groups, or G = 1 for K = 1).  Per-block sums of res^2
 // and b^2 per channel go to `partials` for a deterministic norm reduction.
 // ----------------------------------------------------------------------------
+// KT: K (one channel group), or 0 for any K.
+template <int KT>
 __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restrict__ runs, int nRuns, const double* __restrict__ coef,
                                                       int planeStride, const int* __restrict__ bPtr, const int* __restrict__ bCol,
                                                       const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
                                                       const double* __restrict__ b, const double* __restrict__ x,
-                                                      double* __restrict__ out, int K, int G, int mode, double* __restrict__ partials,
+                                                      double* __restrict__ out, int Kany, int G, int mode, double* __restrict__ partials,
                                                       float* __restrict__ out32, int KP) {
+  const int K = KT ? KT : Kany;
+  constexpr int kCh = KT ? KT : 4;
   grid_dependency_wait();
   grid_launch_dependents();
-  // grid-stride over deep items (runs x 32 x G) then boundary items (rows x G);
-  // the stride is a multiple of G, so every thread keeps one channel group q
-  const long long nDeepItems = (long long)nRuns * 32 * G, nItems = nDeepItems + (long long)nB * G;
+  const long long nDeepItems = (long long)nRuns * 32 * G, nItems = nDeepItems + (KT ? 0 : (long long)nB * G);
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int q = int(t0 % G);
+  const int q = KT ? 0 : int(t0 % G);
   double rr[4] = {0, 0, 0, 0}, bb[4] = {0, 0, 0, 0};
+  // row g: its value from the sums, its share of the norms
+  auto finish = [&](int g, const double (&acc)[kCh]) {
+#pragma unroll
+    for (int ch = 0; ch < kCh; ch++) {
+      const int c = 4 * q + ch;
+      if (c >= K) continue;
+      const double bv = b ? b[(long long)g * K + c] : 0.0;
+      const double v = (mode == 0 || mode == 3) ? bv - acc[ch] : acc[ch];
+      if (out32) out32[(long long)g * KP + c] = float(v);
+      else out[(long long)g * K + c] = v;
+      rr[ch] += mode == 2 ? x[(long long)g * K + c] * v : v * v;  // mode 2: x . A x
+      bb[ch] += bv * bv;
+    }
+    if (out32)  // zero the padding channels of this group
+      for (int c = max(K, 4 * q); c < min(KP, 4 * q + 4); c++) out32[(long long)g * KP + c] = 0.f;
+  };
+  if constexpr (KT > 0) {
+    // boundary rows first, 8 lanes each (a chain of trips that the deep rows then
+    // hide), summed in the rows' order
+    const int lane8 = threadIdx.x & 7;
+    for (long long w0 = t0 >> 5; w0 * 4 < nB; w0 += stride >> 5) {
+      const long long row = w0 * 4 + ((threadIdx.x & 31) >> 3);
+      const bool valid = row < nB;
+      const int g = valid ? bGlobal[row] : 0, k0 = valid && mode != 3 ? bPtr[row] : 0, k1 = valid && mode != 3 ? bPtr[row + 1] : 0;
+      OrderedRow8<double, kCh, 2> entries(bCol, bVal, k0, k1, lane8);
+      Vec<double, kCh> acc;
+#pragma unroll
+      for (int ch = 0; ch < kCh; ch++) acc.v[ch] = 0;
+      entries.add_to(acc, false, bCol, bVal, lane8, [&](int c) {
+        Vec<double, kCh> v;
+#pragma unroll
+        for (int ch = 0; ch < kCh; ch++) v.v[ch] = x[(long long)c * K + ch];
+        return v;
+      });
+      if (valid && lane8 == 0) finish(g, acc.v);
+    }
+  }
+  // grid-stride over deep items (runs x 32 x G) then boundary items (rows x G);
+  // the stride is a multiple of G, so every thread keeps one channel group q
   for (long long t = t0; t < nItems; t += stride) {
-    double acc[4] = {0, 0, 0, 0};
+    double acc[kCh];
+#pragma unroll
+    for (int ch = 0; ch < kCh; ch++) acc[ch] = 0;
     int g = -1;
     if (t < nDeepItems) {
       const long long r = t / (32 * G);
@@ -1012,37 +1088,23 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
           const double w = c[s * planeStride];
           const double* xs = x + (long long)nb[s] * K + 4 * q;
 #pragma unroll
-          for (int ch = 0; ch < 4; ch++)
-            if (4 * q + ch < K) acc[ch] += w * xs[ch];
+          for (int ch = 0; ch < kCh; ch++)
+            if (KT || 4 * q + ch < K) acc[ch] = fma(w, xs[ch], acc[ch]);
         }
         g = pos;
       }
-    } else {
+    } else if constexpr (KT == 0) {
       const long long row = (t - nDeepItems) / G;
       for (int k = mode == 3 ? bPtr[row + 1] : bPtr[row]; k < bPtr[row + 1]; k++) {
         const double w = bVal[k];
         const double* xs = x + (long long)bCol[k] * K + 4 * q;
 #pragma unroll
-        for (int ch = 0; ch < 4; ch++)
-          if (4 * q + ch < K) acc[ch] += w * xs[ch];
+        for (int ch = 0; ch < kCh; ch++)
+          if (4 * q + ch < K) acc[ch] = fma(w, xs[ch], acc[ch]);
       }
       g = bGlobal[row];
     }
-    if (g >= 0) {
-#pragma unroll
-      for (int ch = 0; ch < 4; ch++) {
-        const int c = 4 * q + ch;
-        if (c >= K) continue;
-        const double bv = b ? b[(long long)g * K + c] : 0.0;
-        const double v = (mode == 0 || mode == 3) ? bv - acc[ch] : acc[ch];
-        if (out32) out32[(long long)g * KP + c] = float(v);
-        else out[(long long)g * K + c] = v;
-        rr[ch] += mode == 2 ? x[(long long)g * K + c] * v : v * v;  // mode 2: x . A x
-        bb[ch] += bv * bv;
-      }
-      if (out32)  // zero the padding channels of this group
-        for (int c = max(K, 4 * q); c < min(KP, 4 * q + 4); c++) out32[(long long)g * KP + c] = 0.f;
-    }
+    if (g >= 0) finish(g, acc);
   }
   if (!partials) return;
   block_partials(rr, bb, G, K, partials);
@@ -1304,12 +1366,19 @@ bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cu
   return cudaLaunchKernelEx(&cfg, k_gs_groups<T, W>, D.runs, D.groups, (const T*)D.coef, D.planeStride, (const T*)D.b, D.x, KP, G,
                             sweeps, reverse ? 1 : 0) == cudaSuccess;
 }
+// Lanes per boundary row of the residual and the restriction: 8 for one channel
+// group (a row one term after another was the launch's time: residual and
+// restriction of a 256^2 torus 4.7 and 3.9 us, the FP64 operator of a 1024^2 genus-2
+// 15.5 us of a 146 us CG step; 140 -> 152 us per step without the 8 lanes for a
+// 1013 x 1187 genus-2); with several groups the threads of a row's groups read its
+// texels' values contiguously, and there are enough rows in flight.
+static int row8_lanes(int G) { return G == 1 ? 8 : 1; }
 template <typename T, int W>
 void launch_residual(const ColourRun* runs, int nRuns, const T* coef, int planeStride, const int* bPtr, const int* bCol,
                      const T* bVal, const int* bGlobal, int nB, const T* rhs, const T* x, T* res, int KP, cudaStream_t s,
                      bool rhsEarly) {
   const int G = KP / W;
-  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G);
+  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * row8_lanes(G));
   if (db + bb == 0) return;
   launch(k_residual<T, W>, dim3(db + bb), s, runs, nRuns, coef, planeStride, db, bPtr, bCol, bVal, bGlobal, nB, rhs, x, res, KP, G,
          rhsEarly ? 1 : 0);
@@ -1318,7 +1387,7 @@ template <typename T, int W>
 void launch_restrict(const RestrictRun* runs, int nRuns, const int* rPtr, const int* rCol, const T* rVal, const int* rOut,
                      int nB, const T* res, T* coarseRhs, T* coarseX, long long coarseTexels, int KP, cudaStream_t s) {
   const int G = KP / W;
-  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G);
+  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * row8_lanes(G));
   if (db + bb == 0 && coarseTexels == 0) return;
   launch(k_restrict<T, W>, dim3(std::max(1, db + bb)), s, runs, nRuns, db, rPtr, rCol, rVal, rOut, nB, res, coarseRhs, coarseX,
          coarseTexels * KP, KP, G);
@@ -1410,6 +1479,10 @@ void launch_coarse_solve(int n, const double* ainv, const double* scale, const T
   go(k_coarse_solve<T, W, 4, 1, 4>, 4, 1);
 }
 
+// the operator's kernel for K right-hand sides
+static auto raw_kernel(int K) {
+  return K == 1 ? k_raw_operator<1> : K == 2 ? k_raw_operator<2> : K == 3 ? k_raw_operator<3> : K == 4 ? k_raw_operator<4> : k_raw_operator<0>;
+}
 static inline int raw_groups(int K) { int G = 1; while (4 * G < K) G *= 2; return G; }
 // fixed grid (grid-stride): bounded number of partial sums, launch-shape-independent order
 // Fixed grid of the FP64 operator and its reductions: 8 blocks per SM of the
@@ -1446,7 +1519,7 @@ void launch_raw_operator(const ColourRun* runs, int nRuns, const double* coef, i
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, G, mode,
+  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, G, mode,
          t.partials, (float*)nullptr, 0);
   if (t.partials && t.sums) launch_sums(t, blocks, K, s);
 }
@@ -1458,7 +1531,7 @@ void launch_raw_residual_f32(const ColourRun* runs, int nRuns, const double* coe
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, (double*)nullptr, K,
+  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, (double*)nullptr, K,
          G, xZero ? 3 : 0, t.partials, rhs32, KP);
   launch_sums(t, blocks, K, s);
 }
@@ -1487,7 +1560,7 @@ void launch_raw_apply_dot(const ColourRun* runs, int nRuns, const double* coef, 
   const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
   if (items == 0) return;
   const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, (const double*)nullptr, x,
+  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, (const double*)nullptr, x,
          out, K, G, 2, t.partials, (float*)nullptr, 0);
   if (!launch_sums(t, blocks, K, s, 2, sc, frozen)) launch(k_fcg_alpha, dim3(1), s, K, (const double*)t.sums, frozen, sc);
 }

@@ -86,6 +86,56 @@ __device__ __forceinline__ void fma_to(Vec<T, W>& acc, T a, const Vec<T, W>& v) 
   for (int c = 0; c < W; c++) acc.v[c] = fma(a, v.v[c], acc.v[c]);
 }
 
+// A sparse row on an aligned group of 8 lanes with the sum of a single thread: lane l
+// loads terms l, l + 8, ... (their entries, set-up data, U ahead of time by the
+// constructor), and the terms are then added one by one in their order, handed
+// round by shuffles, in every lane of the group.  A row so costs a few trips, not
+// two per term.  Whole warps call it (a lane past the rows has k0 = k1).
+template <typename T, int W, int U>
+struct OrderedRow8 {
+  int k, k1, c[U];
+  T w[U];
+  __device__ __forceinline__ OrderedRow8(const int* col, const T* val, int k0, int k1_, int lane8) : k(k0), k1(k1_) { load(col, val, lane8); }
+  __device__ __forceinline__ void load(const int* col, const T* val, int lane8) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = k + 8 * u + lane8;
+      c[u] = 0;
+      w[u] = T(0);
+      if (e < k1) {
+        c[u] = col[e];
+        w[u] = val[e];
+      }
+    }
+  }
+  // acc += sign sum w x(column), x: the value of a column
+  template <typename X>
+  __device__ __forceinline__ void add_to(Vec<T, W>& acc, bool minus, const int* col, const T* val, int lane8, const X& x) {
+    while (__any_sync(0xffffffffu, k < k1)) {
+      Vec<T, W> v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (k + 8 * u + lane8 < k1) v[u] = x(c[u]);
+        else
+#pragma unroll
+          for (int q = 0; q < W; q++) v[u].v[q] = T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+          const T ws = __shfl_sync(0xffffffffu, w[u], s, 8);
+          Vec<T, W> vs;
+#pragma unroll
+          for (int q = 0; q < W; q++) vs.v[q] = __shfl_sync(0xffffffffu, v[u].v[q], s, 8);
+          if (k + 8 * u + s < k1) fma_to(acc, minus ? -ws : ws, vs);
+        }
+      k += 8 * U;
+      load(col, val, lane8);
+    }
+  }
+};
+
 // Gauss-Seidel update of one colour-run texel: x = rhs*c4 - sum_{k!=4} c_k x_k
 // (IterativeSolvers.inl:449-463).  Items: runs x 32 x G.
 template <typename T, int W, typename LD>
