@@ -980,18 +980,19 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* __re
 // Per-block sums of two per-channel accumulators into partials[block][0..K) and
 // [K..2K): lanes l and l^s (s >= G) hold the same channel group, then the warps
 // are added in a fixed order (deterministic).  All threads of the block call it.
+template <int NCH = 4>
 __device__ __forceinline__ void block_partials(double (&ra)[4], double (&rb)[4], int G, int K, double* partials) {
   __shared__ double red[8][2][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int ch = 0; ch < 4; ch++)
+  for (int ch = 0; ch < NCH; ch++)
     for (int s = 16; s >= G; s >>= 1) {
       ra[ch] += __shfl_xor_sync(0xffffffffu, ra[ch], s);
       rb[ch] += __shfl_xor_sync(0xffffffffu, rb[ch], s);
     }
   if (lane < G)
 #pragma unroll
-    for (int ch = 0; ch < 4; ch++)
+    for (int ch = 0; ch < NCH; ch++)
       if (4 * lane + ch < K) { red[warp][0][4 * lane + ch] = ra[ch]; red[warp][1][4 * lane + ch] = rb[ch]; }
   __syncthreads();
   if ((int)threadIdx.x < K) {
@@ -1012,66 +1013,24 @@ __device__ __forceinline__ void block_partials(double (&ra)[4], double (&rb)[4],
 // (group q of G = KP/4 groups, or G = 1 for K = 1).  Per-block sums of res^2
 // and b^2 per channel go to `partials` for a deterministic norm reduction.
 // ----------------------------------------------------------------------------
-// KT: K (one channel group), or 0 for any K.
-template <int KT>
+// Any K (k_raw_few below for K <= 4).
 __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restrict__ runs, int nRuns, const double* __restrict__ coef,
                                                       int planeStride, const int* __restrict__ bPtr, const int* __restrict__ bCol,
                                                       const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
                                                       const double* __restrict__ b, const double* __restrict__ x,
-                                                      double* __restrict__ out, int Kany, int G, int mode, double* __restrict__ partials,
+                                                      double* __restrict__ out, int K, int G, int mode, double* __restrict__ partials,
                                                       float* __restrict__ out32, int KP) {
-  const int K = KT ? KT : Kany;
-  constexpr int kCh = KT ? KT : 4;
   grid_dependency_wait();
   grid_launch_dependents();
-  const long long nDeepItems = (long long)nRuns * 32 * G, nItems = nDeepItems + (KT ? 0 : (long long)nB * G);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int q = KT ? 0 : int(t0 % G);
-  double rr[4] = {0, 0, 0, 0}, bb[4] = {0, 0, 0, 0};
-  // row g: its value from the sums, its share of the norms
-  auto finish = [&](int g, const double (&acc)[kCh]) {
-#pragma unroll
-    for (int ch = 0; ch < kCh; ch++) {
-      const int c = 4 * q + ch;
-      if (c >= K) continue;
-      const double bv = b ? b[(long long)g * K + c] : 0.0;
-      const double v = (mode == 0 || mode == 3) ? bv - acc[ch] : acc[ch];
-      if (out32) out32[(long long)g * KP + c] = float(v);
-      else out[(long long)g * K + c] = v;
-      rr[ch] += mode == 2 ? x[(long long)g * K + c] * v : v * v;  // mode 2: x . A x
-      bb[ch] += bv * bv;
-    }
-    if (out32)  // zero the padding channels of this group
-      for (int c = max(K, 4 * q); c < min(KP, 4 * q + 4); c++) out32[(long long)g * KP + c] = 0.f;
-  };
-  if constexpr (KT > 0) {
-    // boundary rows first, 8 lanes each (a chain of trips that the deep rows then
-    // hide), summed in the rows' order
-    const int lane8 = threadIdx.x & 7;
-    for (long long w0 = t0 >> 5; w0 * 4 < nB; w0 += stride >> 5) {
-      const long long row = w0 * 4 + ((threadIdx.x & 31) >> 3);
-      const bool valid = row < nB;
-      const int g = valid ? bGlobal[row] : 0, k0 = valid && mode != 3 ? bPtr[row] : 0, k1 = valid && mode != 3 ? bPtr[row + 1] : 0;
-      OrderedRow8<double, kCh, 2> entries(bCol, bVal, k0, k1, lane8);
-      Vec<double, kCh> acc;
-#pragma unroll
-      for (int ch = 0; ch < kCh; ch++) acc.v[ch] = 0;
-      entries.add_to(acc, false, bCol, bVal, lane8, [&](int c) {
-        Vec<double, kCh> v;
-#pragma unroll
-        for (int ch = 0; ch < kCh; ch++) v.v[ch] = x[(long long)c * K + ch];
-        return v;
-      });
-      if (valid && lane8 == 0) finish(g, acc.v);
-    }
-  }
   // grid-stride over deep items (runs x 32 x G) then boundary items (rows x G);
   // the stride is a multiple of G, so every thread keeps one channel group q
+  const long long nDeepItems = (long long)nRuns * 32 * G, nItems = nDeepItems + (long long)nB * G;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int q = int(t0 % G);
+  double rr[4] = {0, 0, 0, 0}, bb[4] = {0, 0, 0, 0};
   for (long long t = t0; t < nItems; t += stride) {
-    double acc[kCh];
-#pragma unroll
-    for (int ch = 0; ch < kCh; ch++) acc[ch] = 0;
+    double acc[4] = {0, 0, 0, 0};
     int g = -1;
     if (t < nDeepItems) {
       const long long r = t / (32 * G);
@@ -1088,26 +1047,131 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
           const double w = c[s * planeStride];
           const double* xs = x + (long long)nb[s] * K + 4 * q;
 #pragma unroll
-          for (int ch = 0; ch < kCh; ch++)
-            if (KT || 4 * q + ch < K) acc[ch] = fma(w, xs[ch], acc[ch]);
+          for (int ch = 0; ch < 4; ch++)
+            if (4 * q + ch < K) acc[ch] = fma(w, xs[ch], acc[ch]);
         }
         g = pos;
       }
-    } else if constexpr (KT == 0) {
+    } else {
       const long long row = (t - nDeepItems) / G;
       for (int k = mode == 3 ? bPtr[row + 1] : bPtr[row]; k < bPtr[row + 1]; k++) {
         const double w = bVal[k];
         const double* xs = x + (long long)bCol[k] * K + 4 * q;
 #pragma unroll
-        for (int ch = 0; ch < kCh; ch++)
+        for (int ch = 0; ch < 4; ch++)
           if (4 * q + ch < K) acc[ch] = fma(w, xs[ch], acc[ch]);
       }
       g = bGlobal[row];
     }
-    if (g >= 0) finish(g, acc);
+    if (g >= 0) {
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        const int c = 4 * q + ch;
+        if (c >= K) continue;
+        const double bv = b ? b[(long long)g * K + c] : 0.0;
+        const double v = (mode == 0 || mode == 3) ? bv - acc[ch] : acc[ch];
+        if (out32) out32[(long long)g * KP + c] = float(v);
+        else out[(long long)g * K + c] = v;
+        rr[ch] += mode == 2 ? x[(long long)g * K + c] * v : v * v;  // mode 2: x . A x
+        bb[ch] += bv * bv;
+      }
+      if (out32)  // zero the padding channels of this group
+        for (int c = max(K, 4 * q); c < min(KP, 4 * q + 4); c++) out32[(long long)g * KP + c] = 0.f;
+    }
   }
   if (!partials) return;
   block_partials(rr, bb, G, K, partials);
+}
+
+// The same for K = KT <= 4 right-hand sides.
+//  * A warp takes a run, its header loaded during the run before.
+//  * Boundary rows run on 8 lanes (OrderedRow8), before the deep rows, whose loads
+//    hide their trips; the first rows' entries are loaded before the dependency wait.
+// What bounds it at 2048^2 (77 us for 203 MB): half the warps (64 registers), each a
+// long-scoreboard wait of 10.6 of 17.9 cycles per issue, and 58 % of the first-level
+// cache's cycles; a lane per value instead of per texel (consecutive addresses, but
+// the coefficients read for every channel) took 85 us.
+template <int KT>
+__global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict__ runs, int nRuns, const double* __restrict__ coef,
+                                                    int planeStride, const int* __restrict__ bPtr, const int* __restrict__ bCol,
+                                                    const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
+                                                    const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ out,
+                                                    int mode, double* __restrict__ partials, float* __restrict__ out32, int KP) {
+  const int lane = threadIdx.x & 31, lane8 = threadIdx.x & 7;
+  const int warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+  double rr[4] = {0, 0, 0, 0}, bb[4] = {0, 0, 0, 0};
+  // row g: its value from the sums, its share of the norms
+  auto finish = [&](int g, const double (&acc)[KT]) {
+#pragma unroll
+    for (int ch = 0; ch < KT; ch++) {
+      const double bv = b ? b[(long long)g * KT + ch] : 0.0;
+      const double v = (mode == 0 || mode == 3) ? bv - acc[ch] : acc[ch];
+      if (out32) out32[(long long)g * KP + ch] = float(v);
+      else out[(long long)g * KT + ch] = v;
+      rr[ch] += mode == 2 ? x[(long long)g * KT + ch] * v : v * v;  // mode 2: x . A x
+      bb[ch] += bv * bv;
+    }
+    if (out32)  // zero the padding channels
+      for (int c = KT; c < KP; c++) out32[(long long)g * KP + c] = 0.f;
+  };
+  {
+    int row = warp0 * 4 + (lane >> 3);
+    auto range = [&](int r, int& k0, int& k1, int& g) {
+      const bool valid = r < nB;
+      g = valid ? bGlobal[r] : 0;
+      k0 = valid && mode != 3 ? bPtr[r] : 0;
+      k1 = valid && mode != 3 ? bPtr[r + 1] : 0;
+    };
+    int k0, k1, g;
+    range(row, k0, k1, g);
+    OrderedRow8<double, KT, 2> entries(bCol, bVal, k0, k1, lane8);
+    grid_dependency_wait();
+    grid_launch_dependents();
+    for (int w = warp0; w * 4 < nB; w += warps) {
+      Vec<double, KT> acc;
+#pragma unroll
+      for (int ch = 0; ch < KT; ch++) acc.v[ch] = 0;
+      entries.add_to(acc, false, bCol, bVal, lane8, [&](int c) {
+        Vec<double, KT> v;
+#pragma unroll
+        for (int ch = 0; ch < KT; ch++) v.v[ch] = x[(long long)c * KT + ch];
+        return v;
+      });
+      if (row < nB && lane8 == 0) finish(g, acc.v);
+      row += warps * 4;
+      range(row, k0, k1, g);
+      entries = OrderedRow8<double, KT, 2>(bCol, bVal, k0, k1, lane8);
+    }
+  }
+  ColourRun R;
+  R.len = 0;
+  if (warp0 < nRuns) R = runs[warp0];
+  for (int r = warp0; r < nRuns; r += warps) {
+    ColourRun next;
+    next.len = 0;
+    if (r + warps < nRuns) next = runs[r + warps];  // on its way during this run
+    if (lane < R.len) {
+      double acc[KT];
+#pragma unroll
+      for (int ch = 0; ch < KT; ch++) acc[ch] = 0;
+      const int pos = R.pos0 + lane;
+      if (mode != 3) {
+        const double* c = coef + R.coef0 + lane;
+        const int nb[3] = {R.prev0 + lane, pos, R.next0 + lane};
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+          const double w = c[k * planeStride];
+          const double* xs = x + (long long)(nb[k / 3] + k % 3 - 1) * KT;
+#pragma unroll
+          for (int ch = 0; ch < KT; ch++) acc[ch] = fma(w, xs[ch], acc[ch]);
+        }
+      }
+      finish(pos, acc);
+    }
+    R = next;
+  }
+  if (!partials) return;
+  block_partials<KT>(rr, bb, 1, KT, partials);
 }
 
 // The solve loops' per-right-hand-side flags come in as a kernel argument (and
@@ -1479,10 +1543,6 @@ void launch_coarse_solve(int n, const double* ainv, const double* scale, const T
   go(k_coarse_solve<T, W, 4, 1, 4>, 4, 1);
 }
 
-// the operator's kernel for K right-hand sides
-static auto raw_kernel(int K) {
-  return K == 1 ? k_raw_operator<1> : K == 2 ? k_raw_operator<2> : K == 3 ? k_raw_operator<3> : K == 4 ? k_raw_operator<4> : k_raw_operator<0>;
-}
 static inline int raw_groups(int K) { int G = 1; while (4 * G < K) G *= 2; return G; }
 // fixed grid (grid-stride): bounded number of partial sums, launch-shape-independent order
 // Fixed grid of the FP64 operator and its reductions: 8 blocks per SM of the
@@ -1512,27 +1572,43 @@ static bool launch_sums(const SumTarget& t, int blocks, int K, cudaStream_t s, i
          sc, frozen);
   return one;
 }
+// Launches the operator for K right-hand sides; returns its blocks (a grid of at
+// most 8 per SM).  K <= 4 against the kernel for any K, per step: LIC on a 1024^2
+// genus-2 134 -> 129 us, its filtering at 1013 x 1187 140 -> 134, 1024^2 icosphere 307
+// -> 303; half the blocks (one wave) 127, 136 and 306.
+static int launch_raw(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
+                      const double* bVal, const int* bGlobal, int nB, const double* b, const double* x, double* out, int K, int mode,
+                      double* partials, float* out32, int KP, cudaStream_t s) {
+  const int G = raw_groups(K);
+  if (K > 4) {
+    const int blocks = int(std::min<long long>(raw_blocks(), nblk((long long)nRuns * 32 * G + (long long)nB * G)));
+    launch(k_raw_operator, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, G, mode, partials,
+           out32, KP);
+    return blocks;
+  }
+  const int blocks = int(std::min<long long>(raw_blocks(), nblk(32LL * std::max((long long)nRuns, (nB + 3) / 4LL))));
+  auto go = [&](auto kernel) {
+    launch(kernel, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, mode, partials, out32, KP);
+  };
+  if (K == 1) go(k_raw_few<1>);
+  else if (K == 2) go(k_raw_few<2>);
+  else if (K == 3) go(k_raw_few<3>);
+  else go(k_raw_few<4>);
+  return blocks;
+}
 void launch_raw_operator(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
                          const double* bVal, const int* bGlobal, int nB, const double* b, const double* x, double* out, int K,
                          int mode, const SumTarget& t, cudaStream_t s) {
-  const int G = raw_groups(K);
-  const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
-  if (items == 0) return;
-  const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, G, mode,
-         t.partials, (float*)nullptr, 0);
+  if (nRuns == 0 && nB == 0) return;
+  const int blocks = launch_raw(runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, K, mode, t.partials, nullptr, 0, s);
   if (t.partials && t.sums) launch_sums(t, blocks, K, s);
 }
 int raw_operator_blocks(int nRuns, int nB, int K) { return raw_blocks(); }
 void launch_raw_residual_f32(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr,
                              const int* bCol, const double* bVal, const int* bGlobal, int nB, const double* b, const double* x,
                              float* rhs32, int K, int KP, const SumTarget& t, cudaStream_t s, bool xZero) {
-  const int G = raw_groups(K);
-  const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
-  if (items == 0) return;
-  const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, (double*)nullptr, K,
-         G, xZero ? 3 : 0, t.partials, rhs32, KP);
+  if (nRuns == 0 && nB == 0) return;
+  const int blocks = launch_raw(runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, nullptr, K, xZero ? 3 : 0, t.partials, rhs32, KP, s);
   launch_sums(t, blocks, K, s);
 }
 
@@ -1556,12 +1632,8 @@ void launch_fcg_update(long long n, int K, int KP, const double* sc, const doubl
 void launch_raw_apply_dot(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
                           const double* bVal, const int* bGlobal, int nB, const double* x, double* out, int K, const int* frozen,
                           double* sc, const SumTarget& t, cudaStream_t s) {
-  const int G = raw_groups(K);
-  const long long items = (long long)nRuns * 32 * G + (long long)nB * G;
-  if (items == 0) return;
-  const int blocks = int(std::min<long long>(raw_blocks(), nblk(items)));
-  launch(raw_kernel(K), dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, (const double*)nullptr, x,
-         out, K, G, 2, t.partials, (float*)nullptr, 0);
+  if (nRuns == 0 && nB == 0) return;
+  const int blocks = launch_raw(runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, nullptr, x, out, K, 2, t.partials, nullptr, 0, s);
   if (!launch_sums(t, blocks, K, s, 2, sc, frozen)) launch(k_fcg_alpha, dim3(1), s, K, (const double*)t.sums, frozen, sc);
 }
 
