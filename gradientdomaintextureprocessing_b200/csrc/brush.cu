@@ -46,27 +46,59 @@ __global__ void k_brush_deep_coef(int nDeep, int k, const int* __restrict__ deep
   }
 }
 
-// out[texel] = c0 m[prev i] + c1 m[prev i+1] + c2 m[next i] + c3 m[next i+1]
-__global__ void k_brush_deep_apply(int nDeep, int k, const int* __restrict__ deepGlobal, const int4* __restrict__ cells,
-                                   const double* __restrict__ coef, const double* __restrict__ mask, double* __restrict__ out) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nDeep * k) return;
-  const long long d = t / k;
-  const int c = int(t - d * k);
-  const int4 cl = cells[d];
-  const double* a = coef + 4 * d * k + c;
-  out[(long long)deepGlobal[d] * k + c] = a[0] * mask[cl.x] + a[k] * mask[cl.y] + a[2 * k] * mask[cl.z] + a[3 * k] * mask[cl.w];
-}
+struct BrushRows {  // per channel the boundary x cells matrix
+  const int* ptr[4];
+  const int* col[4];
+  const double* val[4];
+};
 
-// out[boundary texel] = row of channel c's boundary x cells matrix times m
-__global__ void k_brush_boundary_apply(int nB, int k, int c, const int* __restrict__ bGlobal, const int* __restrict__ ptr,
-                                       const int* __restrict__ col, const double* __restrict__ val, const double* __restrict__ mask,
-                                       double* __restrict__ out) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nB) return;
-  double s = 0.0;
-  for (int e = ptr[b]; e < ptr[b + 1]; e++) s += val[e] * mask[col[e]];
-  out[(long long)bGlobal[b] * k + c] = s;
+// One stroke, every texel and channel in one launch.  The first blocks take the
+// boundary texels, 8 lanes per row and channel (a chain of loads that the deep
+// texels hide): out = row times m.  The others a deep texel per thread: out = c0
+// m[prev i] + c1 m[prev i+1] + c2 m[next i] + c3 m[next i+1], its 4 K coefficients
+// read as pairs.  The bytes (140 per deep texel at K = 3) take 8 us at 1024^2; as a
+// launch for the deep values, with a division per value, and a launch per channel of
+// one thread per row a call took 34.8 us, now 18.3 with the host's share.
+template <int K>
+__global__ void __launch_bounds__(256) k_brush_apply(int rowBlocks, int nB, const int* __restrict__ bGlobal, BrushRows rows, int nDeep,
+                                                     const int* __restrict__ deepGlobal, const int4* __restrict__ cells,
+                                                     const double* __restrict__ coef, const double* __restrict__ mask,
+                                                     double* __restrict__ out) {
+  if ((int)blockIdx.x < rowBlocks) {
+    const int t = blockIdx.x * 256 + threadIdx.x, item = t >> 3, lane8 = t & 7, b = item / K, c = item - b * K;
+    double s = 0.0;
+    if (b < nB) {
+      const int *ptr = rows.ptr[0], *col = rows.col[0];
+      const double* val = rows.val[0];
+#pragma unroll
+      for (int q = 1; q < K; q++)
+        if (c == q) {
+          ptr = rows.ptr[q];
+          col = rows.col[q];
+          val = rows.val[q];
+        }
+      for (int e = ptr[b] + lane8; e < ptr[b + 1]; e += 8) s += val[e] * mask[col[e]];
+    }
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+    if (b < nB && lane8 == 0) out[(long long)bGlobal[b] * K + c] = s;
+    return;
+  }
+  const int d = (blockIdx.x - rowBlocks) * 256 + threadIdx.x;
+  if (d >= nDeep) return;
+  const int4 cl = cells[d];
+  double a[4 * K];
+  const double2* p = reinterpret_cast<const double2*>(coef + 4ll * K * d);
+#pragma unroll
+  for (int i = 0; i < 2 * K; i++) {
+    const double2 v = p[i];
+    a[2 * i] = v.x;
+    a[2 * i + 1] = v.y;
+  }
+  const double m0 = mask[cl.x], m1 = mask[cl.y], m2 = mask[cl.z], m3 = mask[cl.w];
+  double* o = out + (long long)deepGlobal[d] * K;
+#pragma unroll
+  for (int c = 0; c < K; c++) o[c] = a[c] * m0 + a[K + c] * m1 + a[2 * K + c] * m2 + a[3 * K + c] * m3;
 }
 
 }  // namespace
@@ -232,12 +264,17 @@ extern "C" int gdtp_brush_apply_device(gdtp_brush* b, const double* mask_dev, do
     if (cudaSetDevice(b->sys->device()) != cudaSuccess) return fail(GDTP_ERR_CUDA, "gdtp_brush_apply_device: no usable device");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int k = b->k;
-    if (b->nDeep > 0)
-      k_brush_deep_apply<<<int(((long long)b->nDeep * k + 255) / 256), 256, 0, st>>>(b->nDeep, k, b->deepGlobal, b->deepCells, b->coef,
-                                                                                      mask_dev, out_dev);
-    for (int c = 0; c < k && b->nB > 0; c++)
-      k_brush_boundary_apply<<<(b->nB + 255) / 256, 256, 0, st>>>(b->nB, k, c, b->bGlobal, b->bPtr[c], b->bCol[c], b->bVal[c], mask_dev,
-                                                                  out_dev);
+    BrushRows rows{};
+    for (int c = 0; c < k; c++) {
+      rows.ptr[c] = b->bPtr[c];
+      rows.col[c] = b->bCol[c];
+      rows.val[c] = b->bVal[c];
+    }
+    const int rowBlocks = int(((long long)b->nB * k * 8 + 255) / 256), blocks = rowBlocks + (b->nDeep + 255) / 256;
+    if (blocks > 0) {
+      auto kernel = k == 1 ? k_brush_apply<1> : k == 2 ? k_brush_apply<2> : k == 3 ? k_brush_apply<3> : k_brush_apply<4>;
+      kernel<<<blocks, 256, 0, st>>>(rowBlocks, b->nB, b->bGlobal, rows, b->nDeep, b->deepGlobal, b->deepCells, b->coef, mask_dev, out_dev);
+    }
     return cuda_ok(cudaGetLastError(), "apply") ? GDTP_OK : GDTP_ERR_CUDA;
   });
 }

@@ -153,3 +153,54 @@ def test_boundary_products_at_every_chunking(ico, k, knobs):
         ico.update(1e-3, 1.0)
     for precision in ("mixed", "fp64"):
         np.testing.assert_array_equal(out[precision, 0], out[precision, 1 << 30])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+def test_brush_at_every_width(torus, ico, k):
+    """A uniform mask is S f and masks that add up to one add up to it, per channel:
+    both sides are FP64 sums of the same at most 64 products per texel, so they
+    agree to 64 x 2^-53 of the largest product sum, taken as 1e-12 of the largest
+    entry times the cancellation of a stiffness row (at most 10)."""
+    from gradientdomaintextureprocessing_b200.system import STIFFNESS, Brush
+    for s in (torus, ico):
+        f, _ = vectors(s.n, k)
+        brush = Brush(s, f)
+        cells = s.hierarchy.counts(0)["numCells"]
+        sf = s.apply(f, STIFFNESS)
+        scale = np.abs(sf).max()
+        assert np.abs(brush.apply(np.ones(cells)) - sf).max() <= 1e-11 * scale
+        part = np.random.default_rng(3).integers(0, 3, cells)
+        total = sum(brush.apply((part == i).astype(float)) for i in range(3))
+        assert np.abs(total - sf).max() <= 1e-11 * scale
+        single = Brush(s, f[:, k - 1]).apply((part == 1).astype(float))
+        assert np.abs(single[:, 0] - brush.apply((part == 1).astype(float))[:, k - 1]).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 6, 16, 64])
+def test_host_vectors_of_every_size(torus, ico, k):
+    """Host vectors below and above the staging size, with a ragged last chunk, pageable
+    and pinned: the operator is linear and exact in powers of two, and the same call
+    on pinned memory is a plain copy, so every comparison is bitwise."""
+    import torch
+    for s in (torus, ico):
+        b, x = vectors(s.n, k)
+        y = s.apply(x)
+        pinned = torch.from_numpy(x).pin_memory().numpy()
+        np.testing.assert_array_equal(s.apply(pinned), y)
+        np.testing.assert_array_equal(s.apply(4.0 * x), 4.0 * y)
+        np.testing.assert_array_equal(s.apply(x[:, k - 1])[:, 0], y[:, k - 1])
+        np.testing.assert_array_equal(s.residual(b, x), s.residual(torch.from_numpy(b).pin_memory().numpy(), pinned))
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 12, 64])
+def test_host_vcycle_and_sweeps(ico, k):
+    """The V-cycle and the sweeps on host vectors, packed on the device: no sweeps give
+    the vector back, and a column's result does not depend on the others."""
+    b, x = (v.astype(np.float32) for v in vectors(ico.n, k))
+    np.testing.assert_array_equal(ico.relax(x, b, sweeps=0), x)
+    wide = ico.relax(x, b, sweeps=2)
+    for c in (0, k - 1):
+        np.testing.assert_array_equal(wide[:, c], ico.relax(x[:, c], b[:, c], sweeps=2)[:, 0])
+    x0 = x.copy()
+    ico.vcycle(x, b)
+    np.testing.assert_array_equal(x, x0)
