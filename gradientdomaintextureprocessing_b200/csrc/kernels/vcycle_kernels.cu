@@ -1276,9 +1276,10 @@ __global__ void k_axpby(double* __restrict__ out, double a, const double* __rest
   if (i < n) out[i] = a * x[i] + b * y[i];
 }
 
-// FP64 residual (n*K, tight) -> FP32 right-hand side (n*KP, padded)
-template <typename T>
-__global__ void k_pack_rhs(const double* __restrict__ r, T* __restrict__ rhs, long long n, int K, int KP) {
+// n*K, tight -> n*KP, padded with zeros: the FP64 residual as a right-hand side, or
+// the caller's vectors
+template <typename S, typename T>
+__global__ void k_pack(const S* __restrict__ r, T* __restrict__ rhs, long long n, int K, int KP) {
   grid_dependency_wait();
   grid_launch_dependents();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1286,6 +1287,15 @@ __global__ void k_pack_rhs(const double* __restrict__ r, T* __restrict__ rhs, lo
   const long long i = t / KP;
   const int c = int(t - i * KP);
   rhs[t] = c < K ? T(r[i * K + c]) : T(0);
+}
+template <typename T>
+__global__ void k_unpack(const T* __restrict__ padded, T* __restrict__ tight, long long n, int K, int KP) {
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * K) return;
+  const long long i = t / K;
+  tight[t] = padded[i * KP + (t - i * K)];
 }
 // x64 += e (padded FP32/FP64 correction); e is cleared for the next V-cycle
 // (its padding lanes stay zero through the V-cycle).  Columns with frozen[c]
@@ -1642,7 +1652,15 @@ void launch_axpby(double* out, double a, const double* x, double b, const double
 }
 template <typename T>
 void launch_pack_rhs(const double* r, T* rhs, long long n, int K, int KP, cudaStream_t s) {
-  launch(k_pack_rhs<T>, dim3(nblk(n * KP)), s, r, rhs, n, K, KP);
+  launch(k_pack<double, T>, dim3(nblk(n * KP)), s, r, rhs, n, K, KP);
+}
+template <typename T>
+void launch_pad_vector(const T* tight, T* padded, long long n, int K, int KP, cudaStream_t s) {
+  launch(k_pack<T, T>, dim3(nblk(n * KP)), s, tight, padded, n, K, KP);
+}
+template <typename T>
+void launch_unpad_vector(const T* padded, T* tight, long long n, int K, int KP, cudaStream_t s) {
+  launch(k_unpack<T>, dim3(nblk(n * K)), s, padded, tight, n, K, KP);
 }
 void launch_set_flags(int* flags, unsigned long long mask, int k, cudaStream_t s) {
   launch(k_set_flags, dim3(1), s, flags, mask, k);
@@ -1669,6 +1687,10 @@ GDTP_INSTANTIATE(float, 1)
 GDTP_INSTANTIATE(float, 4)
 GDTP_INSTANTIATE(double, 1)
 GDTP_INSTANTIATE(double, 4)
+template void launch_pad_vector<float>(const float*, float*, long long, int, int, cudaStream_t);
+template void launch_pad_vector<double>(const double*, double*, long long, int, int, cudaStream_t);
+template void launch_unpad_vector<float>(const float*, float*, long long, int, int, cudaStream_t);
+template void launch_unpad_vector<double>(const double*, double*, long long, int, int, cudaStream_t);
 template void launch_pack_rhs<float>(const double*, float*, long long, int, int, cudaStream_t);
 template void launch_pack_rhs<double>(const double*, double*, long long, int, int, cudaStream_t);
 template void launch_add_correction<float>(double*, float*, long long, int, int, cudaStream_t, const int*);

@@ -230,6 +230,12 @@ void launch_raw_residual_f32(const ColourRun* runs, int nRuns, const double* coe
                              float* rhs32, int K, int KP, const SumTarget& t, cudaStream_t s, bool xZero = false);
 template <typename T>
 void launch_pack_rhs(const double* r, T* rhs, long long n, int K, int KP, cudaStream_t s);
+// vectors of one type between the caller's layout (n x K, tight) and the multigrid's
+// (n x KP; padding channels zero)
+template <typename T>
+void launch_pad_vector(const T* tight, T* padded, long long n, int K, int KP, cudaStream_t s);
+template <typename T>
+void launch_unpad_vector(const T* padded, T* tight, long long n, int K, int KP, cudaStream_t s);
 // flags[c] = bit c of mask, c < k <= 64
 void launch_set_flags(int* flags, unsigned long long mask, int k, cudaStream_t s);
 // Flexible preconditioned CG around the FP32 V-cycle (vcycle_kernels.cu).  sc: 4K

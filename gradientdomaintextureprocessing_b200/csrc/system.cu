@@ -1590,10 +1590,9 @@ bool DeviceSystem::apply(int which, const double* x, double* y, int k) {
   if (which == 0 && !updated_) { err_ = "apply(A) before update"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  return check(cudaMemcpyAsync(x64_, x, n * k * 8, cudaMemcpyHostToDevice, stream_), "h2d") &&
+  return check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") &&
          raw_apply_dev(*op, nullptr, x64_, r64_, k, 1, stream_, nullptr) &&
-         check(cudaMemcpyAsync(y, r64_, n * k * 8, cudaMemcpyDeviceToHost, stream_), "d2h") &&
-         check(cudaStreamSynchronize(stream_), "apply");
+         check(hostCopy.download(y, r64_, n * k * 8, stream_), "apply");
 }
 
 bool DeviceSystem::apply_combination(double a, double b, const double* x, double* y, int k) {
@@ -1602,13 +1601,12 @@ bool DeviceSystem::apply_combination(double a, double b, const double* x, double
   if (k < 1 || k > 64) { err_ = "k must be in [1, 64]"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  if (!check(cudaMemcpyAsync(x64_, x, n * k * 8, cudaMemcpyHostToDevice, stream_), "h2d") ||
+  if (!check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") ||
       !raw_apply_dev(rawM_, nullptr, x64_, r64_, k, 1, stream_, nullptr) ||
       !raw_apply_dev(rawS_, nullptr, x64_, b64_, k, 1, stream_, nullptr))
     return false;
   dev::launch_axpby(r64_, a, r64_, b, b64_, (long long)(n * k), stream_);
-  return check(cudaMemcpyAsync(y, r64_, n * k * 8, cudaMemcpyDeviceToHost, stream_), "d2h") &&
-         check(cudaStreamSynchronize(stream_), "apply");
+  return check(hostCopy.download(y, r64_, n * k * 8, stream_), "apply");
 }
 
 bool DeviceSystem::residual_host(const double* b, const double* x, int k, double* rel) {
@@ -1618,8 +1616,8 @@ bool DeviceSystem::residual_host(const double* b, const double* x, int k, double
   if (k < 1 || k > 64) { err_ = "k must be in [1, 64]"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  if (!check(cudaMemcpyAsync(b64_, b, n * k * 8, cudaMemcpyHostToDevice, stream_), "h2d") ||
-      !check(cudaMemcpyAsync(x64_, x, n * k * 8, cudaMemcpyHostToDevice, stream_), "h2d") ||
+  if (!check(hostCopy.upload(b64_, b, n * k * 8, stream_), "h2d") ||
+      !check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") ||
       !raw_apply_dev(rawA_, b64_, x64_, r64_, k, 0, stream_, sumsHost_))
     return false;
   for (int c = 0; c < k; c++) rel[c] = std::sqrt(sumsHost_[c] / std::max(sumsHost_[k + c], 1e-300));
@@ -1642,7 +1640,7 @@ bool DeviceSystem::solve_filtering(const double* f_host, double* x_host, int k, 
     filterK_ = workK_;
   }
   // b = M f (+ coefS S f) on the device from one upload of f
-  if (!check(cudaMemcpyAsync(fDev_, f_host, n * k * sizeof(double), cudaMemcpyHostToDevice, stream_), "h2d f") ||
+  if (!check(hostCopy.upload(fDev_, f_host, n * k * sizeof(double), stream_), "h2d f") ||
       !raw_apply_dev(rawM_, nullptr, fDev_, b64_, k, 1, stream_, nullptr))
     return false;
   kernelLaunches += 1;
@@ -1652,6 +1650,30 @@ bool DeviceSystem::solve_filtering(const double* f_host, double* x_host, int k, 
     kernelLaunches += 2;
   }
   return solve_mixed(nullptr, x_host, b64_, x64_, k, tol, maxIters, nullptr, rep, true);
+}
+
+template <typename T>
+bool DeviceSystem::vectors_in(Multigrid<T>& mg, const T* x, const T* rhs, int k) {
+  if (!ensure_work(k)) return false;
+  const size_t n = h_.levels[0].numTexels;
+  LevelDev<T>& D0 = mg.levels[0];
+  // through the FP64 work vectors (at least n x k values of either type)
+  T *xs = reinterpret_cast<T*>(x64_), *bs = reinterpret_cast<T*>(b64_);
+  if (!check(hostCopy.upload(xs, x, n * k * sizeof(T), stream_), "h2d") || !check(hostCopy.upload(bs, rhs, n * k * sizeof(T), stream_), "h2d"))
+    return false;
+  dev::launch_pad_vector<T>(xs, D0.x, (long long)n, k, mg.KP, stream_);
+  dev::launch_pad_vector<T>(bs, D0.b, (long long)n, k, mg.KP, stream_);
+  return check(cudaGetLastError(), "pad vectors");
+}
+
+template <typename T>
+bool DeviceSystem::iterate_out(Multigrid<T>& mg, T* x, int k, const char* what) {
+  const size_t n = h_.levels[0].numTexels;
+  T* xs = reinterpret_cast<T*>(x64_);
+  dev::launch_unpad_vector<T>(mg.levels[0].x, xs, (long long)n, k, mg.KP, stream_);
+  queue_barrier_check(mg, stream_);
+  // (the download ends with the stream's work done, the barrier check's word included)
+  return check(cudaGetLastError(), what) && check(hostCopy.download(x, xs, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
 }
 
 bool DeviceSystem::vcycle_host64(double* x, const double* rhs, int k) {
@@ -1666,23 +1688,9 @@ bool DeviceSystem::vcycle_host64(double* x, const double* rhs, int k) {
     if (!build_multigrid(*mg64_, KP)) return false;
   }
   Multigrid<double>& mg = *mg64_;
-  const size_t n = h_.levels[0].numTexels;
-  std::vector<double> px(n * mg.KP, 0.0), pb(n * mg.KP, 0.0);
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) { px[i * mg.KP + c] = x[i * k + c]; pb[i * mg.KP + c] = rhs[i * k + c]; }
-  LevelDev<double>& D0 = mg.levels[0];
-  if (!check(cudaMemcpyAsync(D0.x, px.data(), px.size() * 8, cudaMemcpyHostToDevice, stream_), "h2d") ||
-      !check(cudaMemcpyAsync(D0.b, pb.data(), pb.size() * 8, cudaMemcpyHostToDevice, stream_), "h2d"))
-    return false;
+  if (!vectors_in(mg, x, rhs, k)) return false;
   if (mg.KP == 1) vcycle<double, 1>(mg, stream_); else vcycle<double, 4>(mg, stream_);
-  queue_barrier_check(mg, stream_);
-  if (!check(cudaGetLastError(), "vcycle") ||
-      !check(cudaMemcpyAsync(px.data(), D0.x, px.size() * 8, cudaMemcpyDeviceToHost, stream_), "d2h") ||
-      !check(cudaStreamSynchronize(stream_), "vcycle") || !barrier_ok(mg))
-    return false;
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) x[i * k + c] = px[i * mg.KP + c];
-  return true;
+  return iterate_out(mg, x, k, "vcycle");
 }
 
 bool DeviceSystem::relax_host(float* x, const float* rhs, int k, int sweeps, bool reverse) {
@@ -1693,14 +1701,8 @@ bool DeviceSystem::relax_host(float* x, const float* rhs, int k, int sweeps, boo
   Multigrid<float>* mgp = mg32_for(kp_for(k));
   if (!mgp) return false;
   Multigrid<float>& mg = *mgp;
-  const size_t n = h_.levels[0].numTexels;
-  std::vector<float> px(n * mg.KP, 0.f), pb(n * mg.KP, 0.f);
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) { px[i * mg.KP + c] = x[i * k + c]; pb[i * mg.KP + c] = rhs[i * k + c]; }
   LevelDev<float>& D0 = mg.levels[0];
-  if (!check(cudaMemcpyAsync(D0.x, px.data(), px.size() * 4, cudaMemcpyHostToDevice, stream_), "h2d") ||
-      !check(cudaMemcpyAsync(D0.b, pb.data(), pb.size() * 4, cudaMemcpyHostToDevice, stream_), "h2d"))
-    return false;
+  if (!vectors_in(mg, x, rhs, k)) return false;
   if (tiled(D0, mg.KP)) {
     if (sweeps > 0) tile_smooth(mg, D0, sweeps, reverse, false, stream_, false);
   } else {
@@ -1711,14 +1713,7 @@ bool DeviceSystem::relax_host(float* x, const float* rhs, int k, int sweeps, boo
         colour_sweep<float, 1>(D0, mg.KP, reverse, false, sw > 0, stream_);
     }
   }
-  queue_barrier_check(mg, stream_);
-  if (!check(cudaGetLastError(), "relax") ||
-      !check(cudaMemcpyAsync(px.data(), D0.x, px.size() * 4, cudaMemcpyDeviceToHost, stream_), "d2h") ||
-      !check(cudaStreamSynchronize(stream_), "relax") || !barrier_ok(mg))
-    return false;
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) x[i * k + c] = px[i * mg.KP + c];
-  return true;
+  return iterate_out(mg, x, k, "relax");
 }
 
 bool DeviceSystem::vcycle_host(float* x, const float* rhs, int k) {
@@ -1729,23 +1724,9 @@ bool DeviceSystem::vcycle_host(float* x, const float* rhs, int k) {
   Multigrid<float>* mgp = mg32_for(kp_for(k));
   if (!mgp) return false;
   Multigrid<float>& mg = *mgp;
-  const size_t n = h_.levels[0].numTexels;
-  std::vector<float> px(n * mg.KP, 0.f), pb(n * mg.KP, 0.f);
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) { px[i * mg.KP + c] = x[i * k + c]; pb[i * mg.KP + c] = rhs[i * k + c]; }
-  LevelDev<float>& D0 = mg.levels[0];
-  if (!check(cudaMemcpyAsync(D0.x, px.data(), px.size() * 4, cudaMemcpyHostToDevice, stream_), "h2d") ||
-      !check(cudaMemcpyAsync(D0.b, pb.data(), pb.size() * 4, cudaMemcpyHostToDevice, stream_), "h2d"))
-    return false;
+  if (!vectors_in(mg, x, rhs, k)) return false;
   if (mg.KP == 1) vcycle<float, 1>(mg, stream_); else vcycle<float, 4>(mg, stream_);
-  queue_barrier_check(mg, stream_);
-  if (!check(cudaGetLastError(), "vcycle") ||
-      !check(cudaMemcpyAsync(px.data(), D0.x, px.size() * 4, cudaMemcpyDeviceToHost, stream_), "d2h") ||
-      !check(cudaStreamSynchronize(stream_), "vcycle") || !barrier_ok(mg))
-    return false;
-  for (size_t i = 0; i < n; i++)
-    for (int c = 0; c < k; c++) x[i * k + c] = px[i * mg.KP + c];
-  return true;
+  return iterate_out(mg, x, k, "vcycle");
 }
 
 bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const double* b_dev, double* x_dev, int k, double tol,
@@ -1769,8 +1750,8 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
   cudaEventRecord(e0, s);
   const double* B = b_dev ? b_dev : b64_;
   double* X = x_dev ? x_dev : x64_;
-  if (b_host && !check(cudaMemcpyAsync(b64_, b_host, n * k * 8, cudaMemcpyHostToDevice, s), "h2d b")) return false;
-  if (x_host && !zeroGuess && !check(cudaMemcpyAsync(x64_, x_host, n * k * 8, cudaMemcpyHostToDevice, s), "h2d x")) return false;
+  if (b_host && !check(hostCopy.upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
+  if (x_host && !zeroGuess && !check(hostCopy.upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
   if (zeroGuess && !check(cudaMemsetAsync(X, 0, n * k * 8, s), "zero x")) return false;
   int it = 0;
   double rm = 0;
@@ -1842,7 +1823,7 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
       collect_timing(mg);
     }
   }
-  if (x_host && !check(cudaMemcpyAsync(x_host, x64_, n * k * 8, cudaMemcpyDeviceToHost, s), "d2h x")) return false;
+  if (x_host && !check(hostCopy.download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
   queue_barrier_check(mg, s);
   cudaEventRecord(e1, s);
   if (userStream) cudaStreamWaitEvent(userStream, e1, 0);
@@ -2161,8 +2142,8 @@ bool DeviceSystem::solve_fp64(const double* b_host, double* x_host, const double
   // filled from the host
   const double* B = b_dev ? b_dev : b64_;
   double* X = x_dev ? x_dev : x64_;
-  if (b_host && !check(cudaMemcpyAsync(b64_, b_host, n * k * 8, cudaMemcpyHostToDevice, s), "h2d b")) return false;
-  if (x_host && !check(cudaMemcpyAsync(x64_, x_host, n * k * 8, cudaMemcpyHostToDevice, s), "h2d x")) return false;
+  if (b_host && !check(hostCopy.upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
+  if (x_host && !check(hostCopy.upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
   kernelLaunches += 2;  // operator + norm reduction
   if (!raw_apply_dev(rawA_, B, X, r64_, k, 0, s, nullptr) || !read_norms(k, s, "initial residual")) return false;
   rep = SolveReport();
@@ -2207,7 +2188,7 @@ bool DeviceSystem::solve_fp64(const double* b_host, double* x_host, const double
     it++;
     rm = rel_max();
   }
-  if (x_host && !check(cudaMemcpyAsync(x_host, x64_, n * k * 8, cudaMemcpyDeviceToHost, s), "d2h x")) return false;
+  if (x_host && !check(hostCopy.download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
   queue_barrier_check(mg, s);
   cudaEventRecord(e1, s);
   if (userStream) cudaStreamWaitEvent(userStream, e1, 0);
