@@ -50,24 +50,35 @@ __global__ void __launch_bounds__(256) k_gemm(const GemmTask* __restrict__ tasks
     for (int c = 0; c < 4; c++) acc[r][c] = 0.0;
   const double* Ab = A + T.a;
   const double* Bb = B + T.b;
+  // the next chunk of K is loaded into registers while this one is multiplied
+  double an[4], bn[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int e = tid + 256 * q;
+      an[q] = 0.0;
+      if (T.transA) {  // A stored K x M: consecutive threads along the rows of the tile
+        const int gr = row0 + (e & 63), gk = k0 + (e >> 6);
+        if (gr < T.M && gk < T.K) an[q] = Ab[(long long)gk * T.lda + gr];
+      } else {  // A stored M x K: consecutive threads along k
+        const int gr = row0 + (e >> 4), gk = k0 + (e & 15);
+        if (gr < T.M && gk < T.K) an[q] = Ab[(long long)gr * T.lda + gk];
+      }
+      const int gk = k0 + (e >> 6), gc = col0 + (e & 63);
+      bn[q] = (gk < T.K && gc < T.N) ? Bb[(long long)gk * T.ldb + gc] : 0.0;
+    }
+  };
+  fetch(0);
   for (int k0 = 0; k0 < T.K; k0 += 16) {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int e = tid + 256 * q;
-      double av = 0.0;
-      if (T.transA) {  // A stored K x M: consecutive threads along the rows of the tile
-        const int kk = e >> 6, rr = e & 63, gr = row0 + rr, gk = k0 + kk;
-        if (gr < T.M && gk < T.K) av = Ab[(long long)gk * T.lda + gr];
-        As[kk][rr] = av;
-      } else {  // A stored M x K: consecutive threads along k
-        const int rr = e >> 4, kk = e & 15, gr = row0 + rr, gk = k0 + kk;
-        if (gr < T.M && gk < T.K) av = Ab[(long long)gr * T.lda + gk];
-        As[kk][rr] = av;
-      }
-      const int kk = e >> 6, cc = e & 63, gk = k0 + kk, gc = col0 + cc;
-      Bs[kk][cc] = (gk < T.K && gc < T.N) ? Bb[(long long)gk * T.ldb + gc] : 0.0;
+      if (T.transA) As[e >> 6][e & 63] = an[q];
+      else As[e & 15][e >> 4] = an[q];
+      Bs[e >> 6][e & 63] = bn[q];
     }
     __syncthreads();
+    if (k0 + 16 < T.K) fetch(k0 + 16);
 #pragma unroll
     for (int kk = 0; kk < 16; kk++) {
       double a[4], b[4];
@@ -137,19 +148,23 @@ __global__ void __launch_bounds__(256) k_bgj_diag(int k, const long long* __rest
       p = 1.0;
     }
     const double ip = 1.0 / p;
+    // one update for every entry, the pivot row and column selected into it: a
+    // branch per entry (four cases, divergent) made a step 1.3 us.  Entries past bs
+    // stay zero.
+    double tb[4];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int b = 0; b < 4; b++) tb[b] = rowS[buf][tc + 16 * b] * ip;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      const double ca = colS[buf][tr + 16 * a], cp = -ca * ip;
+      const bool row = tr + 16 * a == s;
 #pragma unroll
       for (int b = 0; b < 4; b++) {
-        const int i = tr + 16 * a, j = tc + 16 * b;
-        if (i >= bs || j >= bs) continue;
-        double v;
-        if (i == s && j == s) v = ip;
-        else if (i == s) v = rowS[buf][j] * ip;
-        else if (j == s) v = -colS[buf][i] * ip;
-        else v = P[a][b] - colS[buf][i] * (rowS[buf][j] * ip);
-        P[a][b] = v;
+        const bool col = tc + 16 * b == s;
+        const double v = fma(-ca, tb[b], P[a][b]);
+        P[a][b] = row ? (col ? ip : tb[b]) : (col ? cp : v);
       }
+    }
   }
   double* Pq = Pinv + (long long)q * kPB * kPB;
 #pragma unroll
@@ -197,15 +212,36 @@ __global__ void __launch_bounds__(256) k_bgj_panel(int k, const long long* __res
     Xs[r][c] = x;
   }
   __syncthreads();
+  // 4 x 4 outputs per thread (rows ty + 16 r, columns tx + 16 c): 8 shared-memory
+  // reads for 16 products, not two for each
   double* Rq = R + wsOff[q];
-  for (int e = threadIdx.x; e < kPB * kPB; e += 256) {
-    const int r = e / kPB, c = e % kPB, j = t0 + c;
-    if (r >= bs || j >= m) continue;
-    double v = 0.0;
-    for (int d = 0; d < bs; d++) v = fma(Ps[r][d], Xs[d][c], v);
-    Rq[(long long)r * m + j] = v;
-    Aq[(long long)(kb + r) * m + j] = v;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double acc[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[r][c] = 0.0;
+#pragma unroll 4
+  for (int d = 0; d < bs; d++) {
+    double a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) a[r] = Ps[ty + 16 * r][d];
+#pragma unroll
+    for (int c = 0; c < 4; c++) b[c] = Xs[d][tx + 16 * c];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[r][c] = fma(a[r], b[c], acc[r][c]);
   }
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int rr = ty + 16 * r, j = t0 + tx + 16 * c;
+      if (rr >= bs || j >= m) continue;
+      Rq[(long long)rr * m + j] = acc[r][c];
+      Aq[(long long)(kb + rr) * m + j] = acc[r][c];
+    }
 }
 
 __global__ void k_symmetrise(int nMat, const long long* __restrict__ off, const int* __restrict__ size,

@@ -131,18 +131,19 @@ __global__ void k_symmetrise_pairs(int n, double* __restrict__ S) {
   S[(long long)c * n + a] = v;
 }
 
-// subdomain inverses, rows padded to a multiple of 4 (zeros past m): block per subdomain
+// subdomain inverses, rows padded to a multiple of 4 (zeros past m): kPadBlocks
+// blocks per subdomain, a warp per row (one block per subdomain with a 64-bit
+// division per entry took 340 us on level 0 at 1024^2)
+constexpr int kPadBlocks = 12;
 template <typename T>
 __global__ void k_pad_blocks(const int* __restrict__ subPtr, const long long* __restrict__ invOff, const long long* __restrict__ invOffPad,
                              const double* __restrict__ src, T* __restrict__ dst) {
-  const int p = blockIdx.x;
+  const int p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int m = subPtr[p + 1] - subPtr[p], mp = (m + 3) & ~3;
   const double* s = src + invOff[p];
   T* d = dst + invOffPad[p];
-  for (long long e = threadIdx.x; e < (long long)m * mp; e += blockDim.x) {
-    const int j = int(e / mp), a = int(e - (long long)j * mp);
-    d[e] = a < m ? T(s[(long long)j * m + a]) : T(0);
-  }
+  for (int j = blockIdx.y * warps + warp; j < m; j += gridDim.y * warps)
+    for (int a = lane; a < mp; a += 32) d[(long long)j * mp + a] = a < m ? T(s[(long long)j * m + a]) : T(0);
 }
 
 template <typename T>
@@ -153,18 +154,17 @@ __global__ void k_pad_square(int n, int np, const double* __restrict__ src, T* _
   dst[e] = a < n ? T(src[(long long)j * n + a]) : T(0);
 }
 
-// back-substitution blocks: W_p (m x t, column-major) from G_p (m x t, row-major)
+// back-substitution blocks: W_p (m x t, column-major) from G_p (m x t, row-major),
+// kPadBlocks blocks per subdomain, a warp per column
 template <typename T>
 __global__ void k_wt(const int* __restrict__ subPtr, const int* __restrict__ touchPtr, const long long* __restrict__ wOff,
                      const double* __restrict__ G, T* __restrict__ wt) {
-  const int p = blockIdx.x;
+  const int p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int m = subPtr[p + 1] - subPtr[p], t = touchPtr[p + 1] - touchPtr[p];
   const double* g = G + wOff[p];
   T* w = wt + wOff[p];
-  for (long long e = threadIdx.x; e < (long long)m * t; e += blockDim.x) {
-    const int c = int(e / m), a = int(e - (long long)c * m);
-    w[e] = T(g[(long long)a * t + c]);
-  }
+  for (int c = blockIdx.y * warps + warp; c < t; c += gridDim.y * warps)
+    for (int a = lane; a < m; a += 32) w[(long long)c * m + a] = T(g[(long long)a * t + c]);
 }
 
 // coarsest level: a source is kind << 40 | index (0 deep coefficient, 1 bd, 2 bb)
@@ -435,8 +435,8 @@ template <typename T>
 void convert_boundary(const NumericLevel& N, const BoundarySymbolic& sym, const Scaled& sc, const double* invS, const double* G,
                       const double* Ss, const double* scale64, LevelValues<T>& v, cudaStream_t s) {
   if (sym.nSub > 0) {
-    k_pad_blocks<T><<<sym.nSub, kThreads, 0, s>>>(N.subPtr, N.invOff, N.invOffPad, invS, v.inv);
-    k_wt<T><<<sym.nSub, kThreads, 0, s>>>(N.subPtr, N.touchPtr, N.wOff, G, v.wt);
+    k_pad_blocks<T><<<dim3(sym.nSub, kPadBlocks), kThreads, 0, s>>>(N.subPtr, N.invOff, N.invOffPad, invS, v.inv);
+    k_wt<T><<<dim3(sym.nSub, kPadBlocks), kThreads, 0, s>>>(N.subPtr, N.touchPtr, N.wOff, G, v.wt);
   }
   if (sym.nS > 0) {
     const long long e = (long long)sym.nS * v.nSp;
