@@ -137,9 +137,12 @@ class NumericPlan {
   bool combine(double screen, double stiffness, cudaStream_t s, std::string& err);
   // run order of a level's smoother planes (the multigrid's deep runs)
   bool set_run_order(int l, const std::vector<int>& runTexel, std::string& err);
-  // values of level l into up to two multigrids' buffers (FP32 and FP64; either
-  // may be null): the factorisations run once, in FP64, and are converted
-  bool fill_level(int l, LevelValues<float>* f32, LevelValues<double>* f64, cudaStream_t s, std::string& err);
+  // values of every level into up to two multigrids' buffers (an FP32 and an FP64
+  // one, L entries each, or empty): the factorisations run once, in FP64, and are
+  // converted.  The levels do not depend on each other: each runs on a stream of its
+  // own, after the work queued on s, and s continues after them.
+  bool fill_levels(const std::vector<LevelValues<float>>& f32, const std::vector<LevelValues<double>>& f64, cudaStream_t s,
+                   std::string& err);
   // the level-0 FP64 operator's boundary rows (same layout as the smoother's)
   bool fill_raw_rows(double* bVal, cudaStream_t s, std::string& err);
 
@@ -148,13 +151,26 @@ class NumericPlan {
   int gen = 0;                // generation: multigrids laid out for this plan carry it
   double screen = 0, stiffness = 0;
   size_t deviceBytes() const;
-  // ms of the fill_level calls since the caller last zeroed it, per phase
-  // {values and conversions, subdomain inverses, Schur products and assembly,
-  // Schur complement or coarsest inverse}
+  // device ms of the last fill_levels: from its start to the last boundary level's
+  // end, that time's shares of the phases {values and conversions, subdomain
+  // inverses, Schur products and assembly, Schur complement inverses}, and the
+  // coarsest level's inverse beyond it
   double ms[4] = {0, 0, 0, 0};
+  double boundaryMs = 0, coarseMs = 0;
 
  private:
+  struct LevelJob;
+  void queue_level(int l, const LevelValues<float>* f32, const LevelValues<double>* f64, LevelJob& job);
   DeviceArena* arena_ = nullptr;
+  // a stream and the phase marks of each level (created on first use)
+  static constexpr int kMarks = 6;
+  struct LevelStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t mark[kMarks] = {};
+  };
+  std::vector<LevelStream> streams_;
+  cudaEvent_t ready_ = nullptr;
+  bool ensure_streams(std::string& err);
 };
 
 }  // namespace gdtp

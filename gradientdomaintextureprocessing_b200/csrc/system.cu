@@ -618,8 +618,8 @@ bool DeviceSystem::assemble(const Mesh& mesh, const double* parameterMetric) {
 // coefficient hierarchy + device multigrid
 // ----------------------------------------------------------------------------
 namespace {
-bool fill_one(NumericPlan& p, int l, LevelValues<float>& v, cudaStream_t s, std::string& e) { return p.fill_level(l, &v, nullptr, s, e); }
-bool fill_one(NumericPlan& p, int l, LevelValues<double>& v, cudaStream_t s, std::string& e) { return p.fill_level(l, nullptr, &v, s, e); }
+bool fill_all(NumericPlan& p, const std::vector<LevelValues<float>>& v, cudaStream_t s, std::string& e) { return p.fill_levels(v, {}, s, e); }
+bool fill_all(NumericPlan& p, const std::vector<LevelValues<double>>& v, cudaStream_t s, std::string& e) { return p.fill_levels({}, v, s, e); }
 
 // the dense inverses and products of the set-up on the device (kernels/dense_kernels.cu)
 struct DeviceDense final : DenseBackend {
@@ -876,25 +876,17 @@ bool DeviceSystem::refresh_multigrids() {
   Multigrid<double>* m64 = mg64_.get();
   if (m32 && m32->planGen != plan_->gen) m32 = nullptr;
   if (m64 && m64->planGen != plan_->gen) m64 = nullptr;
-  std::fill(plan_->ms, plan_->ms + 4, 0.0);
-  double t0 = now_ms();
+  std::vector<LevelValues<float>> v32;
+  std::vector<LevelValues<double>> v64;
   for (int l = 0; l < levelsUsed_; l++) {
-    if (l == levelsUsed_ - 1) {
-      // boundary factorisations {values, subdomain inverses, Schur products, Schur inverse}
-      setupMs[1] = plan_->ms[0] + plan_->ms[1] + plan_->ms[2] + plan_->ms[3];
-      std::copy(plan_->ms, plan_->ms + 4, setupMs + 4);
-      t0 = now_ms();
-    }
-    LevelValues<float> v32;
-    LevelValues<double> v64;
-    if (m32) v32 = level_values(*m32, l);
-    if (m64) v64 = level_values(*m64, l);
-    if (!plan_->fill_level(l, m32 ? &v32 : nullptr, m64 ? &v64 : nullptr, stream_, err_)) {
-      err_ = "level " + std::to_string(l) + ": " + err_;
-      return false;
-    }
+    if (m32) v32.push_back(level_values(*m32, l));
+    if (m64) v64.push_back(level_values(*m64, l));
   }
-  setupMs[2] = now_ms() - t0;
+  if (!plan_->fill_levels(v32, v64, stream_, err_)) return false;
+  // boundary factorisations {values, subdomain inverses, Schur products, Schur inverse}
+  std::copy(plan_->ms, plan_->ms + 4, setupMs + 4);
+  setupMs[1] = plan_->boundaryMs;
+  setupMs[2] = plan_->coarseMs;
   setupMs[3] = 0;
   return true;
 }
@@ -1191,23 +1183,12 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
   if (numeric) {
     // every value of the layout above, on the device
     const double tLayout = now_ms() - tBuild;
-    std::fill(plan_->ms, plan_->ms + 4, 0.0);
-    for (int l = 0; l + 1 < L; l++) {
-      LevelValues<T> v = level_values(mg, l);
-      if (!fill_one(*plan_, l, v, stream_, err_)) {
-        err_ = "level " + std::to_string(l) + ": " + err_;
-        return false;
-      }
-    }
+    std::vector<LevelValues<T>> v;
+    for (int l = 0; l < L; l++) v.push_back(level_values(mg, l));
+    if (!fill_all(*plan_, v, stream_, err_)) return false;
     std::copy(plan_->ms, plan_->ms + 4, tBs);
-    tBoundary = tBs[0] + tBs[1] + tBs[2] + tBs[3];
-    const double t0 = now_ms();
-    LevelValues<T> vc = level_values(mg, L - 1);
-    if (!fill_one(*plan_, L - 1, vc, stream_, err_)) {
-      err_ = "coarsest level: " + err_;
-      return false;
-    }
-    tCoarse = now_ms() - t0;
+    tBoundary = plan_->boundaryMs;
+    tCoarse = plan_->coarseMs;
     mg.planGen = plan_->gen;
     setupMs[1] = tBoundary;
     setupMs[2] = tCoarse;
