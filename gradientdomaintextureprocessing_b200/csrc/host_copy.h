@@ -4,21 +4,27 @@
 // object: several host threads move a chunk while the copy engine moves the other.
 // A plain copy of pageable memory is one driver thread's, and a fresh destination is
 // faulted in page by page by that thread: 64 geodesic sources at 1024^2 (182 MB of
-// distances) took 63.3 ms, now 40.8, the difference all here.  Pinned memory, and copies too
-// small to gain from threads, are plain copies.
+// distances) took 63.3 ms, now 40.8, the difference all here.  A vector there and
+// back (an operator call), plain against staged: 8.6 MB 1.02 / 0.72 ms, 22.8 MB 2.6 /
+// 1.5, 91 MB 27 / 10, 183 MB 55 / 21 (chunks of 2 and 4 MB: 29 and 23); a V-cycle on
+// 3.4 MB vectors 1.24 / 0.86.  Below 2 MB waking the threads costs what the copy gains,
+// so those, and pinned memory, are plain copies.  The threads sleep between transfers:
+// an OpenMP team's idle spin cost the caller's next host operation 0.2 ms and more
+// (drawing 1 of 512^2 sources 0.53 -> 2.46 ms after a solve; with these 0.41 on both).
 //
-// One object per stream user (not for concurrent calls); the chunks are allocated on
-// the first staged copy and freed with the object.
+// One object per stream user (not for concurrent calls); the chunks and threads
+// come with the first staged copy and go with the object.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <memory>
 
 namespace gdtp {
 
 class HostCopy {
  public:
-  HostCopy() = default;
+  HostCopy();
   HostCopy(const HostCopy&) = delete;
   HostCopy& operator=(const HostCopy&) = delete;
   ~HostCopy();
@@ -29,12 +35,17 @@ class HostCopy {
   cudaError_t download(void* host, const void* device, size_t bytes, cudaStream_t s);
 
  private:
-  static constexpr size_t kChunk = size_t(4) << 20;
-  static constexpr size_t kStagedMin = size_t(1) << 20;
+  class Workers;
+  struct Transfer;
+  static constexpr size_t kChunk = size_t(8) << 20;
+  static constexpr size_t kChunkMin = size_t(1) << 20;
+  static constexpr size_t kStagedMin = size_t(2) << 20;
   static constexpr int kSlots = 2;
   bool staged(const void* host, size_t bytes);
+  static size_t piece(size_t bytes);
   unsigned char* chunks_ = nullptr;  // kSlots x kChunk, pinned
   cudaEvent_t done_[kSlots] = {};
+  std::unique_ptr<Workers> workers_;
   bool failed_ = false;              // no pinned memory to be had: plain copies
 };
 
