@@ -7,16 +7,23 @@
 // symmetric positive definite, so every pivot block is a principal block of a
 // Schur complement, itself SPD).  Step k takes the 64 pivot rows and columns
 // K = [64k, 64k + 64):
-//   P    = A[K,K]^-1                                  (k_bgj_diag, one CTA)
+//   P    = A[K,K]^-1              (k_bgj_first, then by the update of step k - 1)
 //   R    = P [A[K,:] with A[K,K] replaced by I]       (k_bgj_panel, row tiles)
 //   Cold = A[:,K] with rows K zeroed; A[i,K] = 0, i not in K (k_bgj_panel)
-//   A[K,:] = R;  A -= Cold R                          (k_gemm, rank-64 update)
+//   A[K,:] = R;  A -= Cold R                          (k_bgj_update, rank-64 update)
 // after which A[K,K] = P, A[K,j] = P A[K,j], A[i,K] = -A[i,K] P and
 // A[i,j] -= A[i,K] P A[K,j]: the n/64 steps leave A^-1.  Every matrix of a
 // batch takes part in the steps k < ceil(m/64); the update is 2 n^3 flops in
 // 64 x 64 register-tiled FP64 tiles.  A non-positive pivot sets an error flag
 // (and the result is discarded).  The result is made exactly symmetric by
 // averaging with its transpose.
+//
+// What bounds it: the steps are a chain, so a lone matrix pays each step's latency
+// (pivot inverse, panel, update) and a batch or a large matrix the update's products.
+// Steps of a 2240 x 2240 matrix (the coarsest level of a 1024^2 atlas): 49 us each
+// (panel 8.7, update 40.2 with the next pivot's inverse in it), before 95 (panel 21,
+// update 74 with the selects and 16-wide chunks) and, with the pivot in a launch of its
+// own, 160; new weights and a solve there 9.4 -> 5.3 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -107,79 +114,162 @@ __global__ void __launch_bounds__(256) k_gemm(const GemmTask* __restrict__ tasks
   }
 }
 
-// P_q = A_q[K,K]^-1 for every matrix q with m_q > 64k (one CTA each):
-// unblocked Gauss-Jordan on the pivot block, held in registers.
-__global__ void __launch_bounds__(256) k_bgj_diag(int k, const long long* __restrict__ off, const int* __restrict__ size,
-                                                  const double* __restrict__ A, double* __restrict__ Pinv, int* __restrict__ bad) {
-  const int q = blockIdx.x, m = size[q], kb = k * kPB;
-  if (kb >= m) return;
-  const int bs = min(kPB, m - kb);
-  // thread (tr, tc) holds entries (tr + 16 a, tc + 16 b), a, b < 4, in
-  // registers; the pivot row and column of each step go through shared
-  // memory, double-buffered so that one barrier per step orders them
-  const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
-  __shared__ double rowS[2][kPB], colS[2][kPB];
-  const double* Aq = A + off[q];
-  double P[4][4];
+// Product of two 64 x 64 tiles, the part [K0, K1) of the inner dimension, on 128
+// threads of 8 x 4 outputs each (rows ty + 8 r, columns tx + 16 c): 16 shared-memory
+// reads for 64 products.
+constexpr int kEThreads = 128;
+constexpr int kPitchA = kPB + 2;  // the two rows that a warp reads lie in different banks
+constexpr size_t kETile = (size_t(kPB) * kPitchA + size_t(kPB) * kPB) * sizeof(double);
+__device__ __forceinline__ void tile_product(double (&acc)[8][4], const double* As, const double* Bs, int tx, int ty, int K0, int K1) {
+#pragma unroll 4
+  for (int kk = K0; kk < K1; kk += 2) {
+    double2 a[8];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+    for (int r = 0; r < 8; r++) a[r] = *reinterpret_cast<const double2*>(As + (ty + 8 * r) * kPitchA + kk);
+    double b[4];
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int i = tr + 16 * a, j = tc + 16 * b;
-      P[a][b] = (i < bs && j < bs) ? Aq[(long long)(kb + i) * m + kb + j] : 0.0;
-    }
-  for (int s = 0; s < bs; s++) {
-    const int buf = s & 1;
-    // the pivot row s and column s as they stand before step s
+    for (int c = 0; c < 4; c++) b[c] = Bs[kk * kPB + tx + 16 * c];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-      if (tr + 16 * a == s)
+    for (int r = 0; r < 8; r++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) rowS[buf][tc + 16 * b] = P[a][b];
+      for (int c = 0; c < 4; c++) acc[r][c] = fma(a[r].x, b[c], acc[r][c]);
 #pragma unroll
-    for (int b = 0; b < 4; b++)
-      if (tc + 16 * b == s)
+    for (int c = 0; c < 4; c++) b[c] = Bs[(kk + 1) * kPB + tx + 16 * c];
 #pragma unroll
-        for (int a = 0; a < 4; a++) colS[buf][tr + 16 * a] = P[a][b];
-    __syncthreads();
-    double p = rowS[buf][s];
+    for (int r = 0; r < 8; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) acc[r][c] = fma(a[r].y, b[c], acc[r][c]);
+  }
+}
+
+// asynchronous copies to shared memory, zeros where !in
+__device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void copy16(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// queue the inner part [K0, K0 + 32) of the tiles: A rows [0, rows) (64 wide, 16-byte
+// aligned) and B rows below K, columns [0, cols) (leading dimension ldb)
+__device__ __forceinline__ void queue_half(double* As, double* Bs, const double* A, int rows, const double* B, int ldb, int K, int cols, int K0) {
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int e = threadIdx.x + kEThreads * q, r = e >> 4, c = K0 + 2 * (e & 15);
+    copy16(As + r * kPitchA + c, r < rows ? A + r * kPB + c : A, r < rows);
+  }
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int e = threadIdx.x + kEThreads * q, r = K0 + (e >> 6), c = e & 63;
+    const bool in = r < K && c < cols;
+    copy8(Bs + r * kPB + c, in ? B + (long long)r * ldb + c : B, in);
+  }
+  copies_commit();
+}
+
+// Unblocked Gauss-Jordan inverse of the bs x bs block (bs <= 64) whose entries (ty +
+// 8 r, tx + 16 c) thread (ty, tx) of 8 x 16 holds in P[r][c] (zeros past bs), in
+// registers.  The pivot row and column of each step go through shared memory (sm:
+// 2 x 3 x 64 doubles), double-buffered so that one barrier per step orders them, with
+// the next diagonal entry, so that the next pivot's reciprocal is taken beside this
+// step's update.  The steps are a chain: s = 8 sr + sy with sr unrolled fixes at
+// compile time which of a thread's entries can be in the pivot row or column (selects
+// over all 32, and the division between the barrier and the update: 0.55 us a step).
+__device__ __forceinline__ void invert_block(double (&P)[8][4], int bs, double* sm, int* __restrict__ bad) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  if (threadIdx.x == 0) sm[3 * kPB + 2 * kPB] = P[0][0];  // the second buffer's diagonal slot
+  __syncthreads();
+  auto reciprocal = [&](double p) {
     if (!(p > 0.0)) {
       if (threadIdx.x == 0) atomicExch(bad, 1);
       p = 1.0;
     }
-    const double ip = 1.0 / p;
-    // one update for every entry, the pivot row and column selected into it: a
-    // branch per entry (four cases, divergent) made a step 1.3 us.  Entries past bs
-    // stay zero.
-    double tb[4];
+    return 1.0 / p;
+  };
+  double ip = reciprocal(sm[3 * kPB + 2 * kPB]);
 #pragma unroll
-    for (int b = 0; b < 4; b++) tb[b] = rowS[buf][tc + 16 * b] * ip;
+  for (int sr = 0; sr < 8; sr++) {
+    constexpr int kLast = 7;
+    for (int sy = 0; sy < 8; sy++) {
+      const int s = 8 * sr + sy;
+      if (s >= bs) break;
+      double* rowS = sm + (s & 1) * 3 * kPB;
+      double* colS = rowS + kPB;
+      double* diag = colS + kPB;
+      const int sx = 8 * (sr & 1) + sy;  // s & 15
+      const bool row = ty == sy, col = tx == sx;
+      // the pivot row s and column s as they stand before step s
+      if (row)
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const double ca = colS[buf][tr + 16 * a], cp = -ca * ip;
-      const bool row = tr + 16 * a == s;
+        for (int c = 0; c < 4; c++) rowS[tx + 16 * c] = P[sr][c];
+      if (col)
 #pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const bool col = tc + 16 * b == s;
-        const double v = fma(-ca, tb[b], P[a][b]);
-        P[a][b] = row ? (col ? ip : tb[b]) : (col ? cp : v);
+        for (int r = 0; r < 8; r++) colS[ty + 8 * r] = P[r][sr >> 1];
+      if (ty == ((sy + 1) & 7) && tx == ((s + 1) & 15)) {
+        if (sy < 7) *diag = P[sr][sr >> 1];
+        else if (sr < kLast) *diag = P[sr < kLast ? sr + 1 : sr][(sr < kLast ? sr + 1 : sr) >> 1];
       }
+      __syncthreads();
+      double tb[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) tb[c] = rowS[tx + 16 * c] * ip;
+      // the next pivot as this step leaves it
+      double next = 1.0;
+      if (s + 1 < bs) next = fma(-colS[s + 1], rowS[s + 1] * ip, *diag);
+      const double ipn = reciprocal(next);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const double ca = colS[ty + 8 * r];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const double v = fma(-ca, tb[c], P[r][c]);
+          const bool inRow = r == sr && row, inCol = c == (sr >> 1) && col;
+          P[r][c] = inRow ? (inCol ? ip : tb[c]) : (inCol ? -ca * ip : v);
+        }
+      }
+      ip = ipn;
     }
   }
-  double* Pq = Pinv + (long long)q * kPB * kPB;
+}
+
+__device__ __forceinline__ void store_inverse(const double (&P)[8][4], double* __restrict__ Pq) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int r = 0; r < 8; r++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) Pq[(tr + 16 * a) * kPB + tc + 16 * b] = P[a][b];
+    for (int c = 0; c < 4; c++) Pq[(ty + 8 * r) * kPB + tx + 16 * c] = P[r][c];
+}
+
+// P_q = A_q[0:64, 0:64]^-1, the first pivot block of every matrix q (one CTA each;
+// the later ones are inverted by the update before them)
+__global__ void __launch_bounds__(kEThreads) k_bgj_first(const long long* __restrict__ off, const int* __restrict__ size,
+                                                         const double* __restrict__ A, double* __restrict__ Pinv, int* __restrict__ bad) {
+  const int q = blockIdx.x, m = size[q], bs = min(kPB, m), tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  if (m <= 0) return;
+  __shared__ double sm[6 * kPB];
+  const double* Aq = A + off[q];
+  double P[8][4];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int i = ty + 8 * r, j = tx + 16 * c;
+      P[r][c] = (i < bs && j < bs) ? Aq[(long long)i * m + j] : 0.0;
+    }
+  invert_block(P, bs, sm, bad);
+  store_inverse(P, Pinv + (long long)q * kPB * kPB);
 }
 
 // blockIdx.y == 0: row tile t of R = P [A[K,:], A[K,K] -> I], written to R
 // (64 x m per matrix) and to A[K,:].  blockIdx.y == 1: row tile t of
 // Cold = A[:,K] (rows K zeroed, 64 columns per row), A[i,K] = 0 for i not in K.
 // The two roles touch disjoint entries of A (rows K, and columns K outside rows K).
-__global__ void __launch_bounds__(256) k_bgj_panel(int k, const long long* __restrict__ off, const int* __restrict__ size,
-                                                   const long long* __restrict__ wsOff, double* __restrict__ A,
-                                                   const double* __restrict__ Pinv, double* __restrict__ R, double* __restrict__ Cold) {
+__global__ void __launch_bounds__(kEThreads, 3) k_bgj_panel(int k, const long long* __restrict__ off, const int* __restrict__ size,
+                                                            const long long* __restrict__ wsOff, double* A,
+                                                            const double* __restrict__ Pinv, double* __restrict__ R, double* __restrict__ Cold) {
   const int q = blockIdx.z, m = size[q], kb = k * kPB;
   if (kb >= m) return;
   const int bs = min(kPB, m - kb), t0 = blockIdx.x * kPB;
@@ -187,61 +277,114 @@ __global__ void __launch_bounds__(256) k_bgj_panel(int k, const long long* __res
   double* Aq = A + off[q];
   if (blockIdx.y == 1) {
     double* Cq = Cold + wsOff[q];
-    for (int e = threadIdx.x; e < kPB * kPB; e += 256) {
-      const int i = t0 + e / kPB, c = e % kPB;
-      if (i >= m) continue;
-      double v = 0.0;
-      if (c < bs && (i < kb || i >= kb + bs)) {
-        double* src = Aq + (long long)i * m + kb + c;
-        v = *src;
-        *src = 0.0;
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int e = threadIdx.x + kEThreads * (8 * h + u), i = t0 + (e >> 6), c = e & 63;
+        v[u] = 0.0;
+        if (i < m && c < bs && (i < kb || i >= kb + bs)) v[u] = Aq[(long long)i * m + kb + c];
       }
-      Cq[(long long)i * kPB + c] = v;
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int e = threadIdx.x + kEThreads * (8 * h + u), i = t0 + (e >> 6), c = e & 63;
+        if (i >= m) continue;
+        if (c < bs && (i < kb || i >= kb + bs)) Aq[(long long)i * m + kb + c] = 0.0;
+        Cq[(long long)i * kPB + c] = v[u];
+      }
     }
     return;
   }
-  extern __shared__ double sm[];
-  double(*Ps)[kPB + 1] = reinterpret_cast<double(*)[kPB + 1]>(sm);
-  double(*Xs)[kPB + 1] = reinterpret_cast<double(*)[kPB + 1]>(sm + kPB * (kPB + 1));
+  extern __shared__ __align__(16) double sm[];
+  double *As = sm, *Bs = sm + kPB * kPitchA;
   const double* Pq = Pinv + (long long)q * kPB * kPB;
-  for (int e = threadIdx.x; e < kPB * kPB; e += 256) {
-    const int r = e / kPB, c = e % kPB, j = t0 + c;
-    Ps[r][c] = Pq[e];
-    double x = 0.0;
-    if (r < bs && j < m) x = (j >= kb && j < kb + bs) ? (j - kb == r ? 1.0 : 0.0) : Aq[(long long)(kb + r) * m + j];
-    Xs[r][c] = x;
-  }
-  __syncthreads();
-  // 4 x 4 outputs per thread (rows ty + 16 r, columns tx + 16 c): 8 shared-memory
-  // reads for 16 products, not two for each
-  double* Rq = R + wsOff[q];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, cols = t0 == kb ? 0 : m - t0;
+  const double* X = Aq + (long long)kb * m + t0;
+  queue_half(As, Bs, Pq, kPB, X, m, bs, cols, 0);
+  queue_half(As, Bs, Pq, kPB, X, m, bs, cols, kPB / 2);
+  double acc[8][4];
 #pragma unroll
-  for (int r = 0; r < 4; r++)
+  for (int r = 0; r < 8; r++)
 #pragma unroll
     for (int c = 0; c < 4; c++) acc[r][c] = 0.0;
-#pragma unroll 4
-  for (int d = 0; d < bs; d++) {
-    double a[4], b[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) a[r] = Ps[ty + 16 * r][d];
-#pragma unroll
-    for (int c = 0; c < 4; c++) b[c] = Xs[d][tx + 16 * c];
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+  if (t0 == kb) {  // columns K: the identity
+    copies_wait<0>();
+    __syncthreads();
+    if (threadIdx.x < bs) Bs[threadIdx.x * (kPB + 1)] = 1.0;
   }
+  copies_wait<1>();
+  __syncthreads();
+  tile_product(acc, As, Bs, tx, ty, 0, kPB / 2);
+  copies_wait<0>();
+  __syncthreads();
+  tile_product(acc, As, Bs, tx, ty, kPB / 2, kPB);
+  double* Rq = R + wsOff[q];
 #pragma unroll
-  for (int r = 0; r < 4; r++)
+  for (int r = 0; r < 8; r++)
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const int rr = ty + 16 * r, j = t0 + tx + 16 * c;
+      const int rr = ty + 8 * r, j = t0 + tx + 16 * c;
       if (rr >= bs || j >= m) continue;
       Rq[(long long)rr * m + j] = acc[r][c];
       Aq[(long long)(kb + rr) * m + j] = acc[r][c];
     }
+}
+
+// A_q -= Cold_q R_q (64 x 64 tiles, one per CTA) over the step's tasks, the rank-64
+// update of elimination step kNext - 1.  The whole inner dimension is copied to shared
+// memory at once, in two halves, so that a tile waits for memory once or twice, not
+// for every 16 of the 64.  The tile of the next pivot block, taken by the task's first
+// CTA, goes on to be inverted: the inversion, a chain of 64 barriers, runs beside the
+// other tiles instead of in a launch of its own.
+__global__ void __launch_bounds__(kEThreads, 3) k_bgj_update(const GemmTask* __restrict__ tasks, const double* __restrict__ Cold,
+                                                             const double* __restrict__ R, double* __restrict__ A, int kNext,
+                                                             double* __restrict__ Pinv, int* __restrict__ bad) {
+  const GemmTask T = tasks[blockIdx.z];
+  int bx = blockIdx.x, by = blockIdx.y;
+  bool pivot = false;
+  if (kNext * kPB < T.M) {  // the next pivot block's tile changes places with the first
+    pivot = bx == 0 && by == 0;
+    if (pivot) bx = by = kNext;
+    else if (bx == kNext && by == kNext) bx = by = 0;
+  }
+  const int row0 = by * kPB, col0 = bx * kPB;
+  if (row0 >= T.M || col0 >= T.N) return;
+  extern __shared__ __align__(16) double sm[];
+  double *As = sm, *Bs = sm + kPB * kPitchA;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const double* At = Cold + T.a + (long long)row0 * kPB;
+  const double* Bt = R + T.b + col0;
+  queue_half(As, Bs, At, T.M - row0, Bt, T.ldb, T.K, T.N - col0, 0);
+  queue_half(As, Bs, At, T.M - row0, Bt, T.ldb, T.K, T.N - col0, kPB / 2);
+  double acc[8][4];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[r][c] = 0.0;
+  copies_wait<1>();
+  __syncthreads();
+  tile_product(acc, As, Bs, tx, ty, 0, kPB / 2);
+  copies_wait<0>();
+  __syncthreads();
+  tile_product(acc, As, Bs, tx, ty, kPB / 2, kPB);
+  double* Ct = A + T.c + (long long)(row0 + ty) * T.ldc + col0 + tx;
+  double P[8][4];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) P[r][c] = (row0 + ty + 8 * r < T.M && col0 + tx + 16 * c < T.N) ? Ct[(long long)(8 * r) * T.ldc + 16 * c] : 0.0;
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      P[r][c] -= acc[r][c];
+      if (row0 + ty + 8 * r < T.M && col0 + tx + 16 * c < T.N) Ct[(long long)(8 * r) * T.ldc + 16 * c] = P[r][c];
+    }
+  if (!pivot) return;
+  __syncthreads();  // As is free
+  invert_block(P, min(kPB, T.M - row0), As, bad);
+  store_inverse(P, Pinv + (long long)T.pad * kPB * kPB);
 }
 
 __global__ void k_symmetrise(int nMat, const long long* __restrict__ off, const int* __restrict__ size,
@@ -344,6 +487,7 @@ bool spd_inverse_layout(const std::vector<int64_t>& offsets, const std::vector<i
       T.ldc = m;
       T.alpha = -1.0;
       T.beta = 1.0;
+      T.pad = q;
       L.tasks.push_back(T);
       L.stepMax[k] = std::max(L.stepMax[k], m);
     }
@@ -357,17 +501,18 @@ size_t spd_inverse_scratch_doubles(const SpdInverseLayout& L) { return size_t(L.
 bool launch_spd_inverse(const SpdInverseLayout& L, const SpdInverseDevice& D, double* A, double* out, double* scratch, int* bad,
                         cudaStream_t s) {
   if (L.nMat == 0 || L.steps == 0) return true;
-  static const int panelSmem = 2 * kPB * (kPB + 1) * sizeof(double);
-  if (cudaFuncSetAttribute(k_bgj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, panelSmem) != cudaSuccess) return false;
+  for (const void* f : {reinterpret_cast<const void*>(k_bgj_panel), reinterpret_cast<const void*>(k_bgj_update)})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kETile)) != cudaSuccess) return false;
   double* pinv = scratch;
   double* rw = pinv + size_t(L.nMat) * kPB * kPB;
-  double* cw = rw + L.wsTotal;
+  double* cw = rw + L.wsTotal;  // 64 doubles a row, as pinv: rows stay 16-byte aligned
+  k_bgj_first<<<L.nMat, kEThreads, 0, s>>>(D.off, D.size, A, pinv, bad);
   for (int k = 0; k < L.steps; k++) {
     // matrices of size m <= 64k, and tiles past a matrix's own size, return at once
-    k_bgj_diag<<<L.nMat, 256, 0, s>>>(k, D.off, D.size, A, pinv, bad);
-    const dim3 pg(unsigned((L.stepMax[k] + kPB - 1) / kPB), 2, unsigned(L.nMat));
-    k_bgj_panel<<<pg, 256, panelSmem, s>>>(k, D.off, D.size, D.ws, A, pinv, rw, cw);
-    launch_gemm_batch(D.tasks + L.taskStart[k], L.taskStart[k + 1] - L.taskStart[k], L.stepMax[k], L.stepMax[k], cw, rw, A, s);
+    const unsigned tiles = unsigned((L.stepMax[k] + kPB - 1) / kPB);
+    k_bgj_panel<<<dim3(tiles, 2, unsigned(L.nMat)), kEThreads, kETile, s>>>(k, D.off, D.size, D.ws, A, pinv, rw, cw);
+    k_bgj_update<<<dim3(tiles, tiles, unsigned(L.taskStart[k + 1] - L.taskStart[k])), kEThreads, kETile, s>>>(D.tasks + L.taskStart[k], cw, rw, A,
+                                                                                                            k + 1, pinv, bad);
   }
   const unsigned blocks = unsigned((L.total + 255) / 256);
   k_symmetrise<<<blocks, 256, 0, s>>>(L.nMat, D.off, D.size, D.first, L.total, A, out);

@@ -319,7 +319,8 @@ void launch_gather_cells(int n, const int* idx, const double* src, double* dst, 
 // Dense FP64 set-up products (kernels/dense_kernels.cu).
 // One task of a batched C = alpha op(A) B + beta C (row-major, offsets in
 // doubles into the A, B and C buffers of the launch; op(A) = A (M x K) or,
-// transA, the transpose of A stored K x M).
+// transA, the transpose of A stored K x M); pad: in an elimination step's tasks the
+// matrix's index in the batch.
 struct GemmTask {
   long long a, b, c;
   int M, N, K, lda, ldb, ldc, transA, pad;
