@@ -387,20 +387,31 @@ __global__ void __launch_bounds__(kEThreads, 3) k_bgj_update(const GemmTask* __r
   store_inverse(P, Pinv + (long long)T.pad * kPB * kPB);
 }
 
-__global__ void k_symmetrise(int nMat, const long long* __restrict__ off, const int* __restrict__ size,
-                             const long long* __restrict__ first, long long total, const double* __restrict__ in, double* __restrict__ out) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  int lo = 0, hi = nMat - 1;  // the matrix of item t: last with first[q] <= t
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (first[mid] <= t) lo = mid; else hi = mid - 1;
+// out = (in + in^T) / 2, a 32 x 32 tile per CTA (32 x 8 threads) with its transpose
+// turned in shared memory: both are read along rows (an element per thread with the
+// transpose read down a column took 79 us on a 2240 x 2240 matrix, 40 MB).
+constexpr int kSymTile = 32;
+__global__ void __launch_bounds__(256) k_symmetrise(const long long* __restrict__ off, const int* __restrict__ size,
+                                                    const double* __restrict__ in, double* __restrict__ out) {
+  const int m = size[blockIdx.z], i0 = blockIdx.y * kSymTile, j0 = blockIdx.x * kSymTile;
+  if (i0 >= m || j0 >= m) return;
+  __shared__ double t[kSymTile][kSymTile + 1];
+  const double* A = in + off[blockIdx.z];
+  double* O = out + off[blockIdx.z];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  double v[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const int i = i0 + y + 8 * r, j = j0 + x, ti = j0 + y + 8 * r, tj = i0 + x;
+    v[r] = i < m && j < m ? A[(long long)i * m + j] : 0.0;
+    t[y + 8 * r][x] = ti < m && tj < m ? A[(long long)ti * m + tj] : 0.0;
   }
-  const int m = size[lo];
-  const long long e = t - first[lo];
-  const int i = int(e / m), j = int(e - (long long)i * m);
-  const double* A = in + off[lo];
-  out[off[lo] + e] = 0.5 * (A[e] + A[(long long)j * m + i]);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const int i = i0 + y + 8 * r, j = j0 + x;
+    if (i < m && j < m) O[(long long)i * m + j] = 0.5 * (v[r] + t[x][y + 8 * r]);
+  }
 }
 
 // stream-ordered scratch (no device-wide synchronisation on release, so the
@@ -457,13 +468,10 @@ bool spd_inverse_layout(const std::vector<int64_t>& offsets, const std::vector<i
   }
   L.offsets = offsets;
   L.sizes = sizes;
-  L.first.resize(L.nMat);
   L.ws.resize(L.nMat);
   int mMax = 0;
   for (int q = 0; q < L.nMat; q++) {
-    L.first[q] = L.total;
     L.ws[q] = L.wsTotal;
-    L.total += (long long)sizes[q] * sizes[q];
     L.wsTotal += (long long)kPB * sizes[q];
     L.elems = std::max<long long>(L.elems, offsets[q] + (long long)sizes[q] * sizes[q]);
     mMax = std::max(mMax, sizes[q]);
@@ -514,8 +522,8 @@ bool launch_spd_inverse(const SpdInverseLayout& L, const SpdInverseDevice& D, do
     k_bgj_update<<<dim3(tiles, tiles, unsigned(L.taskStart[k + 1] - L.taskStart[k])), kEThreads, kETile, s>>>(D.tasks + L.taskStart[k], cw, rw, A,
                                                                                                             k + 1, pinv, bad);
   }
-  const unsigned blocks = unsigned((L.total + 255) / 256);
-  k_symmetrise<<<blocks, 256, 0, s>>>(L.nMat, D.off, D.size, D.first, L.total, A, out);
+  const unsigned tiles = unsigned((L.stepMax[0] + kSymTile - 1) / kSymTile);
+  k_symmetrise<<<dim3(tiles, tiles, unsigned(L.nMat)), 256, 0, s>>>(D.off, D.size, A, out);
   return cudaGetLastError() == cudaSuccess;
 }
 
@@ -523,13 +531,13 @@ namespace {
 
 // device copies of a layout's arrays in stream-ordered scratch
 struct LayoutUpload {
-  Buf off, size, first, ws, tasks;
+  Buf off, size, ws, tasks;
   SpdInverseDevice dev;
   bool run(const SpdInverseLayout& L, cudaStream_t s, std::string& err) {
-    if (!upload(off, L.offsets, s, err) || !upload(size, L.sizes, s, err) || !upload(first, L.first, s, err) ||
+    if (!upload(off, L.offsets, s, err) || !upload(size, L.sizes, s, err) ||
         !upload(ws, L.ws, s, err) || !upload(tasks, L.tasks, s, err))
       return false;
-    dev = {off.as<long long>(), size.as<int>(), first.as<long long>(), ws.as<long long>(), tasks.as<GemmTask>()};
+    dev = {off.as<long long>(), size.as<int>(), ws.as<long long>(), tasks.as<GemmTask>()};
     return true;
   }
 };

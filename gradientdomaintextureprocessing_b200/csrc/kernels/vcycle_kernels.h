@@ -333,15 +333,14 @@ void launch_gemm_batch(const GemmTask* dTasks, int nTasks, int maxM, int maxN, c
 // its device arrays (uploaded by the caller from the layout's vectors).
 struct SpdInverseLayout {
   int nMat = 0, steps = 0;
-  long long total = 0, elems = 0, wsTotal = 0;
-  std::vector<int64_t> offsets, first, ws;
+  long long elems = 0, wsTotal = 0;
+  std::vector<int64_t> offsets, ws;
   std::vector<int> sizes, taskStart, stepMax;
   std::vector<GemmTask> tasks;
 };
 struct SpdInverseDevice {
   const long long* off;
   const int* size;
-  const long long* first;
   const long long* ws;
   const GemmTask* tasks;
 };

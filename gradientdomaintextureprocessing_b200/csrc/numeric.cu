@@ -346,7 +346,7 @@ bool NumericPlan::build(const Hierarchy& h, int L_, const FineSystem& fine, cons
     }
   // ---- resident sources and structure arrays (device)
   auto layout_dev = [&](const dev::SpdInverseLayout& Ly) -> dev::SpdInverseDevice {
-    return {A.upload(as_ll(Ly.offsets)), A.upload(Ly.sizes), A.upload(as_ll(Ly.first)), A.upload(as_ll(Ly.ws)), A.upload(Ly.tasks)};
+    return {A.upload(as_ll(Ly.offsets)), A.upload(Ly.sizes), A.upload(as_ll(Ly.ws)), A.upload(Ly.tasks)};
   };
   for (int l = 0; l < L; l++) {
     NumericLevel& N = levels[l];
@@ -591,9 +591,11 @@ void NumericPlan::queue_level(int l, const LevelValues<float>* f32, const LevelV
 }
 
 // What bounds it: each level is a chain of small dependent launches (an
-// elimination step of the coarsest matrix is three), some 100 in all for 1024^2, and
-// the levels in turn left most of the chip idle.  Side by side the chain of the
-// coarsest level, queued first, hides the others: re-weighting and solve 13.35 -> 9.4 ms.
+// elimination step of the coarsest matrix is two), some 100 in all for 1024^2, and
+// the levels in turn left most of the chip idle.  Side by side the chains of level 0
+// and of the coarsest level, queued first, hide the others: re-weighting and solve
+// 13.35 -> 9.4 ms (5.0 with the later, faster inverses).  The coarsest level's stream
+// at a higher priority: 5.35, level 0 waits.
 bool NumericPlan::fill_levels(const std::vector<LevelValues<float>>& f32, const std::vector<LevelValues<double>>& f64, cudaStream_t s,
                               std::string& err) {
   if (!ensure_streams(err)) return false;
