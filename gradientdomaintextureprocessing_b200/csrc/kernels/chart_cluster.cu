@@ -28,10 +28,15 @@
 // takes 1.9 us (256^2 torus, 8 CTAs a chart), and a smoothing step of 3 sweeps 12
 // instead of 22 us.  Per refinement step: 256^2 torus 187 -> 134 us, 1024^2 genus-2
 // (one channel) 209 -> 153 us.
-// Which charts: up to 512 pairs of one row parity in each of 8 CTAs.  Larger charts
-// (to 1024 pairs, coefficients in shared memory) were built and measured: at one
-// CTA per SM only 15 clusters of 8 are resident, so 16 charts took two waves, 42 us
-// against 36 for the row launches.
+// Which charts: up to 512 pairs of one row parity in each of 8 CTAs, the coefficients
+// in registers; larger ones, up to 1024 pairs with the coefficients in shared memory
+// (one CTA per SM), where one wave holds every cluster: 15 are resident, and a second
+// wave takes as long as the row launches (42 us against 36 for 3 sweeps).  Smaller
+// charts share a cluster's CTAs (build_chart_clusters): the 8 large and 8 small charts
+// of a 1024^2 icosphere atlas are 12 clusters, not 16, so its level 0 runs in one wave:
+// 305 -> 275 us per refinement step.  Fewer CTAs for small charts elsewhere: 725 x 611
+// with 15 right-hand sides 413 -> 400, 256^2 torus 117 -> 112, 1024^2 genus-2 (one
+// channel) 130.4 -> 127.7, FP64 values at 1024^2 399 -> 393 us.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_gs_cluster(const ClusterPart* __
 
   auto half = [&](auto hc, bool push) {
     constexpr int h = decltype(hc)::value;
-    half_sweep<T, W, (MINB == 1)>(
+    half_sweep<T, W, (MINB == 1 && MAXT <= kClusterMaxThreads)>(
         slab, pos[h], [&](int k) -> T { return CREG ? wr[h][CREG ? k : 0] : sw[(18 * h + k) * nt + tid]; },
         [&](int k) -> Vec<T, W> { return BREG ? br[h][BREG ? k : 0] : sb[(2 * h + k) * nt + tid]; }, push);
   };
@@ -286,8 +291,8 @@ size_t cluster_smem(int slabMax, int threads) {
   return size_t(slabMax) * sizeof(Vec<T, W>) + (BREG ? 0 : size_t(4) * threads * sizeof(Vec<T, W>)) + (CREG ? 0 : size_t(36) * threads * sizeof(T));
 }
 
-// shared memory attribute set, and at least one cluster of 8 CTAs at the largest
-// size resident: 1, else 0 (per device, once)
+// shared memory attribute set, and the clusters resident at the largest size (per
+// device, once)
 template <typename T, int W, int MAXT, int MINB, bool CREG, bool BREG>
 int cluster_ready() {
   static std::atomic<int> slots[kMaxDevices];
@@ -316,7 +321,7 @@ int cluster_ready() {
       cudaGetLastError();
       return 0;
     }
-    return clusters > 0 ? 1 : 0;
+    return clusters;
   });
 }
 
@@ -352,11 +357,18 @@ bool launch_variant(const LevelDev<T>& D, int sweeps, bool reverse, bool zeroSta
 
 }  // namespace
 
+// the large layout: in one wave (one CTA per SM), its coefficients in shared memory
+template <typename T, int W>
+static bool large_in_one_wave(const LevelDev<T>& D, int KP) {
+  return cluster_fits<T, W, kClusterLargeThreads, 1, false, true>(D) &&
+         (long long)(D.nClusterParts / D.clusterSize) * (KP / W) <= cluster_ready<T, W, kClusterLargeThreads, 1, false, true>();
+}
+
 template <typename T, int W>
 bool gs_cluster_available(const LevelDev<T>& D, int KP) {
   if (D.clusterThreads == 0 || (long long)D.nClusterParts * (KP / W) > kClusterMaxCtas) return false;
   if constexpr (std::is_same<T, float>::value)
-    return cluster_fits<T, W, 320, 2, true, false>(D) || cluster_fits<T, W, 512, 1, true, true>(D);
+    return cluster_fits<T, W, 320, 2, true, false>(D) || cluster_fits<T, W, 512, 1, true, true>(D) || large_in_one_wave<T, W>(D, KP);
   else
     return cluster_fits<T, W, 512, 1, false, false>(D);
 }
@@ -371,6 +383,8 @@ bool launch_gs_cluster(const LevelDev<T>& D, int sweeps, bool reverse, bool zero
   if constexpr (std::is_same<T, float>::value) {
     if (cluster_fits<T, W, 320, 2, true, false>(D)) return launch_variant<T, W, 320, 2, true, false>(D, sweeps, reverse, zeroStart, KP, s, rhsEarly);
     if (cluster_fits<T, W, 512, 1, true, true>(D)) return launch_variant<T, W, 512, 1, true, true>(D, sweeps, reverse, zeroStart, KP, s, rhsEarly);
+    if (large_in_one_wave<T, W>(D, KP))
+      return launch_variant<T, W, kClusterLargeThreads, 1, false, true>(D, sweeps, reverse, zeroStart, KP, s, rhsEarly);
   } else {
     if (cluster_fits<T, W, 512, 1, false, false>(D)) return launch_variant<T, W, 512, 1, false, false>(D, sweeps, reverse, zeroStart, KP, s, rhsEarly);
   }

@@ -37,6 +37,7 @@ struct ClusterPart {
 };
 constexpr size_t kClusterSmemMax = 227 * 1024;
 constexpr int kClusterMaxThreads = 512;
+constexpr int kClusterLargeThreads = 1024;  // larger charts, where one wave holds them
 
 // Longest j chunk of a boundary dense product (its input vector is staged in
 // shared memory): subdomains hold at most this many rows, and the separator

@@ -143,7 +143,8 @@ bool build_row_bins(const GridLevel& L, const DeepRuns& R, RowBins& out) {
 
 // The smallest cluster whose CTAs have at most kClusterThreadsGoal pairs per row
 // parity; the largest cluster when none does.  False (cluster smoother unused)
-// when the rows do not fit 8 CTAs or an index its packed field.
+// when the rows do not fit 8 CTAs or an index its packed field.  Charts that need
+// fewer CTAs than the largest share a cluster.
 static constexpr int kClusterThreadsGoal = 256;
 bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& out) {
   out = ChartClusters();
@@ -166,28 +167,64 @@ bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& 
     rc.back().lines.push_back((int)li);
     rc.back().deep += l.end - l.start + 1;
   }
+  // rows [cut[p], cut[p + 1]) of a chart go to part p of K: at least one while rows
+  // remain; and the most pairs that a part has of one row parity
+  auto deal = [](const std::vector<Row>& rc, int K, std::vector<int>& cut) {
+    long long total = 0, done = 0;
+    for (const Row& r : rc) total += r.deep;
+    cut.assign(K + 1, (int)rc.size());
+    cut[0] = 0;
+    int at = 0;
+    for (int p = 0; p < K; p++) {
+      cut[p] = at;
+      const int from = at;
+      while (at < (int)rc.size() && (at == from || (done + rc[at].deep / 2) * K <= total * (p + 1))) done += rc[at++].deep;
+      if (p == K - 1)
+        while (at < (int)rc.size()) done += rc[at++].deep;
+    }
+  };
+  auto most_pairs = [&](const std::vector<Row>& rc, int K, std::vector<int>& cut) {
+    deal(rc, K, cut);
+    int most = 0;
+    for (int p = 0; p < K; p++) {
+      int n[2] = {0, 0};
+      for (int r = cut[p]; r < cut[p + 1]; r++)
+        for (int li : rc[r].lines) n[rc[r].cj & 1] += (L.rasterLines[li].end - L.rasterLines[li].start + 2) / 2;
+      most = std::max(most, std::max(n[0], n[1]));
+    }
+    return most;
+  };
   for (int C = 1; C <= 8; C *= 2) {
     ChartClusters cc;
     cc.size = C;
+    std::vector<int> cut;
+    // the largest chart takes a whole cluster; a smaller one as few CTAs as leave it no
+    // more pairs per CTA than that, and charts share a cluster's CTAs (largest first)
     int pairs = 0;
+    for (const std::vector<Row>& rc : rows) pairs = std::max(pairs, most_pairs(rc, C, cut));
+    std::vector<std::pair<int, int>> order;  // (-CTAs, chart)
     for (int c = 0; c < nc; c++) {
+      if (rows[c].empty()) continue;
+      int K = 1;
+      while (K < C && most_pairs(rows[c], K, cut) > pairs) K++;
+      order.emplace_back(-K, c);
+    }
+    std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+    std::vector<int> room;  // CTAs left in each cluster
+    for (const auto& [negK, c] : order) {
+      const int K = -negK;
       const std::vector<Row>& rc = rows[c];
-      if (rc.empty()) continue;
-      long long total = 0, done = 0;
-      for (const Row& r : rc) total += r.deep;
-      // rows [cut[p], cut[p + 1]) go to part p: at least one while rows remain
-      std::vector<int> cut(C + 1, (int)rc.size());
-      cut[0] = 0;
-      int at = 0;
-      for (int p = 0; p < C; p++) {
-        cut[p] = at;
-        const int from = at;
-        while (at < (int)rc.size() && (at == from || (done + rc[at].deep / 2) * C <= total * (p + 1))) done += rc[at++].deep;
-        if (p == C - 1)
-          while (at < (int)rc.size()) done += rc[at++].deep;
+      size_t at = 0;
+      while (at < room.size() && room[at] < K) at++;
+      if (at == room.size()) {
+        room.push_back(C);
+        cc.parts.resize(cc.parts.size() + C);
       }
-      std::vector<dev::ClusterPart> parts(C);
-      for (int p = 0; p < C; p++) {
+      const size_t base = at * C + (C - room[at]);
+      room[at] -= K;
+      deal(rc, K, cut);
+      std::vector<dev::ClusterPart> parts(K);
+      for (int p = 0; p < K; p++) {
         dev::ClusterPart& P = parts[p];
         P = dev::ClusterPart();
         if (cut[p] == cut[p + 1]) continue;
@@ -204,9 +241,9 @@ bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& 
         P.count = hi - lo + 1;
         cc.slab = std::max(cc.slab, P.count);
       }
-      for (int p = 0; p < C; p++) {
+      for (int p = 0; p < K; p++) {
         dev::ClusterPart& P = parts[p];
-        const bool up = p > 0 && parts[p - 1].count > 0, dn = p + 1 < C && parts[p + 1].count > 0;
+        const bool up = p > 0 && parts[p - 1].count > 0, dn = p + 1 < K && parts[p + 1].count > 0;
         if (up) { P.upLo = parts[p - 1].lo; P.upCount = parts[p - 1].count; }
         if (dn) { P.dnLo = parts[p + 1].lo; P.dnCount = parts[p + 1].count; }
         for (int par = 0; par < 2; par++) {
@@ -231,14 +268,13 @@ bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& 
             }
           }
           P.nItems[par] = (int)cc.items.size() - P.item0[par];
-          pairs = std::max(pairs, P.nItems[par]);
         }
-        cc.parts.push_back(P);
+        cc.parts[base + p] = P;
       }
     }
     cc.threads = std::max(32, (pairs + 31) / 32 * 32);
     cc.slab = (cc.slab + 1) & ~1;  // the kernel may swap the entries of a pair (slab_slot)
-    if (cc.threads <= kClusterThreadsGoal || (C == 8 && cc.threads <= dev::kClusterMaxThreads)) {
+    if (cc.threads <= kClusterThreadsGoal || (C == 8 && cc.threads <= dev::kClusterLargeThreads)) {
       out = std::move(cc);
       return !out.parts.empty();
     }

@@ -89,7 +89,7 @@ def test_coarsest_solve_at_every_size(torus, ico, max_coarse, precision):
 
 
 @pytest.fixture(scope="module", params=[("torus", 256, 256), ("torus", 301, 277), ("icosphere", 512, 512), ("icosphere", 905, 643),
-                                        ("genus2", 643, 905)])
+                                        ("icosphere", 1024, 1024), ("genus2", 643, 905)])
 def atlas(request, built_lib):
     from gradientdomaintextureprocessing_b200 import meshgen
     from gradientdomaintextureprocessing_b200.hierarchy import InitializeHierarchy
