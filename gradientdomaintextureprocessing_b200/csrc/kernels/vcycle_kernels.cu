@@ -809,6 +809,31 @@ __device__ __forceinline__ void prefetch_l2_block(const void* p, long long bytes
     asm volatile("prefetch.global.L2 [%0];" ::"l"(c + o));
 }
 
+// Sums of N values over the warp's lanes, each in the order of a shuffle-down tree
+// (lanes l and l + 16, then l + 8, ...).  While a lane holds several values it keeps
+// half of them and hands the other half over, so the whole takes N - 1 + log2(32 / N)
+// shuffles (N <= 32), not 5 N.  Afterwards value i is in v[i % own] of lane (i / own)
+// lanes, with own = max(1, N / 32) and lanes = max(1, 32 / N).
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&v)[N], int lane) {
+  static_assert(N >= 1 && N <= 64 && (N & (N - 1)) == 0, "a power of two");
+#pragma unroll
+  for (int step = 0; step < 5; step++) {
+    const int s = 16 >> step, half = (N >> step) / 2;
+    if (half > 0) {
+      const bool upper = lane & s;
+#pragma unroll
+      for (int i = 0; i < N / 2; i++)
+        if (i < half) {
+          const double give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], s);
+    }
+  }
+}
+
 // ----------------------------------------------------------------------------
 // Coarsest level: x = D Ainv^ D rhs with the scaled dense inverse (FP64): a
 // stream of the n x n inverse.  A block takes 2 R rows, a warp one part of the
@@ -816,6 +841,11 @@ __device__ __forceinline__ void prefetch_l2_block(const void* p, long long bytes
 // channel groups: a value of the inverse is used for Q W channels, and a
 // right-hand side value, widened to FP64 once, for R rows.  What bounds it is
 // the loads in flight: a lane loads U of its j at once, before their updates.
+// With several channel groups it was the lines that a load touched (a lane's row of
+// the right-hand side) and the shuffles of R Q W sums: with the rows staged and
+// warp_sums, per refinement step at 1024^2, 64 right-hand sides 2120 -> 2078 us (17 of
+// it warp_sums), 32 1096 -> 1075, 16 653 -> 648; 725 x 611 with 15 397 -> 394; up to 4
+// no difference.
 // ----------------------------------------------------------------------------
 template <typename T, int W, int R, int Q, int U>
 __global__ void __launch_bounds__(256, Q == 1 ? 2 : 1) k_coarse_solve(int n, const double* __restrict__ ainv, const double* __restrict__ scale,
@@ -840,43 +870,102 @@ __global__ void __launch_bounds__(256, Q == 1 ? 2 : 1) k_coarse_solve(int n, con
   const double* arow[R];
 #pragma unroll
   for (int r = 0; r < R; r++) arow[r] = ainv + (long long)min(row0 + r, n - 1) * n;  // rows past n: computed, not stored
-  for (int j = j0 + lane; j < j1; j += 32 * U) {
-    double w[U][R], sc[U];
-    Vec<T, W> v[U][Q];
+  if constexpr (Q > 1 && sizeof(T) == 4) {
+    // several FP32 channel groups: a chunk of 32 rows of the right-hand side comes in
+    // contiguous pieces (a lane reading its whole row touches 32 lines per load), one
+    // chunk ahead, and each lane takes its row from shared memory
+    constexpr int kRow = Q * W * int(sizeof(T)), kPieces = kRow / 16, kPitch = kRow + 16;
+    static_assert(kRow % 16 == 0, "16-byte pieces");
+    __shared__ __align__(16) unsigned char stage[8][2][32 * kPitch];
+    auto queue = [&](int j, int buf) {  // rows j .. j + 31 below j1
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int ju = j + 32 * u;
-      if (ju < j1) {
-#pragma unroll
-        for (int r = 0; r < R; r++) w[u][r] = __ldg(arow[r] + ju);
-        sc[u] = scale[ju];
-#pragma unroll
-        for (int q = 0; q < Q; q++) v[u][q] = vload<T, W>(rhs + (long long)ju * KP + c0 + q * W);
+      for (int u = 0; u < kPieces; u++) {
+        const int e = lane + 32 * u, row = e / kPieces, piece = e % kPieces;
+        if (j + row < j1)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(&stage[warp][buf][row * kPitch + piece * 16])),
+                       "l"(reinterpret_cast<const char*>(rhs + (long long)(j + row) * KP + c0) + piece * 16)
+                       : "memory");
       }
-    }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double wn[R], scn = 0;
+    auto fetch = [&](int j) {
+      if (j < j1) {
 #pragma unroll
-    for (int u = 0; u < U; u++)
-      if (j + 32 * u < j1) {
+        for (int r = 0; r < R; r++) wn[r] = __ldg(arow[r] + j);
+        scn = scale[j];
+      }
+    };
+    if (j0 < j1) queue(j0, 0);
+    fetch(j0 + lane);
+    for (int jb = j0, buf = 0; jb < j1; jb += 32, buf ^= 1) {
+      const int j = jb + lane;
+      double w[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) w[u][r] = w[u][r] * sc[u];
+      for (int r = 0; r < R; r++) w[r] = wn[r] * scn;
+      if (jb + 32 < j1) {
+        queue(jb + 32, buf ^ 1);
+        fetch(j + 32);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncwarp();
+      if (j < j1)
 #pragma unroll
-        for (int q = 0; q < Q; q++)
+        for (int q = 0; q < Q; q++) {
+          const Vec<T, W> v = *reinterpret_cast<const Vec<T, W>*>(&stage[warp][buf][lane * kPitch + q * W * int(sizeof(T))]);
 #pragma unroll
           for (int c = 0; c < W; c++) {
-            const double d = double(v[u][q].v[c]);
+            const double d = double(v.v[c]);
 #pragma unroll
-            for (int r = 0; r < R; r++) acc[r][q * W + c] += w[u][r] * d;
+            for (int r = 0; r < R; r++) acc[r][q * W + c] = fma(w[r], d, acc[r][q * W + c]);
           }
+        }
+      __syncwarp();  // before this buffer is filled again
+    }
+  } else {
+    for (int j = j0 + lane; j < j1; j += 32 * U) {
+      double w[U][R], sc[U];
+      Vec<T, W> v[U][Q];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int ju = j + 32 * u;
+        if (ju < j1) {
+#pragma unroll
+          for (int r = 0; r < R; r++) w[u][r] = __ldg(arow[r] + ju);
+          sc[u] = scale[ju];
+#pragma unroll
+          for (int q = 0; q < Q; q++) v[u][q] = vload<T, W>(rhs + (long long)ju * KP + c0 + q * W);
+        }
       }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (j + 32 * u < j1) {
+#pragma unroll
+          for (int r = 0; r < R; r++) w[u][r] = w[u][r] * sc[u];
+#pragma unroll
+          for (int q = 0; q < Q; q++)
+#pragma unroll
+            for (int c = 0; c < W; c++) {
+              const double d = double(v[u][q].v[c]);
+#pragma unroll
+              for (int r = 0; r < R; r++) acc[r][q * W + c] += w[u][r] * d;
+            }
+        }
+    }
   }
+  constexpr int kValues = R * Q * W, kOwn = kValues > 32 ? kValues / 32 : 1, kLanes = kValues > 32 ? 1 : 32 / kValues;
+  double sums[kValues];
 #pragma unroll
-  for (int r = 0; r < R; r++)
+  for (int i = 0; i < kValues; i++) sums[i] = acc[i / (Q * W)][i % (Q * W)];
+  warp_sums(sums, lane);
+  if (lane % kLanes == 0)
 #pragma unroll
-    for (int c = 0; c < Q * W; c++) {
-      double v = acc[r][c];
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
-      if (lane == 0) part[rl][r][p][c] = v;
+    for (int u = 0; u < kOwn; u++) {
+      const int i = lane / kLanes * kOwn + u;
+      part[rl][i / (Q * W)][p][i % (Q * W)] = sums[u];
     }
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * R * Q * W; i += blockDim.x) {

@@ -88,6 +88,23 @@ def test_coarsest_solve_at_every_size(torus, ico, max_coarse, precision):
         np.testing.assert_array_equal(got, ref)
 
 
+@pytest.mark.parametrize("k", [6, 16, 40])
+@pytest.mark.parametrize("max_coarse", [2600, 600, 260])
+def test_coarsest_solve_of_wide_batches(torus, ico, max_coarse, k):
+    """Right-hand sides staged in chunks of 32 rows: one column alone and among k."""
+    for s in (torus, ico):
+        b, x = (v.astype(np.float32) for v in vectors(s.n, k))
+        try:
+            s.set("max_coarse", max_coarse)
+            s.update(1e-3, 1.0)
+            wide = s.vcycle(x, b)
+            for c in (0, k - 1):
+                np.testing.assert_array_equal(wide[:, c], s.vcycle(x[:, c], b[:, c])[:, 0])
+        finally:
+            s.set("max_coarse", 2600)
+            s.update(1e-3, 1.0)
+
+
 @pytest.fixture(scope="module", params=[("torus", 256, 256), ("torus", 301, 277), ("icosphere", 512, 512), ("icosphere", 905, 643),
                                         ("icosphere", 1024, 1024), ("genus2", 643, 905)])
 def atlas(request, built_lib):
