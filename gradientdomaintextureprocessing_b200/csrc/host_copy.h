@@ -5,9 +5,10 @@
 // A plain copy of pageable memory is one driver thread's, and a fresh destination is
 // faulted in page by page by that thread: 64 geodesic sources at 1024^2 (182 MB of
 // distances) took 63.3 ms, now 40.8, the difference all here.  A vector there and
-// back (an operator call), plain against staged: 8.6 MB 1.02 / 0.72 ms, 22.8 MB 2.6 /
-// 1.5, 91 MB 27 / 10, 183 MB 55 / 21 (chunks of 2 and 4 MB: 29 and 23); a V-cycle on
-// 3.4 MB vectors 1.24 / 0.86.  Below 2 MB waking the threads costs what the copy gains,
+// back (an operator call), plain against staged: 8.6 MB 1.02 / 0.65 ms, 22.8 MB 2.6 /
+// 1.2, 91 MB 27 / 8.2, 183 MB 55 / 16.6 (chunks of 2 and 4 MB 29 and 23; 10 or 14
+// threads the same: fresh pages bound it); a V-cycle on 3.4 MB vectors 1.24 / 0.86.
+// Below 2 MB waking the threads costs what the copy gains,
 // so those, and pinned memory, are plain copies.  The threads sleep between transfers:
 // an OpenMP team's idle spin cost the caller's next host operation 0.2 ms and more
 // (drawing 1 of 512^2 sources 0.53 -> 2.46 ms after a solve; with these 0.41 on both).

@@ -221,3 +221,34 @@ def test_host_vcycle_and_sweeps(ico, k):
     x0 = x.copy()
     ico.vcycle(x, b)
     np.testing.assert_array_equal(x, x0)
+
+
+@pytest.mark.parametrize("k", [5, 8, 12, 16, 33, 48, 60, 64])
+def test_operator_columns_do_not_depend_on_the_width(ico, k):
+    """One column of A x alone and among k: the same products in the same order."""
+    x, _ = vectors(ico.n, k, seed=k)
+    y = ico.apply(x)
+    for c in (0, k // 2, k - 1):
+        np.testing.assert_array_equal(y[:, c], ico.apply(np.ascontiguousarray(x[:, c:c + 1]))[:, 0])
+
+
+@pytest.mark.parametrize("k", [8, 12, 64])
+def test_device_vectors_at_any_offset(ico, k):
+    """Device vectors that start at an odd multiple of 8 bytes: the same iterate."""
+    import ctypes as C
+
+    import torch
+    from gradientdomaintextureprocessing_b200 import _lib
+    b, x = vectors(ico.n, k, seed=k)
+    got = []
+    for shift in (0, 1):
+        buf = torch.zeros((2, b.size + 4), dtype=torch.float64, device="cuda")
+        bd, xd = buf[0, shift:shift + b.size], buf[1, shift:shift + b.size]
+        bd.copy_(torch.from_numpy(b.ravel()))
+        xd.copy_(torch.from_numpy(x.ravel()))
+        rep = _lib.Report()
+        _lib.lib().gdtp_solve_device(ico.handle, C.c_void_p(bd.data_ptr()), C.c_void_p(xd.data_ptr()), k, 1e-300, 2,
+                                     C.c_void_p(torch.cuda.current_stream().cuda_stream), C.byref(rep))  # not converged after 2
+        assert rep.iterations == 2
+        got.append(xd.cpu().numpy())
+    np.testing.assert_array_equal(got[0], got[1])
