@@ -1420,16 +1420,41 @@ __global__ void k_unpack(const T* __restrict__ padded, T* __restrict__ tight, lo
 // (its padding lanes stay zero through the V-cycle).  Columns with frozen[c]
 // set keep their x: a right-hand side that has converged stops changing, so
 // its result does not depend on what it was solved together with.
-template <typename T>
-__global__ void k_add_correction(double* __restrict__ x, T* __restrict__ e, long long n, int K, int KP, const int* __restrict__ frozen) {
+// PER values per thread, their loads issued together, and 32-bit divisions (small:
+// n K < 2^32).  Four values where that still fills the chip: per refinement step 64
+// right-hand sides at 1024^2 1961 -> 1942 us, 16 623 -> 617, 2048^2 644 -> 640.5, FP64
+// values at 1024^2 392.6 -> 388; one below (256^2 torus 116.2, with four 116.8).
+template <typename T, int PER>
+__global__ void __launch_bounds__(256) k_add_correction(double* __restrict__ x, T* __restrict__ e, long long n, int K, int KP,
+                                                        const int* __restrict__ frozen, int small) {
   grid_dependency_wait();
   grid_launch_dependents();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * K) return;
-  const long long i = t / K;
-  const int c = int(t - i * K);
-  if (!frozen || !frozen[c]) x[t] += double(e[i * KP + c]);
-  e[i * KP + c] = T(0);
+  const long long t0 = (long long)blockIdx.x * (256 * PER) + threadIdx.x, total = n * K;
+  double xv[PER];
+  T ev[PER];
+  long long at[PER];
+  bool go[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const long long t = t0 + 256 * u;
+    go[u] = false;
+    if (t >= total) continue;
+    const long long i = small ? (long long)((unsigned)t / (unsigned)K) : t / K;
+    const int c = int(t - i * K);
+    at[u] = i * KP + c;
+    go[u] = !frozen || !frozen[c];
+    if (go[u]) {
+      xv[u] = x[t];
+      ev[u] = e[at[u]];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const long long t = t0 + 256 * u;
+    if (t >= total) continue;
+    if (go[u]) x[t] = xv[u] + double(ev[u]);
+    e[at[u]] = T(0);
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -1790,7 +1815,11 @@ void launch_set_flags(int* flags, unsigned long long mask, int k, cudaStream_t s
 }
 template <typename T>
 void launch_add_correction(double* x, T* e, long long n, int K, int KP, cudaStream_t s, const int* frozen) {
-  launch(k_add_correction<T>, dim3(nblk(n * K)), s, x, e, n, K, KP, frozen);
+  const long long total = n * K;
+  const int small = total <= 0xffffffffLL ? 1 : 0;
+  // one value per thread up to two waves of threads (148 SMs of 2048)
+  if (total <= 2 * 148 * 2048LL) launch(k_add_correction<T, 1>, dim3(nblk(total)), s, x, e, n, K, KP, frozen, small);
+  else launch(k_add_correction<T, 4>, dim3(nblk((total + 3) / 4)), s, x, e, n, K, KP, frozen, small);
 }
 
 #define GDTP_INSTANTIATE(T, W)                                                                                             \
