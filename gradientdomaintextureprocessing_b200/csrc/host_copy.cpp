@@ -109,86 +109,143 @@ class HostCopy::Workers {
   std::vector<std::thread> threads_;
 };
 
-// the workers are awake while this is in scope
+// Two pinned chunks, the events after their last copies, and the threads
+struct HostCopy::Set {
+  unsigned char* chunks = nullptr;  // kSlots x kChunk
+  cudaEvent_t done[kSlots] = {};
+  cudaStream_t last = nullptr;      // stream of the last copy
+  Workers workers;
+  bool taken = true;
+  // both chunks have been left
+  bool idle() const {
+    for (cudaEvent_t e : done)
+      if (cudaEventQuery(e) != cudaSuccess) {
+        if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // not an error of the caller's
+        return false;
+      }
+    return true;
+  }
+  bool make() {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kSlots * kChunk, cudaHostAllocDefault) != cudaSuccess) return false;
+    chunks = static_cast<unsigned char*>(p);
+    for (cudaEvent_t& e : done)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        return false;
+      }
+    return true;
+  }
+  ~Set() {
+    for (cudaEvent_t e : done)
+      if (e) {
+        cudaEventSynchronize(e);
+        cudaEventDestroy(e);
+      }
+    if (chunks) cudaFreeHost(chunks);
+  }
+};
+
+// a set in use by one copy; its workers are awake while this is in scope
 struct HostCopy::Transfer {
-  explicit Transfer(Workers& w) : w(w) { w.begin(); }
-  ~Transfer() { w.end(); }
-  Workers& w;
+  Transfer(HostCopy& owner, Set* set) : owner(owner), set(set) { set->workers.begin(); }
+  ~Transfer() {
+    set->workers.end();
+    owner.give(set);
+  }
+  HostCopy& owner;
+  Set* set;
 };
 
 HostCopy::HostCopy() = default;
+HostCopy::~HostCopy() = default;
 
-HostCopy::~HostCopy() {
-  for (cudaEvent_t e : done_)
-    if (e) cudaEventDestroy(e);
-  if (chunks_) cudaFreeHost(chunks_);
-}
-
-// the copy goes through the pinned chunks (allocated here on first use)
-bool HostCopy::staged(const void* host, size_t bytes) {
-  if (failed_ || bytes < kStagedMin) return false;
+// A free set whose chunks are idle, or are left in the order of s: another stream's
+// pending work is not waited for.  None: a new set, up to kMaxSets.
+HostCopy::Set* HostCopy::take(const void* host, size_t bytes, cudaStream_t s) {
+  if (bytes < kStagedMin) return nullptr;
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return nullptr;
   }
-  if (at.type != cudaMemoryTypeUnregistered) return false;
-  if (chunks_) return true;
-  void* p = nullptr;
-  bool ok = cudaHostAlloc(&p, kSlots * kChunk, cudaHostAllocDefault) == cudaSuccess;
-  for (cudaEvent_t& e : done_) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
-    if (p) cudaFreeHost(p);
-    failed_ = true;
-    return false;
+  if (at.type != cudaMemoryTypeUnregistered) return nullptr;
+  Set* made;
+  {
+    std::lock_guard<std::mutex> l(m_);
+    for (std::unique_ptr<Set>& set : sets_)
+      if (!set->taken && (set->last == s || set->idle())) {
+        set->taken = true;
+        set->last = s;
+        return set.get();
+      }
+    if (failed_ || sets_.size() >= kMaxSets) return nullptr;
+    sets_.push_back(std::make_unique<Set>());
+    made = sets_.back().get();
+    made->last = s;
   }
-  chunks_ = static_cast<unsigned char*>(p);
-  workers_ = std::make_unique<Workers>();
-  return true;
+  if (made->make()) return made;  // (allocated while other copies go on)
+  cudaGetLastError();
+  std::lock_guard<std::mutex> l(m_);
+  failed_ = true;
+  sets_.erase(std::find_if(sets_.begin(), sets_.end(), [made](const std::unique_ptr<Set>& set) { return set.get() == made; }));
+  return nullptr;
+}
+
+void HostCopy::give(Set* set) {
+  std::lock_guard<std::mutex> l(m_);
+  set->taken = false;
 }
 
 // a quarter of the vector, so that the two sides overlap, within the chunk's size
 size_t HostCopy::piece(size_t bytes) { return std::min(kChunk, std::max(kChunkMin, bytes / 4)); }
 
 cudaError_t HostCopy::upload(void* device, const void* host, size_t bytes, cudaStream_t s) {
-  if (!staged(host, bytes)) return cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, s);
+  Set* set = take(host, bytes, s);
+  if (!set) return cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, s);
   const size_t step = piece(bytes);
-  Transfer transfer(*workers_);
+  Transfer transfer(*this, set);
   int slot = 0;
   for (size_t at = 0; at < bytes; at += step, slot ^= 1) {
     const size_t len = std::min(step, bytes - at);
-    unsigned char* chunk = chunks_ + slot * kChunk;
+    unsigned char* chunk = set->chunks + slot * kChunk;
     // the chunk's last copy (of this call or an earlier one) has left it
-    cudaError_t e = cudaEventSynchronize(done_[slot]);
-    if (e != cudaSuccess) return e;
-    workers_->copy(chunk, static_cast<const char*>(host) + at, len);
-    e = cudaMemcpyAsync(static_cast<char*>(device) + at, chunk, len, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaEventRecord(done_[slot], s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaEventSynchronize(set->done[slot]);
+    if (e == cudaSuccess) {
+      set->workers.copy(chunk, static_cast<const char*>(host) + at, len);
+      e = cudaMemcpyAsync(static_cast<char*>(device) + at, chunk, len, cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess) e = cudaEventRecord(set->done[slot], s);
+    }
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(s);  // nothing is left reading the chunks
+      return e;
+    }
   }
   return cudaSuccess;
 }
 
 cudaError_t HostCopy::download(void* host, const void* device, size_t bytes, cudaStream_t s) {
-  if (!staged(host, bytes)) {
+  Set* set = take(host, bytes, s);
+  if (!set) {
     const cudaError_t e = cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, s);
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
   }
   const size_t step = piece(bytes);
-  Transfer transfer(*workers_);
-  // stream order keeps these copies behind an upload that still reads a chunk
+  Transfer transfer(*this, set);
+  // after the chunk's last copy, also one of another stream
   auto queue = [&](size_t at, int slot) -> cudaError_t {
-    const cudaError_t e = cudaMemcpyAsync(chunks_ + slot * kChunk, static_cast<const char*>(device) + at, std::min(step, bytes - at),
-                                          cudaMemcpyDeviceToHost, s);
-    return e == cudaSuccess ? cudaEventRecord(done_[slot], s) : e;
+    cudaError_t e = cudaStreamWaitEvent(s, set->done[slot], 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(set->chunks + slot * kChunk, static_cast<const char*>(device) + at, std::min(step, bytes - at),
+                          cudaMemcpyDeviceToHost, s);
+    return e == cudaSuccess ? cudaEventRecord(set->done[slot], s) : e;
   };
   cudaError_t e = queue(0, 0);
   int slot = 0;
   for (size_t at = 0; at < bytes && e == cudaSuccess; at += step, slot ^= 1) {
     if (at + step < bytes) e = queue(at + step, slot ^ 1);
-    if (e == cudaSuccess) e = cudaEventSynchronize(done_[slot]);
-    if (e == cudaSuccess) workers_->copy(static_cast<char*>(host) + at, chunks_ + slot * kChunk, std::min(step, bytes - at));
+    if (e == cudaSuccess) e = cudaEventSynchronize(set->done[slot]);
+    if (e == cudaSuccess) set->workers.copy(static_cast<char*>(host) + at, set->chunks + slot * kChunk, std::min(step, bytes - at));
   }
   if (e != cudaSuccess) cudaStreamSynchronize(s);  // nothing is left writing the chunks
   return e;

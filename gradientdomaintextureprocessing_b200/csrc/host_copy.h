@@ -13,13 +13,18 @@
 // an OpenMP team's idle spin cost the caller's next host operation 0.2 ms and more
 // (drawing 1 of 512^2 sources 0.53 -> 2.46 ms after a solve; with these 0.41 on both).
 //
-// One object per stream user (not for concurrent calls); the chunks and threads
-// come with the first staged copy and go with the object.
+// Calls may overlap, from several threads and on several streams (a geodesics handle
+// copies through its system's object, beside the system's own calls): each takes a set
+// of chunks and threads for its whole length, one that is free; at most kMaxSets are
+// made, and a call that finds none makes a plain copy.  The sets come with the first
+// staged copies and go with the object.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstddef>
 #include <memory>
+#include <mutex>
+#include <vector>
 
 namespace gdtp {
 
@@ -37,17 +42,20 @@ class HostCopy {
 
  private:
   class Workers;
+  struct Set;
   struct Transfer;
   static constexpr size_t kChunk = size_t(8) << 20;
   static constexpr size_t kChunkMin = size_t(1) << 20;
   static constexpr size_t kStagedMin = size_t(2) << 20;
   static constexpr int kSlots = 2;
-  bool staged(const void* host, size_t bytes);
+  static constexpr size_t kMaxSets = 4;
+  // a set for one copy on s, null for a plain copy; the caller returns it
+  Set* take(const void* host, size_t bytes, cudaStream_t s);
+  void give(Set* set);
   static size_t piece(size_t bytes);
-  unsigned char* chunks_ = nullptr;  // kSlots x kChunk, pinned
-  cudaEvent_t done_[kSlots] = {};
-  std::unique_ptr<Workers> workers_;
-  bool failed_ = false;              // no pinned memory to be had: plain copies
+  std::mutex m_;                            // guards sets_ (which are taken) and failed_
+  std::vector<std::unique_ptr<Set>> sets_;
+  bool failed_ = false;                     // no pinned memory to be had: plain copies
 };
 
 }  // namespace gdtp

@@ -1,0 +1,92 @@
+// Staged host copies (csrc/host_copy.cpp) over a CUDA runtime on host memory
+// (fake_cuda_copies.h): copies that overlap in time.
+//
+//   host_copy_check threads   round trips of several threads through one object
+//   host_copy_check streams   a copy on one stream while another's still reads its chunks
+#include <cstdio>
+#include <random>
+#include <string>
+#include <thread>
+#include <vector>
+
+#include "fake_cuda_copies.h"
+#include "host_copy.h"
+
+namespace {
+
+using Data = std::vector<unsigned char>;
+
+Data random_data(size_t n, unsigned seed) {
+  Data v(n);
+  std::mt19937 rng(seed);
+  for (size_t i = 0; i + 4 <= n; i += 4) {
+    const unsigned r = rng();
+    std::memcpy(&v[i], &r, 4);
+  }
+  return v;
+}
+
+// every thread uploads its own vector and reads it back, streams shared or not
+int threads(int nThreads, bool oneStream) {
+  gdtp::HostCopy copier;
+  fake::Stream shared;
+  std::atomic<int> wrong{0};
+  std::vector<std::thread> ts;
+  for (int t = 0; t < nThreads; t++)
+    ts.emplace_back([&, t] {
+      fake::Stream own;
+      fake::Stream& s = oneStream ? shared : own;
+      for (int r = 0; r < 12; r++) {
+        const size_t n = (size_t(3) << 20) + size_t(t) * 700001 + size_t(r) * 4097;
+        const Data in = random_data(n, unsigned(100 * t + r));
+        Data device(n), out(n);
+        if (copier.upload(device.data(), in.data(), n, s.handle()) != cudaSuccess ||
+            copier.download(out.data(), device.data(), n, s.handle()) != cudaSuccess || out != in)
+          wrong++;
+        cudaStreamSynchronize(s.handle());
+      }
+    });
+  for (std::thread& t : ts) t.join();
+  if (wrong) std::printf("%d of %d round trips differ (%d threads, %s)\n", int(wrong), 12 * nThreads, nThreads,
+                         oneStream ? "one stream" : "a stream each");
+  return wrong;
+}
+
+// stream a still reads the chunks of an upload when a copy on stream b begins
+int streams() {
+  gdtp::HostCopy copier;
+  fake::Stream a, b;
+  int wrong = 0;
+  const size_t n = size_t(4) << 20;
+  for (int r = 0; r < 6; r++) {
+    const Data in = random_data(n, unsigned(r)), other = random_data(n, unsigned(50 + r));
+    Data dev(n), dev2 = other, out(n), out2(n), up(n);
+    a.delayUs = 30000;
+    if (copier.upload(dev.data(), in.data(), n, a.handle()) != cudaSuccess) wrong++;
+    if (copier.download(out2.data(), dev2.data(), n, b.handle()) != cudaSuccess || out2 != other) wrong++;
+    if (copier.upload(up.data(), other.data(), n, b.handle()) != cudaSuccess) wrong++;
+    cudaStreamSynchronize(b.handle());
+    if (up != other) wrong++;
+    cudaStreamSynchronize(a.handle());
+    if (dev != in) wrong++;
+    if (copier.download(out.data(), dev.data(), n, a.handle()) != cudaSuccess || out != in) wrong++;
+  }
+  if (wrong) std::printf("%d copies differ between two streams\n", wrong);
+  return wrong;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  int wrong = -1;
+  if (what == "threads") {
+    wrong = 0;
+    for (int n : {2, 3, 7})
+      for (bool oneStream : {false, true}) wrong += threads(n, oneStream);
+  } else if (what == "streams") {
+    wrong = streams();
+  }
+  if (wrong == 0) std::printf("ok\n");
+  return wrong == 0 ? 0 : 1;
+}
