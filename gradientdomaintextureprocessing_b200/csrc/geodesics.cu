@@ -192,8 +192,8 @@ bool GeodesicIntegrator::rhs_host(const double* u, double* rhs, int k) {
   double* du = static_cast<double*>(a.alloc(bytes));
   double* dr = static_cast<double*>(a.alloc(bytes));
   cudaStream_t s = sys_.stream();
-  return check(a.last, "geodesic rhs buffers") && check(sys_.hostCopy.upload(du, u, bytes, s), "h2d u") &&
-         rhs_device(du, dr, k, s) && check(sys_.hostCopy.download(rhs, dr, bytes, s), "geodesic rhs");
+  return check(a.last, "geodesic rhs buffers") && check(sys_.hostCopy->upload(du, u, bytes, s), "h2d u") &&
+         rhs_device(du, dr, k, s) && check(sys_.hostCopy->download(rhs, dr, bytes, s), "geodesic rhs");
 }
 
 bool GeodesicIntegrator::distance(DeviceSystem& smooth, DeviceSystem& dist, const int* sources, int k, double tol, int maxIters,
@@ -228,7 +228,7 @@ bool GeodesicIntegrator::distance(DeviceSystem& smooth, DeviceSystem& dist, cons
   if (!rhs_device(u, r, k, s)) return false;
   if (!dist.solve_mixed(nullptr, nullptr, r, d, k, tol, maxIters, s, distRep, true)) { err_ = dist.error(); return false; }
   dev::launch_geo_shift((long long)G_.n, k, src, d, sv, s);
-  return check(cudaGetLastError(), "geodesic shift") && check(sys_.hostCopy.download(d_host, d, nk * sizeof(double), s), "geodesic distance");
+  return check(cudaGetLastError(), "geodesic shift") && check(sys_.hostCopy->download(d_host, d, nk * sizeof(double), s), "geodesic distance");
 }
 
 }  // namespace gdtp

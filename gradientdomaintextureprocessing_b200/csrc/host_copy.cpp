@@ -157,6 +157,16 @@ struct HostCopy::Transfer {
   Set* set;
 };
 
+std::shared_ptr<HostCopy> HostCopy::of_device(int device) {
+  static std::mutex m;
+  static std::vector<std::weak_ptr<HostCopy>> objects;
+  std::lock_guard<std::mutex> l(m);
+  if (size_t(device) >= objects.size()) objects.resize(size_t(device) + 1);
+  std::shared_ptr<HostCopy> c = objects[device].lock();
+  if (!c) objects[device] = c = std::make_shared<HostCopy>();
+  return c;
+}
+
 HostCopy::HostCopy() = default;
 HostCopy::~HostCopy() = default;
 

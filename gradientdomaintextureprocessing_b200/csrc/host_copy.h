@@ -13,11 +13,12 @@
 // an OpenMP team's idle spin cost the caller's next host operation 0.2 ms and more
 // (drawing 1 of 512^2 sources 0.53 -> 2.46 ms after a solve; with these 0.41 on both).
 //
-// Calls may overlap, from several threads and on several streams (a geodesics handle
-// copies through its system's object, beside the system's own calls): each takes a set
-// of chunks and threads for its whole length, one that is free; at most kMaxSets are
-// made, and a call that finds none makes a plain copy.  The sets come with the first
-// staged copies and go with the object.
+// One object per device, shared by its systems (each with its own held 16 MB of pinned
+// memory and 5 threads per model that ever saw a large vector).  Calls may overlap, from
+// several threads and on several streams: each takes a set of chunks and threads for its
+// whole length, one that is free; at most kMaxSets are made, and a call that finds none
+// makes a plain copy.  The sets come with the first staged copies and go with the last
+// system of the device.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,6 +31,8 @@ namespace gdtp {
 
 class HostCopy {
  public:
+  // the device's object, made here when no system has it
+  static std::shared_ptr<HostCopy> of_device(int device);
   HostCopy();
   HostCopy(const HostCopy&) = delete;
   HostCopy& operator=(const HostCopy&) = delete;

@@ -435,6 +435,7 @@ DeviceSystem::DeviceSystem(const Hierarchy& h, const BoundaryElements& be, int d
   if (device < 0 || device >= n) { err_ = "invalid CUDA device"; return; }
   if (!check(cudaSetDevice(device), "cudaSetDevice")) return;
   if (!check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate")) return;
+  hostCopy = HostCopy::of_device(device);
 }
 
 DeviceSystem::~DeviceSystem() {
@@ -1607,9 +1608,9 @@ bool DeviceSystem::apply(int which, const double* x, double* y, int k) {
   if (which == 0 && !updated_) { err_ = "apply(A) before update"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  return check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") &&
+  return check(hostCopy->upload(x64_, x, n * k * 8, stream_), "h2d") &&
          raw_apply_dev(*op, nullptr, x64_, r64_, k, 1, stream_, nullptr) &&
-         check(hostCopy.download(y, r64_, n * k * 8, stream_), "apply");
+         check(hostCopy->download(y, r64_, n * k * 8, stream_), "apply");
 }
 
 bool DeviceSystem::apply_combination(double a, double b, const double* x, double* y, int k) {
@@ -1618,12 +1619,12 @@ bool DeviceSystem::apply_combination(double a, double b, const double* x, double
   if (k < 1 || k > 64) { err_ = "k must be in [1, 64]"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  if (!check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") ||
+  if (!check(hostCopy->upload(x64_, x, n * k * 8, stream_), "h2d") ||
       !raw_apply_dev(rawM_, nullptr, x64_, r64_, k, 1, stream_, nullptr) ||
       !raw_apply_dev(rawS_, nullptr, x64_, b64_, k, 1, stream_, nullptr))
     return false;
   dev::launch_axpby(r64_, a, r64_, b, b64_, (long long)(n * k), stream_);
-  return check(hostCopy.download(y, r64_, n * k * 8, stream_), "apply");
+  return check(hostCopy->download(y, r64_, n * k * 8, stream_), "apply");
 }
 
 bool DeviceSystem::residual_host(const double* b, const double* x, int k, double* rel) {
@@ -1633,8 +1634,8 @@ bool DeviceSystem::residual_host(const double* b, const double* x, int k, double
   if (k < 1 || k > 64) { err_ = "k must be in [1, 64]"; return false; }
   if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
-  if (!check(hostCopy.upload(b64_, b, n * k * 8, stream_), "h2d") ||
-      !check(hostCopy.upload(x64_, x, n * k * 8, stream_), "h2d") ||
+  if (!check(hostCopy->upload(b64_, b, n * k * 8, stream_), "h2d") ||
+      !check(hostCopy->upload(x64_, x, n * k * 8, stream_), "h2d") ||
       !raw_apply_dev(rawA_, b64_, x64_, r64_, k, 0, stream_, sumsHost_))
     return false;
   for (int c = 0; c < k; c++) rel[c] = std::sqrt(sumsHost_[c] / std::max(sumsHost_[k + c], 1e-300));
@@ -1657,7 +1658,7 @@ bool DeviceSystem::solve_filtering(const double* f_host, double* x_host, int k, 
     filterK_ = workK_;
   }
   // b = M f (+ coefS S f) on the device from one upload of f
-  if (!check(hostCopy.upload(fDev_, f_host, n * k * sizeof(double), stream_), "h2d f") ||
+  if (!check(hostCopy->upload(fDev_, f_host, n * k * sizeof(double), stream_), "h2d f") ||
       !raw_apply_dev(rawM_, nullptr, fDev_, b64_, k, 1, stream_, nullptr))
     return false;
   kernelLaunches += 1;
@@ -1676,7 +1677,7 @@ bool DeviceSystem::vectors_in(Multigrid<T>& mg, const T* x, const T* rhs, int k)
   LevelDev<T>& D0 = mg.levels[0];
   // through the FP64 work vectors (at least n x k values of either type)
   T *xs = reinterpret_cast<T*>(x64_), *bs = reinterpret_cast<T*>(b64_);
-  if (!check(hostCopy.upload(xs, x, n * k * sizeof(T), stream_), "h2d") || !check(hostCopy.upload(bs, rhs, n * k * sizeof(T), stream_), "h2d"))
+  if (!check(hostCopy->upload(xs, x, n * k * sizeof(T), stream_), "h2d") || !check(hostCopy->upload(bs, rhs, n * k * sizeof(T), stream_), "h2d"))
     return false;
   dev::launch_pad_vector<T>(xs, D0.x, (long long)n, k, mg.KP, stream_);
   dev::launch_pad_vector<T>(bs, D0.b, (long long)n, k, mg.KP, stream_);
@@ -1690,7 +1691,7 @@ bool DeviceSystem::iterate_out(Multigrid<T>& mg, T* x, int k, const char* what) 
   dev::launch_unpad_vector<T>(mg.levels[0].x, xs, (long long)n, k, mg.KP, stream_);
   queue_barrier_check(mg, stream_);
   // (the download ends with the stream's work done, the barrier check's word included)
-  return check(cudaGetLastError(), what) && check(hostCopy.download(x, xs, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
+  return check(cudaGetLastError(), what) && check(hostCopy->download(x, xs, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
 }
 
 bool DeviceSystem::vcycle_host64(double* x, const double* rhs, int k) {
@@ -1767,8 +1768,8 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
   cudaEventRecord(e0, s);
   const double* B = b_dev ? b_dev : b64_;
   double* X = x_dev ? x_dev : x64_;
-  if (b_host && !check(hostCopy.upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
-  if (x_host && !zeroGuess && !check(hostCopy.upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
+  if (b_host && !check(hostCopy->upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
+  if (x_host && !zeroGuess && !check(hostCopy->upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
   if (zeroGuess && !check(cudaMemsetAsync(X, 0, n * k * 8, s), "zero x")) return false;
   int it = 0;
   double rm = 0;
@@ -1840,7 +1841,7 @@ bool DeviceSystem::solve_mixed(const double* b_host, double* x_host, const doubl
       collect_timing(mg);
     }
   }
-  if (x_host && !check(hostCopy.download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
+  if (x_host && !check(hostCopy->download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
   queue_barrier_check(mg, s);
   cudaEventRecord(e1, s);
   if (userStream) cudaStreamWaitEvent(userStream, e1, 0);
@@ -2159,8 +2160,8 @@ bool DeviceSystem::solve_fp64(const double* b_host, double* x_host, const double
   // filled from the host
   const double* B = b_dev ? b_dev : b64_;
   double* X = x_dev ? x_dev : x64_;
-  if (b_host && !check(hostCopy.upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
-  if (x_host && !check(hostCopy.upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
+  if (b_host && !check(hostCopy->upload(b64_, b_host, n * k * 8, s), "h2d b")) return false;
+  if (x_host && !check(hostCopy->upload(x64_, x_host, n * k * 8, s), "h2d x")) return false;
   kernelLaunches += 2;  // operator + norm reduction
   if (!raw_apply_dev(rawA_, B, X, r64_, k, 0, s, nullptr) || !read_norms(k, s, "initial residual")) return false;
   rep = SolveReport();
@@ -2205,7 +2206,7 @@ bool DeviceSystem::solve_fp64(const double* b_host, double* x_host, const double
     it++;
     rm = rel_max();
   }
-  if (x_host && !check(hostCopy.download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
+  if (x_host && !check(hostCopy->download(x_host, x64_, n * k * 8, s), "d2h x")) return false;
   queue_barrier_check(mg, s);
   cudaEventRecord(e1, s);
   if (userStream) cudaStreamWaitEvent(userStream, e1, 0);

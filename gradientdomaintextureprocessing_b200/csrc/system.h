@@ -208,8 +208,9 @@ class DeviceSystem {
   bool autotune(const double* b, int k, double tol, SolverKnobs& best, double& bestSeconds);
   bool residual_host(const double* b, const double* x, int k, double* rel);
 
-  // copies between the caller's host vectors and the device, for this system's stream
-  HostCopy hostCopy;
+  // copies between the caller's host vectors and the device (shared with the device's
+  // other systems)
+  std::shared_ptr<HostCopy> hostCopy;
   SolverKnobs knobs;
   bool profTiled() const { return profTiled_; }
   bool profRows() const { return profRows_; }

@@ -3,6 +3,7 @@
 //
 //   host_copy_check threads   round trips of several threads through one object
 //   host_copy_check streams   a copy on one stream while another's still reads its chunks
+//   host_copy_check shared    one object per device, whose memory goes with its last owner
 #include <cstdio>
 #include <random>
 #include <string>
@@ -75,6 +76,37 @@ int streams() {
   return wrong;
 }
 
+// eight owners on a device, one after another and nested: one set's memory, all given back
+int shared() {
+  int wrong = 0;
+  const size_t n = size_t(5) << 20;
+  const Data in = random_data(n, 1);
+  {
+    fake::Stream s;
+    std::vector<std::shared_ptr<gdtp::HostCopy>> owners;
+    for (int i = 0; i < 8; i++) {
+      owners.push_back(gdtp::HostCopy::of_device(0));
+      Data device(n), out(n);
+      owners.back()->upload(device.data(), in.data(), n, s.handle());
+      owners.back()->download(out.data(), device.data(), n, s.handle());
+      if (out != in) wrong++;
+    }
+    if (gdtp::HostCopy::of_device(1) == owners[0]) wrong++;
+    const long long one = fake::pinnedBytes;
+    if (one <= 0 || one > (16 << 20) || fake::pinnedPeak != one) {
+      std::printf("pinned memory of 8 owners: %lld bytes\n", one);
+      wrong++;
+    }
+    owners.erase(owners.begin() + 1, owners.end());
+    if (fake::pinnedBytes != one) wrong++;
+  }
+  if (fake::pinnedBytes != 0 || fake::events != 0) {
+    std::printf("%lld pinned bytes and %d events left\n", (long long)fake::pinnedBytes, int(fake::events));
+    wrong++;
+  }
+  return wrong;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -86,6 +118,8 @@ int main(int argc, char** argv) {
       for (bool oneStream : {false, true}) wrong += threads(n, oneStream);
   } else if (what == "streams") {
     wrong = streams();
+  } else if (what == "shared") {
+    wrong = shared();
   }
   if (wrong == 0) std::printf("ok\n");
   return wrong == 0 ? 0 : 1;

@@ -27,3 +27,8 @@ def check(tmp_path_factory):
 def test_copies_that_overlap(check, what):
     """Every copy arrives whole whatever other copies of the same object are under way."""
     check(what)
+
+
+def test_systems_of_a_device_share_one(check):
+    """The pinned memory and the threads do not grow with the systems and go with the last."""
+    check("shared")
