@@ -111,7 +111,9 @@ class HostCopy::Workers {
 
 // Two pinned chunks, the events after their last copies, and the threads
 struct HostCopy::Set {
-  unsigned char* chunks = nullptr;  // kSlots x kChunk
+  unsigned char* chunks = nullptr;  // kSlots x size
+  size_t size = 0;
+  size_t small = 0;                 // moved in steps that the chunks' size limited
   cudaEvent_t done[kSlots] = {};
   cudaStream_t last = nullptr;      // stream of the last copy
   Workers workers;
@@ -125,15 +127,22 @@ struct HostCopy::Set {
       }
     return true;
   }
-  bool make() {
+  // (new) chunks of this size, once the old ones are left
+  bool make(size_t bytes) {
     void* p = nullptr;
-    if (cudaHostAlloc(&p, kSlots * kChunk, cudaHostAllocDefault) != cudaSuccess) return false;
-    chunks = static_cast<unsigned char*>(p);
-    for (cudaEvent_t& e : done)
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+    if (cudaHostAlloc(&p, kSlots * bytes, cudaHostAllocDefault) != cudaSuccess) return false;
+    for (cudaEvent_t& e : done) {
+      if (e) cudaEventSynchronize(e);
+      else if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
         e = nullptr;
+        cudaFreeHost(p);
         return false;
       }
+    }
+    if (chunks) cudaFreeHost(chunks);
+    chunks = static_cast<unsigned char*>(p);
+    size = bytes;
+    small = 0;
     return true;
   }
   ~Set() {
@@ -167,11 +176,11 @@ std::shared_ptr<HostCopy> HostCopy::of_device(int device) {
   return c;
 }
 
-HostCopy::HostCopy() = default;
+HostCopy::HostCopy(size_t payback) : payback_(payback) {}
 HostCopy::~HostCopy() = default;
 
 // A free set whose chunks are idle, or are left in the order of s: another stream's
-// pending work is not waited for.  None: a new set, up to kMaxSets.
+// pending work is not waited for.  None: a new set, up to kMaxSets, once it is paid for.
 HostCopy::Set* HostCopy::take(const void* host, size_t bytes, cudaStream_t s) {
   if (bytes < kStagedMin) return nullptr;
   cudaPointerAttributes at{};
@@ -180,25 +189,38 @@ HostCopy::Set* HostCopy::take(const void* host, size_t bytes, cudaStream_t s) {
     return nullptr;
   }
   if (at.type != cudaMemoryTypeUnregistered) return nullptr;
-  Set* made;
+  Set* set = nullptr;
+  const size_t want = (piece(bytes) + kChunkMin - 1) / kChunkMin * kChunkMin;
+  bool made = false;
   {
     std::lock_guard<std::mutex> l(m_);
-    for (std::unique_ptr<Set>& set : sets_)
-      if (!set->taken && (set->last == s || set->idle())) {
-        set->taken = true;
-        set->last = s;
-        return set.get();
-      }
-    if (failed_ || sets_.size() >= kMaxSets) return nullptr;
-    sets_.push_back(std::make_unique<Set>());
-    made = sets_.back().get();
-    made->last = s;
+    for (std::unique_ptr<Set>& q : sets_)
+      if (!set && !q->taken && (q->last == s || q->idle())) set = q.get();
+    if (!set) {
+      plain_ += bytes;
+      if (failed_ || sets_.size() >= kMaxSets || plain_ < payback_) return nullptr;
+      plain_ = 0;
+      made = true;
+      sets_.push_back(std::make_unique<Set>());
+      set = sets_.back().get();
+    }
+    set->taken = true;
+    set->last = s;
+    if (!made && set->size < want) set->small += bytes;
   }
-  if (made->make()) return made;  // (allocated while other copies go on)
+  // (allocations go on beside other copies)
+  if (!made) {
+    if (set->size < want && set->small >= payback_ && !set->make(std::min(kChunkMax, std::max(want, 2 * set->size)))) {
+      cudaGetLastError();  // none of that size: the chunks stay as they are
+      set->small = 0;
+    }
+    return set;
+  }
+  if (set->make(want)) return set;
   cudaGetLastError();
   std::lock_guard<std::mutex> l(m_);
   failed_ = true;
-  sets_.erase(std::find_if(sets_.begin(), sets_.end(), [made](const std::unique_ptr<Set>& set) { return set.get() == made; }));
+  sets_.erase(std::find_if(sets_.begin(), sets_.end(), [set](const std::unique_ptr<Set>& q) { return q.get() == set; }));
   return nullptr;
 }
 
@@ -207,18 +229,18 @@ void HostCopy::give(Set* set) {
   set->taken = false;
 }
 
-// a quarter of the vector, so that the two sides overlap, within the chunk's size
-size_t HostCopy::piece(size_t bytes) { return std::min(kChunk, std::max(kChunkMin, bytes / 4)); }
+// a quarter of the vector, so that the two sides overlap, within a chunk's size
+size_t HostCopy::piece(size_t bytes) { return std::min(kChunkMax, std::max(kChunkMin, bytes / 4)); }
 
 cudaError_t HostCopy::upload(void* device, const void* host, size_t bytes, cudaStream_t s) {
   Set* set = take(host, bytes, s);
   if (!set) return cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, s);
-  const size_t step = piece(bytes);
+  const size_t step = std::min(set->size, piece(bytes));
   Transfer transfer(*this, set);
   int slot = 0;
   for (size_t at = 0; at < bytes; at += step, slot ^= 1) {
     const size_t len = std::min(step, bytes - at);
-    unsigned char* chunk = set->chunks + slot * kChunk;
+    unsigned char* chunk = set->chunks + slot * set->size;
     // the chunk's last copy (of this call or an earlier one) has left it
     cudaError_t e = cudaEventSynchronize(set->done[slot]);
     if (e == cudaSuccess) {
@@ -240,13 +262,13 @@ cudaError_t HostCopy::download(void* host, const void* device, size_t bytes, cud
     const cudaError_t e = cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, s);
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
   }
-  const size_t step = piece(bytes);
+  const size_t step = std::min(set->size, piece(bytes));
   Transfer transfer(*this, set);
   // after the chunk's last copy, also one of another stream
   auto queue = [&](size_t at, int slot) -> cudaError_t {
     cudaError_t e = cudaStreamWaitEvent(s, set->done[slot], 0);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(set->chunks + slot * kChunk, static_cast<const char*>(device) + at, std::min(step, bytes - at),
+      e = cudaMemcpyAsync(set->chunks + slot * set->size, static_cast<const char*>(device) + at, std::min(step, bytes - at),
                           cudaMemcpyDeviceToHost, s);
     return e == cudaSuccess ? cudaEventRecord(set->done[slot], s) : e;
   };
@@ -255,7 +277,7 @@ cudaError_t HostCopy::download(void* host, const void* device, size_t bytes, cud
   for (size_t at = 0; at < bytes && e == cudaSuccess; at += step, slot ^= 1) {
     if (at + step < bytes) e = queue(at + step, slot ^ 1);
     if (e == cudaSuccess) e = cudaEventSynchronize(set->done[slot]);
-    if (e == cudaSuccess) set->workers.copy(static_cast<char*>(host) + at, set->chunks + slot * kChunk, std::min(step, bytes - at));
+    if (e == cudaSuccess) set->workers.copy(static_cast<char*>(host) + at, set->chunks + slot * set->size, std::min(step, bytes - at));
   }
   if (e != cudaSuccess) cudaStreamSynchronize(s);  // nothing is left writing the chunks
   return e;

@@ -3,6 +3,7 @@
 //
 //   host_copy_check threads   round trips of several threads through one object
 //   host_copy_check streams   a copy on one stream while another's still reads its chunks
+//   host_copy_check first     when chunks are made, and how large
 //   host_copy_check shared    one object per device, whose memory goes with its last owner
 #include <cstdio>
 #include <random>
@@ -29,7 +30,7 @@ Data random_data(size_t n, unsigned seed) {
 
 // every thread uploads its own vector and reads it back, streams shared or not
 int threads(int nThreads, bool oneStream) {
-  gdtp::HostCopy copier;
+  gdtp::HostCopy copier(0);  // staged from the first copy on
   fake::Stream shared;
   std::atomic<int> wrong{0};
   std::vector<std::thread> ts;
@@ -55,7 +56,7 @@ int threads(int nThreads, bool oneStream) {
 
 // stream a still reads the chunks of an upload when a copy on stream b begins
 int streams() {
-  gdtp::HostCopy copier;
+  gdtp::HostCopy copier(0);  // staged from the first copy on
   fake::Stream a, b;
   int wrong = 0;
   const size_t n = size_t(4) << 20;
@@ -76,6 +77,49 @@ int streams() {
   return wrong;
 }
 
+// few copies make no chunks; many, or one large enough, make them of the size they need
+int first() {
+  int wrong = 0;
+  fake::Stream s;
+  auto trips = [&](gdtp::HostCopy& copier, size_t n, int count) {
+    const Data in = random_data(n, unsigned(n));
+    Data device(n), out(n);
+    for (int r = 0; r < count; r++) {
+      copier.upload(device.data(), in.data(), n, s.handle());
+      copier.download(out.data(), device.data(), n, s.handle());
+      if (out != in) wrong++;
+    }
+  };
+  auto expect = [&](const char* what, long long low, long long high) {
+    if (fake::pinnedBytes >= low && fake::pinnedBytes <= high) return;
+    std::printf("%s: %lld pinned bytes\n", what, (long long)fake::pinnedBytes);
+    wrong++;
+  };
+  const long long MB = 1 << 20;
+  {
+    gdtp::HostCopy copier;
+    trips(copier, 5 * MB, 6);
+    expect("60 MB moved", 0, 0);
+    trips(copier, 5 * MB, 1);
+    expect("70 MB moved", 2 * MB, 4 * MB);
+    trips(copier, 21 * MB, 1);
+    expect("one larger vector", 2 * MB, 4 * MB);
+    trips(copier, 21 * MB, 1);
+    expect("larger vectors", 12 * MB, 12 * MB);
+    trips(copier, 50 * MB, 2);
+    expect("the largest", 16 * MB, 16 * MB);
+    trips(copier, 5 * MB, 2);
+    expect("as before", 16 * MB, 16 * MB);
+  }
+  {
+    gdtp::HostCopy copier;
+    trips(copier, 70 * MB, 1);
+    expect("one vector of 70 MB", 16 * MB, 16 * MB);
+  }
+  expect("all gone", 0, 0);
+  return wrong;
+}
+
 // eight owners on a device, one after another and nested: one set's memory, all given back
 int shared() {
   int wrong = 0;
@@ -83,7 +127,10 @@ int shared() {
   const Data in = random_data(n, 1);
   {
     fake::Stream s;
-    std::vector<std::shared_ptr<gdtp::HostCopy>> owners;
+    std::vector<std::shared_ptr<gdtp::HostCopy>> owners{gdtp::HostCopy::of_device(0)};
+    Data large(size_t(64) << 20), device(large.size());
+    owners[0]->upload(device.data(), large.data(), large.size(), s.handle());  // staged from here on
+    cudaStreamSynchronize(s.handle());
     for (int i = 0; i < 8; i++) {
       owners.push_back(gdtp::HostCopy::of_device(0));
       Data device(n), out(n);
@@ -118,6 +165,8 @@ int main(int argc, char** argv) {
       for (bool oneStream : {false, true}) wrong += threads(n, oneStream);
   } else if (what == "streams") {
     wrong = streams();
+  } else if (what == "first") {
+    wrong = first();
   } else if (what == "shared") {
     wrong = shared();
   }

@@ -32,3 +32,8 @@ def test_copies_that_overlap(check, what):
 def test_systems_of_a_device_share_one(check):
     """The pinned memory and the threads do not grow with the systems and go with the last."""
     check("shared")
+
+
+def test_chunks_are_made_once_they_pay(check):
+    """Pinned memory costs more than the first copies gain: a program of a few calls has none."""
+    check("first")
