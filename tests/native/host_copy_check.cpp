@@ -4,8 +4,10 @@
 //   host_copy_check threads   round trips of several threads through one object
 //   host_copy_check streams   a copy on one stream while another's still reads its chunks
 //   host_copy_check first     when chunks are made, and how large
+//   host_copy_check idle      copies that wait for the work queued before them
 //   host_copy_check shared    one object per device, whose memory goes with its last owner
 #include <cstdio>
+#include <ctime>
 #include <random>
 #include <string>
 #include <thread>
@@ -120,6 +122,35 @@ int first() {
   return wrong;
 }
 
+// copies behind 0.3 s of queued work: the host threads sleep meanwhile
+int idle() {
+  gdtp::HostCopy copier(0);
+  fake::Stream s;
+  const size_t n = size_t(12) << 20;
+  const Data in = random_data(n, 3);
+  Data device(n), out(n);
+  copier.upload(device.data(), in.data(), n, s.handle());
+  cudaStreamSynchronize(s.handle());
+  int wrong = 0;
+  auto cpu = [&](const char* what, auto&& copy) {
+    s.sleep(300000);
+    const std::clock_t c0 = std::clock();
+    copy();
+    cudaStreamSynchronize(s.handle());
+    const double t = double(std::clock() - c0) / CLOCKS_PER_SEC;
+    if (t > 0.15) {
+      std::printf("%s: %.2f s of processor time\n", what, t);
+      wrong++;
+    }
+  };
+  cpu("download", [&] { copier.download(out.data(), device.data(), n, s.handle()); });
+  if (out != in) wrong++;
+  std::fill(device.begin(), device.end(), 0);
+  cpu("upload", [&] { copier.upload(device.data(), in.data(), n, s.handle()); });
+  if (device != in) wrong++;
+  return wrong;
+}
+
 // eight owners on a device, one after another and nested: one set's memory, all given back
 int shared() {
   int wrong = 0;
@@ -165,6 +196,8 @@ int main(int argc, char** argv) {
       for (bool oneStream : {false, true}) wrong += threads(n, oneStream);
   } else if (what == "streams") {
     wrong = streams();
+  } else if (what == "idle") {
+    wrong = idle();
   } else if (what == "first") {
     wrong = first();
   } else if (what == "shared") {
