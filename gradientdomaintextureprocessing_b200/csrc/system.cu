@@ -1672,26 +1672,25 @@ bool DeviceSystem::solve_filtering(const double* f_host, double* x_host, int k, 
 
 template <typename T>
 bool DeviceSystem::vectors_in(Multigrid<T>& mg, const T* x, const T* rhs, int k) {
-  if (!ensure_work(k)) return false;
   const size_t n = h_.levels[0].numTexels;
   LevelDev<T>& D0 = mg.levels[0];
-  // through the FP64 work vectors (at least n x k values of either type)
-  T *xs = reinterpret_cast<T*>(x64_), *bs = reinterpret_cast<T*>(b64_);
-  if (!check(hostCopy->upload(xs, x, n * k * sizeof(T), stream_), "h2d") || !check(hostCopy->upload(bs, rhs, n * k * sizeof(T), stream_), "h2d"))
-    return false;
-  dev::launch_pad_vector<T>(xs, D0.x, (long long)n, k, mg.KP, stream_);
-  dev::launch_pad_vector<T>(bs, D0.b, (long long)n, k, mg.KP, stream_);
+  // one after the other through the level's residual, which a V-cycle writes before it
+  // reads it: no vectors of their own, and the solves' work vectors are not needed
+  if (!check(hostCopy->upload(D0.r, x, n * k * sizeof(T), stream_), "h2d")) return false;
+  dev::launch_pad_vector<T>(D0.r, D0.x, (long long)n, k, mg.KP, stream_);
+  if (!check(hostCopy->upload(D0.r, rhs, n * k * sizeof(T), stream_), "h2d")) return false;
+  dev::launch_pad_vector<T>(D0.r, D0.b, (long long)n, k, mg.KP, stream_);
   return check(cudaGetLastError(), "pad vectors");
 }
 
 template <typename T>
 bool DeviceSystem::iterate_out(Multigrid<T>& mg, T* x, int k, const char* what) {
   const size_t n = h_.levels[0].numTexels;
-  T* xs = reinterpret_cast<T*>(x64_);
-  dev::launch_unpad_vector<T>(mg.levels[0].x, xs, (long long)n, k, mg.KP, stream_);
+  LevelDev<T>& D0 = mg.levels[0];
+  dev::launch_unpad_vector<T>(D0.x, D0.r, (long long)n, k, mg.KP, stream_);
   queue_barrier_check(mg, stream_);
   // (the download ends with the stream's work done, the barrier check's word included)
-  return check(cudaGetLastError(), what) && check(hostCopy->download(x, xs, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
+  return check(cudaGetLastError(), what) && check(hostCopy->download(x, D0.r, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
 }
 
 bool DeviceSystem::vcycle_host64(double* x, const double* rhs, int k) {
