@@ -127,6 +127,11 @@ extern "C" int gdtp_system_array(const gdtp_system* s, const char* cname, int le
       if (count) *count = 0;
       return GDTP_OK;
     }
+    if (name == "fault.barrier") {
+      const_cast<DeviceSystem*>(s->sys.get())->fail_barriers();
+      if (count) *count = 0;
+      return GDTP_OK;
+    }
     if (name == "profile.setup") return vec(std::vector<double>(s->sys->setupMs, s->sys->setupMs + 14));
     if (name == "levelStats") return vec(s->sys->level_stats());  // 9 per level, see DeviceSystem::level_stats
     if (name == "levelsUsed") {

@@ -1331,6 +1331,13 @@ void DeviceSystem::queue_barrier_check(Multigrid<T>& mg, cudaStream_t s) {
   *barrierErrHost_ = 0;
   cudaMemcpyAsync(barrierErrHost_, &mg.barrier->error, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
 }
+void DeviceSystem::fail_barriers() {
+  const unsigned int code = 1;
+  cudaSetDevice(device_);
+  for (const auto& m : mg32_)
+    if (m->barrier) cudaMemcpy(&m->barrier->error, &code, sizeof(code), cudaMemcpyHostToDevice);
+  if (mg64_ && mg64_->barrier) cudaMemcpy(&mg64_->barrier->error, &code, sizeof(code), cudaMemcpyHostToDevice);
+}
 template <typename T>
 bool DeviceSystem::barrier_ok(Multigrid<T>& mg) {
   if (!(usedGridBarrier_ || usedTileWait_) || !mg.barrier || !barrierErrHost_ || *barrierErrHost_ == 0) return true;
@@ -1689,8 +1696,11 @@ bool DeviceSystem::iterate_out(Multigrid<T>& mg, T* x, int k, const char* what) 
   LevelDev<T>& D0 = mg.levels[0];
   dev::launch_unpad_vector<T>(D0.x, D0.r, (long long)n, k, mg.KP, stream_);
   queue_barrier_check(mg, stream_);
-  // (the download ends with the stream's work done, the barrier check's word included)
-  return check(cudaGetLastError(), what) && check(hostCopy->download(x, D0.r, n * k * sizeof(T), stream_), what) && barrier_ok(mg);
+  if (!check(cudaGetLastError(), what)) return false;
+  // a cycle whose grid barrier or tile wait timed out leaves the caller's vector alone
+  // (without either there is nothing to wait for)
+  if ((usedGridBarrier_ || usedTileWait_) && (!check(cudaStreamSynchronize(stream_), what) || !barrier_ok(mg))) return false;
+  return check(hostCopy->download(x, D0.r, n * k * sizeof(T), stream_), what);
 }
 
 bool DeviceSystem::vcycle_host64(double* x, const double* rhs, int k) {

@@ -434,6 +434,9 @@ class DeviceSystem {
   bool barrier_ok(Multigrid<T>& mg);
   unsigned long long* clusterTimeline();
  public:
+  // sets the error word of the built multigrids' grid barriers, as a barrier that timed
+  // out does: their next V-cycle with one fails (for tests)
+  void fail_barriers();
   // last cluster timeline: {code, ns} pairs (empty when not traced)
   bool cluster_timeline(std::vector<unsigned long long>& out);
 };

@@ -123,6 +123,8 @@ void gdtp_system_free(gdtp_system* s);
  *   kernels per step graph, kernels launched by solves, the timed group's smoother:
  *   1 one fused tile-smoother launch, 2 a sweep of two row-smoother launches, 0 a
  *   sweep of four colour passes}; "profile.reset" clears the counts
+ *   "fault.barrier" (no values): the built multigrids' grid barriers read as timed
+ *   out, as after a lost block: the next V-cycle that uses one fails
  *   "profile.setup": ms of the last set-up {update, boundary solver factorisations,
  *   coarsest inverse, other multigrid set-up, then the factorisations split into
  *   partition and sparse assembly, subdomain inverses, Schur products, Schur

@@ -29,3 +29,29 @@ def test_no_solve_vectors_are_allocated(built_lib, call, k):
     s.residual(b.astype(float), x.astype(float))
     assert s.device_bytes() - before >= 3 * 8 * s.n * k
     np.testing.assert_array_equal(getattr(s, call)(x, b), first)
+
+
+@pytest.mark.parametrize("double", [False, True])
+def test_a_failed_cycle_leaves_the_vector_alone(built_lib, double):
+    """A grid barrier that timed out (its error word set from the host) fails the call; the
+    caller's x keeps its values."""
+    import ctypes as C
+    from gradientdomaintextureprocessing_b200 import _lib
+    L, s = _lib.lib(), make("torus128")
+    s.set("grid_texels", 1 << 30)
+    kind = np.float64 if double else np.float32
+    call = L.gdtp_vcycle64 if double else L.gdtp_vcycle
+    rng = np.random.default_rng(0)
+    x, b = (rng.standard_normal((s.n, 3)).astype(kind) for _ in range(2))
+
+    def run():
+        y = x.copy()
+        return call(s.handle, _lib.ptr(y), _lib.ptr(b), 3), y
+
+    code, good = run()
+    assert code == 0 and not np.array_equal(good, x)
+    count = C.c_int64()
+    assert L.gdtp_system_array(s.handle, b"fault.barrier", 0, None, C.byref(count)) == 0
+    code, failed = run()
+    assert code != 0
+    np.testing.assert_array_equal(failed, x)
