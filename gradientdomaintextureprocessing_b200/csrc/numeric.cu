@@ -600,38 +600,69 @@ bool NumericPlan::fill_levels(const std::vector<LevelValues<float>>& f32, const 
                               std::string& err) {
   if (!ensure_streams(err)) return false;
   std::vector<int> badHost(2 * size_t(L), 0);
-  cudaError_t e = cudaSuccess;
   std::vector<std::unique_ptr<LevelJob>> jobs(L);
-  {
-    StreamScratch words(s);
-    int* bad = words.get<int>(2 * size_t(L));
-    if (!bad) {
-      err = std::string("numeric scratch: ") + cudaGetErrorString(words.last);
-      return false;
-    }
-    e = cudaEventRecord(ready_, s);
-    for (int i = 0; i < L && e == cudaSuccess; i++) {
-      const int l = i == 0 ? L - 1 : i - 1;  // the longest chain first
-      e = cudaStreamWaitEvent(streams_[l].s, ready_, 0);
-      if (e != cudaSuccess) break;
-      jobs[l].reset(new LevelJob(streams_[l]));
-      jobs[l]->bad = bad + 2 * l;
-      queue_level(l, f32.empty() ? nullptr : &f32[l], f64.empty() ? nullptr : &f64[l], *jobs[l]);
-    }
-    // s continues after every level that was queued, also after an error
+  StreamScratch words(s);
+  int* bad = words.get<int>(2 * size_t(L));
+  if (!bad) {
+    cudaGetLastError();
+    err = std::string("numeric scratch: ") + cudaGetErrorString(words.last);
+    return false;
+  }
+  // a level on its stream, after the work queued on s
+  auto queue = [&](int l) -> cudaError_t {
+    const cudaError_t w = cudaStreamWaitEvent(streams_[l].s, ready_, 0);
+    if (w != cudaSuccess) return w;
+    jobs[l].reset(new LevelJob(streams_[l]));
+    jobs[l]->bad = bad + 2 * l;
+    queue_level(l, f32.empty() ? nullptr : &f32[l], f64.empty() ? nullptr : &f64[l], *jobs[l]);
+    return cudaSuccess;
+  };
+  // s continues after every level that was queued, also after an error; the error words
+  auto finish = [&](cudaError_t e) -> cudaError_t {
     for (int l = 0; l < L; l++)
       if (jobs[l]) {
         const cudaError_t w = cudaStreamWaitEvent(s, streams_[l].mark[kMarks - 1], 0);
         if (e == cudaSuccess) e = w;
       }
-    if (e == cudaSuccess) e = cudaGetLastError();
     const cudaError_t d = cudaMemcpyAsync(badHost.data(), bad, badHost.size() * sizeof(int), cudaMemcpyDeviceToHost, s);
     const cudaError_t y = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) e = d != cudaSuccess ? d : y;
+    const cudaError_t last = cudaGetLastError();
+    for (cudaError_t q : {d, y, last})
+      if (e == cudaSuccess) e = q;
+    return e;
+  };
+  auto order = [this](int i) { return i == 0 ? L - 1 : i - 1; };  // the longest chain first
+  auto scratch_failed = [&] {
+    for (int l = 0; l < L; l++)
+      if (jobs[l] && jobs[l]->S.last != cudaSuccess) return l;
+    return -1;
+  };
+  cudaError_t e = cudaEventRecord(ready_, s);
+  for (int i = 0; i < L && e == cudaSuccess; i++) e = queue(order(i));
+  e = finish(e);
+  if (scratch_failed() >= 0) {
+    // no room for the scratch of all levels at once (their sum): in turn, each giving its
+    // scratch back before the next, so that the largest level's is enough
+    e = cudaSuccess;
+    for (int i = 0; i < L && e == cudaSuccess && (i == 0 || scratch_failed() < 0); i++) {
+      for (int l = 0; l < L; l++) {
+        jobs[l].reset();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(streams_[l].s);
+      }
+      int device = 0;
+      cudaMemPool_t pool;
+      if (cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+      if (e == cudaSuccess) e = queue(order(i));
+      e = finish(e);
+      const int l = order(i);
+      if (jobs[l] && scratch_failed() < 0 && !jobs[l]->launchOk) break;
+      if (badHost[2 * size_t(l)] || badHost[2 * size_t(l) + 1]) break;
+    }
   }
+  const int starved = scratch_failed();
   for (int l = 0; l < L; l++) {
     const std::string where = l == L - 1 ? "coarsest level: " : "level " + std::to_string(l) + ": ";
-    if (jobs[l] && e == cudaSuccess && jobs[l]->S.last != cudaSuccess) {
+    if (l == starved) {
       err = where + "scratch: " + cudaGetErrorString(jobs[l]->S.last);
       return false;
     }

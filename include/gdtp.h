@@ -142,7 +142,10 @@ int gdtp_system_array(const gdtp_system* s, const char* name, int level, void* o
  * device_factor 1 (the default) every weight-dependent value -- smoother planes,
  * boundary rows, boundary-block and coarsest-level inverses -- is recomputed on
  * the device, in place in a multigrid already built; otherwise the next solve
- * rebuilds the multigrid from host-combined coefficients.
+ * rebuilds the multigrid from host-combined coefficients.  The levels run side by
+ * side in the scratch of all of them (413 MB for a 1024^2 atlas), which stays in
+ * the device's memory pool for the next update; where that does not fit they run
+ * one after another in the largest one's, same values.
  * Replaces UpdateLinearSystem (include/Src/UpdateCoefficients.inl:463-513),
  * UpdateMultigridCoefficients (:285-399) and UpdateMultigridSolvers (:402-439). */
 int gdtp_system_update(gdtp_system* s, double stiffness_weight, double screen_weight);
