@@ -1301,6 +1301,22 @@ std::vector<double> DeviceSystem::level_stats() const {
   return v;
 }
 
+template <typename T>
+std::vector<double> DeviceSystem::level_routes() const {
+  const Multigrid<T>* mg = nullptr;
+  if constexpr (sizeof(T) == 4) mg = mg32_.empty() ? nullptr : mg32_.back().get();
+  else mg = mg64_.get();
+  std::vector<double> v;
+  for (size_t l = 0; mg && l + 1 < mg->levels.size(); l++) {
+    const LevelDev<T>& D = mg->levels[l];
+    const int KP = mg->KP, W = KP % 4 == 0 ? 4 : 1;
+    v.push_back(tiled(D, KP) ? 4 : clustered(D, KP) ? 3 : grouped(D, KP) ? 2 : row_sweeps_on(D, KP, sizeof(T), W) ? 1 : 0);
+  }
+  return v;
+}
+template std::vector<double> DeviceSystem::level_routes<float>() const;
+template std::vector<double> DeviceSystem::level_routes<double>() const;
+
 bool DeviceSystem::cluster_timeline(std::vector<unsigned long long>& out) {
   out.clear();
   if (!timeline_) return true;

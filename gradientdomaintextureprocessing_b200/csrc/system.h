@@ -282,6 +282,10 @@ class DeviceSystem {
   // texels, subdomain rows, separator rows, subdomain tasks x chunks, Schur tasks
   // x chunks, chart groups, largest chart (deep texels)
   std::vector<double> level_stats() const;
+  // per level but the coarsest of the last built FP32 (or FP64) multigrid, what smooths it:
+  // 0 colour passes, 1 row launches, 2 a block per chart, 3 chart clusters, 4 tiles
+  template <typename T>
+  std::vector<double> level_routes() const;
   // last set-up, ms: update (weights, Galerkin coarsening, FP64 operators),
   // boundary solver factorisations, coarsest inverse, other multigrid set-up
   // (device layouts, uploads); the last three when the multigrid is built;

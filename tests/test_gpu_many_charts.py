@@ -1,0 +1,70 @@
+"""Atlases of many small charts: which kernels take their levels, and the same bits from all.
+
+The FP32 V-cycle's arithmetic per right-hand side does not depend on how many are solved
+together nor on which kernel variant runs, so every comparison is bitwise."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def grid_atlas(n, size, sub=2, gutter=2.0, seed=0):
+    """n x n square charts of a wavy sheet, sub x sub quads each, corners moved by up to 0.3 texels."""
+    from gradientdomaintextureprocessing_b200 import meshgen
+    rng = np.random.default_rng(seed)
+    m = n * sub
+    i, j = np.meshgrid(np.arange(m + 1), np.arange(m + 1), indexing="xy")
+    vertices = np.stack([i / m, j / m, 0.1 * np.sin(5 * i / m) * np.cos(4 * j / m)], -1).reshape(-1, 3)
+    jitter = rng.uniform(-0.3, 0.3, (n, n, sub + 1, sub + 1, 2))
+    inner = size / n - 2 * gutter
+    triangles, uv = [], []
+    for cy, cx, b, a in np.ndindex(n, n, sub, sub):
+        quad = [(a, b), (a + 1, b), (a + 1, b + 1), (a, b + 1)]
+        for t in ((0, 1, 2), (0, 2, 3)):
+            triangles.append([(cy * sub + quad[q][1]) * (m + 1) + cx * sub + quad[q][0] for q in t])
+            uv.append([[(c * size / n + gutter + p / sub * inner + jitter[cy, cx, quad[q][1], quad[q][0], x]) / size
+                        for x, (c, p) in enumerate(((cx, quad[q][0]), (cy, quad[q][1])))] for q in t])
+    uv = meshgen._keep_off_texel_grid(np.array(uv), size, size)
+    return {"vertices": vertices, "triangles": np.array(triangles, dtype=np.int32), "uv": uv}
+
+
+@pytest.fixture(scope="module", params=[(26, 832), (32, 1024), (12, 640)])
+def atlas(request, built_lib):
+    from gradientdomaintextureprocessing_b200.hierarchy import InitializeHierarchy
+    from gradientdomaintextureprocessing_b200.system import System
+    n, size = request.param
+    s = System(InitializeHierarchy(grid_atlas(n, size), size, size, levels=4))
+    s.update(1e-3, 1.0)
+    s.charts = n * n
+    return s
+
+
+def vectors(n, k, seed=0):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal((n, k)), rng.standard_normal((n, k))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("k", [1, 3, 9])
+def test_charts_smooth_on_clusters(atlas, k, precision):
+    """Up to 4 channels every level with deep texels smooths on clusters, however many charts
+    it has; the launches give the same bits."""
+    b, _ = vectors(atlas.n, k)
+    got = {}
+    try:
+        for on, texels in ((1, 1000), (0, 1000), (0, 0)):
+            atlas.set("chart_cluster", on)
+            atlas.set("chart_texels", texels)
+            got[on, texels] = atlas.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+            routes = atlas.array("levelRoutes", 1 if precision == "fp64" else 0)
+            deep = [atlas.hierarchy.counts(l)["numDeepTexels"] for l in range(min(4, len(routes)))]
+            if on and k <= 4:
+                assert all(r == 3 for r, d in zip(routes, deep) if d > 0), routes
+            if not on:
+                assert 3 not in routes
+                assert texels == 0 or 2 in routes
+    finally:
+        atlas.set("chart_cluster", 1)
+        atlas.set("chart_texels", 1000)
+    np.testing.assert_array_equal(got[1, 1000], got[0, 0])
+    np.testing.assert_array_equal(got[0, 1000], got[0, 0])
