@@ -668,6 +668,126 @@ __global__ void __launch_bounds__(bs_dense_threads<T>(Q, mode)) k_bs_dense(Bound
   }
 }
 
+// The same products with a CTA per chunk of a row group and the chunks' sums in global
+// memory; the last CTA of a row group to finish adds them in chunk order.  The same bits.
+template <typename T, int W>
+__global__ void __launch_bounds__(256, 3) k_bs_chunks(BoundaryDev<T> B, int mode, T* __restrict__ x, int KP, int G) {
+  __shared__ T red[8][32][4 * W];
+  __shared__ Vec<T, W> vin[kBoundaryChunkMax];
+  __shared__ int lastFlag;
+  // the block's task, its matrix and its rows of it are set-up data: read (and
+  // the rows prefetched into L2) before waiting for the previous launch
+  const int4 task = (mode == 0 ? B.subTasks : B.schurTasks)[blockIdx.x];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rq = task.y + lane;
+  const int r0 = mode == 0 ? B.subPtr[task.x] : 0;
+  const int m = mode == 0 ? B.subPtr[task.x + 1] - r0 : B.nS, mp = (m + 3) & ~3;
+  const T* M = mode == 0 ? B.inv + B.invOff[task.x] : B.sinv;
+  const int nch = gridDim.y, chunk = blockIdx.y;
+  const int clen = (m + nch - 1) / nch, j0 = min(m, chunk * clen), j1 = min(m, j0 + clen);
+  {
+    // rows j0..j1 of columns 4 task.y .. 4 task.y + 127 (clipped to the padded row)
+    const int col0 = 4 * task.y, cols = max(0, min(mp - col0, 128));
+    if (lane * 32 < cols * (int)sizeof(T))
+      for (int j = j0 + warp; j < j1; j += 8)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(M + (long long)j * mp + col0) + lane * 32));
+  }
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const bool active = 4 * rq < m;
+  T* part = mode == 0 ? B.subPart : B.schurPart;
+  auto store = [&](int row, int off, Vec<T, W> sum) {
+    if (mode == 0) {
+      vstore<T, W>(B.y + (long long)(r0 + row) * KP + off, sum);
+    } else {
+      vstore<T, W>(B.xs + (long long)row * KP + off, sum);
+      const T sc = B.scale[B.nI + row];
+#pragma unroll
+      for (int c = 0; c < W; c++) sum.v[c] *= sc;
+      vstore<T, W>(x + (long long)B.posGlobal[B.nI + row] * KP + off, sum);
+    }
+  };
+  for (int q = 0; q < G; q++) {
+    const int off = q * W;
+    // the chunk's input vector (mode 0: the scaled right-hand side from k_bs_prep;
+    // mode 1: minus the coupling to the interior solution)
+    if (mode == 0) {
+      for (int j = j0 + (int)threadIdx.x; j < j1; j += blockDim.x) vin[j - j0] = vload<T, W>(B.rhat + (long long)(r0 + j) * KP + off);
+    } else {
+      const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3;
+      for (int jb = j0; jb < j1; jb += 32) {  // 32 groups of 8 lanes
+        const int j = jb + grp;
+        const Vec<T, W> v = bs_schur_input_group<T, W, LoadDefault>(B, j, j < j1, KP, off, lane8);
+        if (j < j1 && lane8 == 0) vin[j - j0] = v;
+      }
+    }
+    __syncthreads();
+    T acc[4][W];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int c = 0; c < W; c++) acc[a][c] = 0;
+    if (active) {
+#pragma unroll 8
+      for (int j = j0 + warp; j < j1; j += 8) {
+        const Quad<T> mq = *reinterpret_cast<const Quad<T>*>(M + (long long)j * mp + 4 * rq);
+        const Vec<T, W> v = vin[j - j0];
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int c = 0; c < W; c++) acc[a][c] = fma(mq.v[a], v.v[c], acc[a][c]);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int c = 0; c < W; c++) red[warp][lane][a * W + c] = acc[a][c];
+    __syncthreads();
+    if (warp == 0 && active) {
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const int row = 4 * rq + a;
+        if (row >= m) continue;
+        Vec<T, W> sum;
+#pragma unroll
+        for (int c = 0; c < W; c++) {
+          T v = 0;
+          for (int w = 0; w < 8; w++) v += red[w][lane][a * W + c];
+          sum.v[c] = v;
+        }
+        if (nch > 1) vstore<T, W>(part + (((long long)blockIdx.x * nch + chunk) * 128 + 4 * lane + a) * KP + off, sum);
+        else store(row, off, sum);
+      }
+    }
+    __syncthreads();
+  }
+  if (nch == 1) return;
+  __threadfence();
+  __syncthreads();
+  int* counter = (mode == 0 ? B.subCount : B.schurCount) + blockIdx.x;
+  if (threadIdx.x == 0) {
+    const int prev = atomicAdd(counter, 1);
+    lastFlag = prev == nch - 1;
+    if (lastFlag) *counter = 0;  // ready for the next launch
+  }
+  __syncthreads();
+  if (!lastFlag) return;
+  __threadfence();
+  for (int it = threadIdx.x; it < 128 * G; it += blockDim.x) {
+    const int rt = it / G, q = it - rt * G, row = 4 * task.y + rt, off = q * W;
+    if (row >= m) continue;
+    Vec<T, W> sum;
+#pragma unroll
+    for (int c = 0; c < W; c++) sum.v[c] = 0;
+#pragma unroll 4
+    for (int ch = 0; ch < nch; ch++) {
+      const T* src = part + (((long long)blockIdx.x * nch + ch) * 128 + rt) * KP + off;
+#pragma unroll
+      for (int c = 0; c < W; c++) sum.v[c] += __ldcg(src + c);
+    }
+    store(row, off, sum);
+  }
+}
+
 // x_I = s (y - W_p xs[touch_p]) for every interior position (W_p column-major,
 // so a warp reads consecutive rows of one column)
 template <typename T, int W>
@@ -1616,53 +1736,105 @@ void launch_prolong_add(const ProlongRun* runs, int nRuns, const T* coarse, T* f
   const int G = KP / W;
   launch(k_prolong_add<T, W>, dim3(nblk((long long)nRuns * 32 * G)), s, runs, nRuns, coarse, fine, KP, G);
 }
-// One dense product of the boundary solve (mode 0: subdomains, 1: separator).
+// One dense product of the boundary solve (mode 0: subdomains, 1: separator) on clusters.
 // Channel groups per CTA: as many as the registers hold (a matrix value read once
 // for them); warp groups per CTA: one per chunk while the registers last.
 template <typename T, int W, int Q, int mode>
-static bool launch_bs_dense_q(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) {
-  const int nch = mode == 0 ? B.subChunks : B.schurChunks, tasks = mode == 0 ? B.nSubTasks : B.nSchurTasks;
-  const int CS = std::min(kBsClusterMax, nch), slots = (nch + CS - 1) / CS;
-  const int groups = std::min(bs_dense_threads<T>(Q, mode) / 256, slots);
-  const int clen = ((mode == 0 ? kBoundaryChunkMax : B.nS) + nch - 1) / nch;
-  const size_t smem = size_t(groups) * Q * clen * sizeof(Vec<T, W>) + size_t(groups) * 8 * 128 * W * sizeof(T) +
-                      size_t(nch) * ((Q * 128 * W + CS - 1) / CS) * sizeof(T);
-  if (smem > kBsDenseSmemMax) return false;
-  static std::atomic<int> attr[kMaxDevices];
-  static const bool init = [] {
-    for (auto& a : attr) a.store(kUnset);
-    return true;
-  }();
-  (void)init;
-  if (!per_device_once(attr, [] {
-        return cudaFuncSetAttribute(k_bs_dense<T, W, Q, mode>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBsDenseSmemMax)) == cudaSuccess
-                   ? 1
-                   : 0;
-      }))
-    return false;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(tasks), unsigned(CS), unsigned(KP / W / Q));
-  cfg.blockDim = dim3(unsigned(256 * groups));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim = {1, unsigned(CS), 1};
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = g_programmatic ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, k_bs_dense<T, W, Q, mode>, B, nch, clen, x, KP) == cudaSuccess;
-}
-template <typename T, int W, int mode>
-static void launch_bs_dense(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) {
+struct BsDense {
+  int nch, tasks, CS, groups, clen;
+  unsigned z;
+  size_t smem;
+  BsDense(const BoundaryDev<T>& B, int KP)
+      : nch(mode == 0 ? B.subChunks : B.schurChunks), tasks(mode == 0 ? B.nSubTasks : B.nSchurTasks), z(unsigned(KP / W / Q)) {
+    CS = std::min(kBsClusterMax, nch);
+    groups = std::min(bs_dense_threads<T>(Q, mode) / 256, (nch + CS - 1) / CS);
+    clen = ((mode == 0 ? kBoundaryChunkMax : B.nS) + nch - 1) / nch;
+    smem = size_t(groups) * Q * clen * sizeof(Vec<T, W>) + size_t(groups) * 8 * 128 * W * sizeof(T) +
+           size_t(nch) * ((Q * 128 * W + CS - 1) / CS) * sizeof(T);
+  }
+  static bool ready() {
+    static std::atomic<int> attr[kMaxDevices];
+    static const bool init = [] {
+      for (auto& a : attr) a.store(kUnset);
+      return true;
+    }();
+    (void)init;
+    return per_device_once(attr, [] {
+             return cudaFuncSetAttribute(k_bs_dense<T, W, Q, mode>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBsDenseSmemMax)) ==
+                            cudaSuccess
+                        ? 1
+                        : 0;
+           }) != 0;
+  }
+  bool fits() const { return smem <= kBsDenseSmemMax && ready(); }
+  void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at)[2], cudaStream_t s) const {
+    cfg.gridDim = dim3(unsigned(tasks), unsigned(CS), z);
+    cfg.blockDim = dim3(unsigned(256 * groups));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {1, unsigned(CS), 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = g_programmatic ? 2 : 1;
+  }
+  // clusters of this launch that run at the same time (0: none can)
+  int resident() const {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    config(cfg, at, nullptr);
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_bs_dense<T, W, Q, mode>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return clusters;
+  }
+  bool launch(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) const {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    config(cfg, at, s);
+    return cudaLaunchKernelEx(&cfg, k_bs_dense<T, W, Q, mode>, B, nch, clen, x, KP) == cudaSuccess;
+  }
+};
+// f(the variant for this width); false where none fits
+template <typename T, int W, int mode, typename F>
+static bool bs_dense_variant(const BoundaryDev<T>& B, int KP, const F& f) {
   if constexpr (W > 1) {
     const int G = KP / W;
     if constexpr (sizeof(T) == 4)
-      if (G % 4 == 0 && launch_bs_dense_q<T, W, 4, mode>(B, x, KP, s)) return;
-    if (G % 2 == 0 && launch_bs_dense_q<T, W, 2, mode>(B, x, KP, s)) return;
+      if (const BsDense<T, W, 4, mode> d(B, KP); G % 4 == 0 && d.fits()) return f(d, 4);
+    if (const BsDense<T, W, 2, mode> d(B, KP); G % 2 == 0 && d.fits()) return f(d, 2);
   }
-  launch_bs_dense_q<T, W, 1, mode>(B, x, KP, s);
+  const BsDense<T, W, 1, mode> d(B, KP);
+  return d.fits() && f(d, 1);
+}
+// On clusters: the subdomains' product where a row group has several chunks or a CTA
+// several channel groups; the separator's where its clusters of one channel group set are
+// resident together (15 at 8 CTAs: up to some 1900 rows).  Beyond, a CTA per chunk with
+// three CTAs an SM and 8 rows ahead keeps more of the matrix in flight than the clusters'
+// one or two.  Measured without overlap, FP32 of 4 channels, clusters / a CTA per chunk:
+//   separator    1228 rows 14.6 / 15.8 us, 1919 16.4 / 18.3, 2550 39 / 24, 4347 105 / 41,
+//                12017 594 / 254; 16 channels 1228 28.9 / 38.7, 2550 76 / 57, 12017 1240 / 715
+//   subdomains   112 row groups (3 chunks) 11.2 / 12.4, 263 (2) 17.6 / 19.2, 366 (1) 25.3 /
+//                16.6, 1851 (1) 86.7 / 69.7; 16 channels 450 (1) 42.4 / 41.0, 1851 139 / 178
+// Per refinement step, a 1024^2 atlas of 1024 charts, 1 / 3 / 9 channels: 2278 -> 1477, 2740
+// -> 1777, 6716 -> 5078 us, FP64 values 3880 -> 2898; 256 charts 756 -> 639; 2048^2
+// icosphere 640 -> 631.
+template <typename T, int W>
+bool bs_dense_on_clusters(const BoundaryDev<T>& B, int KP, int mode) {
+  auto rule = [mode](const auto& d, int Q) { return mode == 0 ? (d.nch > 1 || Q > 1) && d.resident() > 0 : d.tasks <= d.resident(); };
+  return mode == 0 ? bs_dense_variant<T, W, 0>(B, KP, rule) : bs_dense_variant<T, W, 1>(B, KP, rule);
+}
+template <typename T, int W, int mode>
+static void launch_bs_dense(const BoundaryDev<T>& B, T* x, int KP, cudaStream_t s) {
+  const int tasks = mode == 0 ? B.nSubTasks : B.nSchurTasks, nch = mode == 0 ? B.subChunks : B.schurChunks;
+  if (mode == 0 ? B.subPart : B.schurPart)
+    launch(k_bs_chunks<T, W>, dim3(tasks, nch), s, B, mode, x, KP, KP / W);
+  else
+    bs_dense_variant<T, W, mode>(B, KP, [&](const auto& d, int) { return d.launch(B, x, KP, s); });
 }
 template <typename T, int W>
 void launch_boundary_solve(const BoundaryDev<T>& B, const T* rhs, T* x, int KP, cudaStream_t s, bool rhsEarly) {
@@ -1828,6 +2000,7 @@ void launch_add_correction(double* x, T* e, long long n, int K, int KP, cudaStre
   template bool gs_rows_available<T, W>(const LevelDev<T>&);                                                             \
   template size_t gs_rows_smem<T, W>(const LevelDev<T>&);                                                                \
   template bool launch_gs_groups<T, W>(const LevelDev<T>&, int, bool, int, cudaStream_t, bool);                          \
+  template bool bs_dense_on_clusters<T, W>(const BoundaryDev<T>&, int, int);                                              \
   template void launch_residual<T, W>(const ColourRun*, int, const T*, int, const int*, const int*, const T*, const int*, \
                                       int, const T*, const T*, T*, int, cudaStream_t, bool);                             \
   template void launch_restrict<T, W>(const RestrictRun*, int, const int*, const int*, const T*, const int*, int,        \

@@ -71,6 +71,10 @@ struct BoundaryDev {
   const long long* wOff = nullptr;
   const T* wt = nullptr;                // Inv_p A_{I_p,touch}, column-major m x t_p
   T *y = nullptr, *xs = nullptr;        // work
+  // chunk sums (tasks x chunks x 128 x KP) and arrival counters (zero between
+  // launches) of the products that run with a CTA per chunk; null: on clusters
+  T *subPart = nullptr, *schurPart = nullptr;
+  int *subCount = nullptr, *schurCount = nullptr;
   T* rhat = nullptr;                    // scaled right-hand side s (rhs - BD x) per position (work)
 };
 
@@ -203,6 +207,10 @@ void launch_restrict(const RestrictRun* runs, int nRuns, const int* rPtr, const 
                      int nB, const T* res, T* coarseRhs, T* coarseX, long long coarseTexels, int KP, cudaStream_t s);
 template <typename T, int W>
 void launch_prolong_add(const ProlongRun* runs, int nRuns, const T* coarse, T* fine, int KP, cudaStream_t s);
+// Whether the dense product of the subdomains (mode 0) or of the separator (1) runs on
+// clusters; otherwise it needs its chunk sums (subPart ... schurCount)
+template <typename T, int W>
+bool bs_dense_on_clusters(const BoundaryDev<T>& B, int KP, int mode);
 template <typename T, int W>
 // rhsEarly: the previous launch in the stream does not write rhs (the
 // prolongation before the solve after the coarse correction)

@@ -928,6 +928,24 @@ bool DeviceSystem::refresh_multigrids() {
   return true;
 }
 
+// the buffers of the boundary products that do not run on clusters
+template <typename T>
+static void alloc_chunk_sums(DeviceArena& A, dev::BoundaryDev<T>& B, int KP) {
+  auto on_clusters = [&](int mode) {
+    return KP % 4 == 0 ? dev::bs_dense_on_clusters<T, 4>(B, KP, mode) : dev::bs_dense_on_clusters<T, 1>(B, KP, mode);
+  };
+  B.subPart = B.schurPart = nullptr;
+  B.subCount = B.schurCount = nullptr;
+  if (B.nSubTasks > 0 && !on_clusters(0)) {
+    B.subPart = static_cast<T*>(A.alloc(size_t(B.nSubTasks) * B.subChunks * 128 * KP * sizeof(T)));
+    B.subCount = A.zeros<int>(B.nSubTasks);
+  }
+  if (B.nS > 0 && !on_clusters(1)) {
+    B.schurPart = static_cast<T*>(A.alloc(size_t(B.nSchurTasks) * B.schurChunks * 128 * KP * sizeof(T)));
+    B.schurCount = A.zeros<int>(B.nSchurTasks);
+  }
+}
+
 template <typename T>
 bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
   const double tBuild = now_ms();
@@ -1166,6 +1184,7 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
       B.asiVal = values(vals ? vals->ASI.val : std::vector<double>(), bs.ASI.col.size());
       B.y = static_cast<T*>(A.alloc(size_t(std::max(1, bs.nI)) * KP * sizeof(T)));
       B.xs = static_cast<T*>(A.alloc(size_t(std::max(1, bs.nS)) * KP * sizeof(T)));
+      alloc_chunk_sums(A, B, KP);
       B.rhat = static_cast<T*>(A.alloc(size_t(std::max(1, bs.nb)) * KP * sizeof(T)));
       return true;
     };
@@ -1264,6 +1283,7 @@ bool DeviceSystem::derive_multigrid(const Multigrid<T>& base, Multigrid<T>& mg, 
     if (B.nb == 0) continue;
     B.y = static_cast<T*>(A.alloc(size_t(std::max(1, B.nI)) * KP * sizeof(T)));
     B.xs = static_cast<T*>(A.alloc(size_t(std::max(1, B.nS)) * KP * sizeof(T)));
+    alloc_chunk_sums(A, B, KP);
     B.rhat = static_cast<T*>(A.alloc(size_t(std::max(1, B.nb)) * KP * sizeof(T)));
   }
   if (!check(A.last, "multigrid vectors")) return false;
@@ -1311,6 +1331,9 @@ std::vector<double> DeviceSystem::level_routes() const {
     const LevelDev<T>& D = mg->levels[l];
     const int KP = mg->KP, W = KP % 4 == 0 ? 4 : 1;
     v.push_back(tiled(D, KP) ? 4 : clustered(D, KP) ? 3 : grouped(D, KP) ? 2 : row_sweeps_on(D, KP, sizeof(T), W) ? 1 : 0);
+    const dev::BoundaryDev<T>& B = D.B;
+    v.push_back(B.nSubTasks == 0 ? 0 : B.subPart ? 2 : 1);
+    v.push_back(B.nS == 0 ? 0 : B.schurPart ? 2 : 1);
   }
   return v;
 }

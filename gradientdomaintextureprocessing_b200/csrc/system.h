@@ -283,7 +283,8 @@ class DeviceSystem {
   // x chunks, chart groups, largest chart (deep texels)
   std::vector<double> level_stats() const;
   // per level but the coarsest of the last built FP32 (or FP64) multigrid, what smooths it:
-  // 0 colour passes, 1 row launches, 2 a block per chart, 3 chart clusters, 4 tiles
+  // 0 colour passes, 1 row launches, 2 a block per chart, 3 chart clusters, 4 tiles; and
+  // its subdomains' and its separator's product: 0 none, 1 on clusters, 2 a CTA per chunk
   template <typename T>
   std::vector<double> level_routes() const;
   // last set-up, ms: update (weights, Galerkin coarsening, FP64 operators),

@@ -56,7 +56,7 @@ def test_charts_smooth_on_clusters(atlas, k, precision):
             atlas.set("chart_cluster", on)
             atlas.set("chart_texels", texels)
             got[on, texels] = atlas.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
-            routes = atlas.array("levelRoutes", 1 if precision == "fp64" else 0)
+            routes = atlas.array("levelRoutes", 1 if precision == "fp64" else 0)[::3]
             deep = [atlas.hierarchy.counts(l)["numDeepTexels"] for l in range(min(4, len(routes)))]
             if on and k <= 4:
                 assert all(r == 3 for r, d in zip(routes, deep) if d > 0), routes
@@ -68,3 +68,41 @@ def test_charts_smooth_on_clusters(atlas, k, precision):
         atlas.set("chart_texels", 1000)
     np.testing.assert_array_equal(got[1, 1000], got[0, 0])
     np.testing.assert_array_equal(got[0, 1000], got[0, 0])
+
+
+def test_boundary_products_run_where_they_are_faster(atlas):
+    """The largest separators, more row groups than there are resident clusters, and the
+    subdomains' product of one chunk take a CTA per chunk."""
+    b, _ = vectors(atlas.n, 3)
+    for precision, wide in (("mixed", 0), ("fp64", 1)):
+        atlas.set("max_block", atlas.get("max_block"))  # drops the multigrids of other widths
+        atlas.solve(b, tol=1e-30, max_iters=1, check=False, precision=precision)
+        routes = atlas.array("levelRoutes", wide).reshape(-1, 3)
+        if not wide:
+            stats = atlas.array("levelStats").reshape(-1, 9)
+            for (_, sub, schur), row in zip(routes, stats):
+                rows = row[4]
+                assert schur == (0 if rows == 0 else 1 if rows <= 1792 else 2) or 1792 < rows <= 2304
+        assert routes[0][1] == 2 or atlas.charts < 400
+        assert routes[0][2] == 2 or atlas.charts < 400
+
+
+@pytest.mark.parametrize("k", [1, 3, 6, 9])
+def test_boundary_products_give_the_same_bits(atlas, k):
+    """A CTA per chunk against the coarse-level cluster kernel (the same chunks, added in the
+    same order), and one column alone against k columns, whose products may run otherwise."""
+    b, x = (v.astype(np.float32) for v in vectors(atlas.n, k))
+    wide = atlas.vcycle(x, b)
+    for c in {0, k - 1}:
+        np.testing.assert_array_equal(wide[:, c], atlas.vcycle(x[:, c], b[:, c])[:, 0])
+    if k > 4:
+        return
+    out = {}
+    for precision in ("mixed", "fp64"):
+        for texels in (0, 1 << 30):
+            try:
+                atlas.set("cluster_texels", texels)
+                out[texels] = atlas.solve(b.astype(float), tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+            finally:
+                atlas.set("cluster_texels", 0)
+        np.testing.assert_array_equal(out[0], out[1 << 30])
