@@ -297,10 +297,10 @@ __global__ void __launch_bounds__(256) k_residual(const ColourRun* __restrict__ 
                                                   int planeStride, int deepBlocks, const int* __restrict__ bPtr,
                                                   const int* __restrict__ bCol, const T* __restrict__ bVal,
                                                   const int* __restrict__ bGlobal, int nB, const T* __restrict__ rhs,
-                                                  const T* __restrict__ x, T* __restrict__ res, int KP, int G, int rhsEarly) {
+                                                  const T* __restrict__ x, T* __restrict__ res, int KP, int G, int rhsEarly, int rowLanes) {
   if ((int)blockIdx.x >= deepBlocks) {
     const long long t = (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x;
-    if (G > 1) {  // several channel groups: a thread per row and group (row8_lanes)
+    if (rowLanes == 1) {  // a thread per row and group (row_lanes)
       grid_dependency_wait();
       grid_launch_dependents();
       residual_boundary_item<T, W, LoadDefault>(bPtr, bCol, bVal, bGlobal, nB, rhs, x, res, KP, G, t);
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(256) k_restrict(const RestrictRun* __restrict_
                                                   const int* __restrict__ rPtr, const int* __restrict__ rCol,
                                                   const T* __restrict__ rVal, const int* __restrict__ rOut, int nB,
                                                   const T* __restrict__ res, T* __restrict__ coarseRhs, T* __restrict__ coarseX,
-                                                  long long coarseVals, int KP, int G) {
+                                                  long long coarseVals, int KP, int G, int rowLanes) {
   // the coarse iterate starts from zero: cleared here (grid-stride), before
   // waiting for the previous launch (the residual of this level, which does
   // not touch the coarse level)
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256) k_restrict(const RestrictRun* __restrict_
     return;
   }
   const long long t = (long long)(blockIdx.x - deepBlocks) * blockDim.x + threadIdx.x;
-  if (G > 1) {
+  if (rowLanes == 1) {
     grid_dependency_wait();
     grid_launch_dependents();
     restrict_boundary_item<T, W, LoadDefault>(rPtr, rCol, rVal, rOut, nB, res, coarseRhs, KP, G, t);
@@ -1324,8 +1324,14 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
 
 // The same for K = KT <= 4 right-hand sides.
 //  * A warp takes a run, its header loaded during the run before.
-//  * Boundary rows run on 8 lanes (OrderedRow8), before the deep rows, whose loads
-//    hide their trips; the first rows' entries are loaded before the dependency wait.
+//  * Boundary rows come before the deep rows, whose loads hide their trips: a thread per
+//    row, the warps of rows dealt to the blocks in turn, since blocks that are launched
+//    early share few SMs (rows in the first blocks: 42.5 instead of 19 us at 1024^2).  On 8
+//    lanes with the first entries loaded ahead (OrderedRow8) the shuffles cost more than
+//    the trips: 3 right-hand sides of a 256^2 torus 116.5 / 111.6 us per step, of icospheres
+//    of 28 k rows 279 / 277, of 60 k 633.5 / 621.7, 16 x 16 charts of 123 k rows 625 / 593; one
+//    right-hand side 15 k rows 134.2 / 135.5, 29 k 197.9 / 200.5, 123 k 461.7 / 449.2.  The
+//    rows' threads are the same for every KT: so are the norms, whatever is solved together.
 // What bounds it at 2048^2 (77 us for 203 MB): half the warps (64 registers), each a
 // long-scoreboard wait of 10.6 of 17.9 cycles per issue, and 58 % of the first-level
 // cache's cycles; a lane per value instead of per texel (consecutive addresses, but
@@ -1336,7 +1342,7 @@ __global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict_
                                                     const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
                                                     const double* __restrict__ b, const double* __restrict__ x, double* __restrict__ out,
                                                     int mode, double* __restrict__ partials, float* __restrict__ out32, int KP) {
-  const int lane = threadIdx.x & 31, lane8 = threadIdx.x & 7;
+  const int lane = threadIdx.x & 31;
   const int warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
   double rr[4] = {0, 0, 0, 0}, bb[4] = {0, 0, 0, 0};
   // row g: its value from the sums, its share of the norms
@@ -1353,34 +1359,19 @@ __global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict_
     if (out32)  // zero the padding channels
       for (int c = KT; c < KP; c++) out32[(long long)g * KP + c] = 0.f;
   };
-  {
-    int row = warp0 * 4 + (lane >> 3);
-    auto range = [&](int r, int& k0, int& k1, int& g) {
-      const bool valid = r < nB;
-      g = valid ? bGlobal[r] : 0;
-      k0 = valid && mode != 3 ? bPtr[r] : 0;
-      k1 = valid && mode != 3 ? bPtr[r + 1] : 0;
-    };
-    int k0, k1, g;
-    range(row, k0, k1, g);
-    OrderedRow8<double, KT, 2> entries(bCol, bVal, k0, k1, lane8);
-    grid_dependency_wait();
-    grid_launch_dependents();
-    for (int w = warp0; w * 4 < nB; w += warps) {
-      Vec<double, KT> acc;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  for (int row = (blockIdx.x + gridDim.x * (threadIdx.x >> 5)) * 32 + lane; row < nB; row += gridDim.x * blockDim.x) {
+    double acc[KT];
 #pragma unroll
-      for (int ch = 0; ch < KT; ch++) acc.v[ch] = 0;
-      entries.add_to(acc, false, bCol, bVal, lane8, [&](int c) {
-        Vec<double, KT> v;
+    for (int ch = 0; ch < KT; ch++) acc[ch] = 0;
+    for (int k = mode == 3 ? bPtr[row + 1] : bPtr[row]; k < bPtr[row + 1]; k++) {
+      const double w = bVal[k];
+      const double* xs = x + (long long)bCol[k] * KT;
 #pragma unroll
-        for (int ch = 0; ch < KT; ch++) v.v[ch] = x[(long long)c * KT + ch];
-        return v;
-      });
-      if (row < nB && lane8 == 0) finish(g, acc.v);
-      row += warps * 4;
-      range(row, k0, k1, g);
-      entries = OrderedRow8<double, KT, 2>(bCol, bVal, k0, k1, lane8);
+      for (int ch = 0; ch < KT; ch++) acc[ch] = fma(w, xs[ch], acc[ch]);
     }
+    finish(bGlobal[row], acc);
   }
   ColourRun R;
   R.len = 0;
@@ -1704,31 +1695,40 @@ bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cu
   return cudaLaunchKernelEx(&cfg, k_gs_groups<T, W>, D.runs, D.groups, (const T*)D.coef, D.planeStride, (const T*)D.b, D.x, KP, G,
                             sweeps, reverse ? 1 : 0) == cudaSuccess;
 }
-// Lanes per boundary row of the residual and the restriction: 8 for one channel
-// group (a row one term after another was the launch's time: residual and
-// restriction of a 256^2 torus 4.7 and 3.9 us, the FP64 operator of a 1024^2 genus-2
-// 15.5 us of a 146 us CG step; 140 -> 152 us per step without the 8 lanes for a
-// 1013 x 1187 genus-2); with several groups the threads of a row's groups read its
-// texels' values contiguously, and there are enough rows in flight.
-static int row8_lanes(int G) { return G == 1 ? 8 : 1; }
+// Lanes per boundary row of the residual and the restriction: 8 for one channel group
+// (a row one term after another was the launch's time: residual and restriction of a
+// 256^2 torus 4.7 and 3.9 us, 140 -> 152 us per step without the 8 lanes for a 1013 x 1187
+// genus-2), as long as the rows do not fill the chip by themselves: 8 lanes hand every
+// term round, (1 + W) words of it, so `limit` is in rows times words.  With several groups
+// the threads of a row's groups read its texels' values contiguously.  Per step, 8 lanes
+// everywhere / the residual's rows on one: 28 k rows of 4 floats 279 / 292 us, 60 k 633 / 631,
+// 123 k 625 / 617, 229 k 1709 / 1686, of 4 doubles 2766 / 2736; the restriction's on one: 60 k
+// 633 / 643, 229 k 1709 / 1707, of 4 doubles 2766 / 2711.  With the operator's rows
+// (k_raw_few): 1024^2 of 1024 charts, 3 channels 1755 -> 1689 us, 256 charts 631 -> 591, 64
+// charts 491 -> 479, 2048^2 icosphere 632 -> 617.
+constexpr long long kResidualRows8 = 200000, kRestrictRows8 = 1200000;
+template <typename T, int W>
+static int row_lanes(int nB, int G, long long limit) {
+  return G == 1 && nB * (1 + W) * (long long)sizeof(T) / 4 <= limit ? 8 : 1;
+}
 template <typename T, int W>
 void launch_residual(const ColourRun* runs, int nRuns, const T* coef, int planeStride, const int* bPtr, const int* bCol,
                      const T* bVal, const int* bGlobal, int nB, const T* rhs, const T* x, T* res, int KP, cudaStream_t s,
                      bool rhsEarly) {
   const int G = KP / W;
-  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * row8_lanes(G));
+  const int lanes = row_lanes<T, W>(nB, G, kResidualRows8), db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * lanes);
   if (db + bb == 0) return;
   launch(k_residual<T, W>, dim3(db + bb), s, runs, nRuns, coef, planeStride, db, bPtr, bCol, bVal, bGlobal, nB, rhs, x, res, KP, G,
-         rhsEarly ? 1 : 0);
+         rhsEarly ? 1 : 0, lanes);
 }
 template <typename T, int W>
 void launch_restrict(const RestrictRun* runs, int nRuns, const int* rPtr, const int* rCol, const T* rVal, const int* rOut,
                      int nB, const T* res, T* coarseRhs, T* coarseX, long long coarseTexels, int KP, cudaStream_t s) {
   const int G = KP / W;
-  const int db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * row8_lanes(G));
+  const int lanes = row_lanes<T, W>(nB, G, kRestrictRows8), db = nblk((long long)nRuns * 32 * G), bb = nblk((long long)nB * G * lanes);
   if (db + bb == 0 && coarseTexels == 0) return;
   launch(k_restrict<T, W>, dim3(std::max(1, db + bb)), s, runs, nRuns, db, rPtr, rCol, rVal, rOut, nB, res, coarseRhs, coarseX,
-         coarseTexels * KP, KP, G);
+         coarseTexels * KP, KP, G, lanes);
 }
 template <typename T, int W>
 void launch_prolong_add(const ProlongRun* runs, int nRuns, const T* coarse, T* fine, int KP, cudaStream_t s) {

@@ -106,3 +106,26 @@ def test_boundary_products_give_the_same_bits(atlas, k):
             finally:
                 atlas.set("cluster_texels", 0)
         np.testing.assert_array_equal(out[0], out[1 << 30])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+def test_boundary_rows_give_the_same_sums(atlas, k):
+    """A boundary row on one lane and on 8, by their number and the width: the operator's and
+    the residual's columns alone and among 9 (several channel groups: a thread per row and
+    group), with odd widths in between."""
+    x, b = vectors(atlas.n, 9)
+    y = atlas.apply(x)
+    part = atlas.apply(np.ascontiguousarray(x[:, :k]))
+    np.testing.assert_array_equal(part, y[:, :k])
+    for precision in ("mixed", "fp64"):
+        wide = atlas.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+        got = atlas.solve(np.ascontiguousarray(b[:, :k]), tol=1e-30, max_iters=2, check=False, precision=precision)[0]
+        np.testing.assert_array_equal(got, wide[:, :k])
+
+
+@pytest.mark.parametrize("k", [1, 3])
+def test_norms_of_many_rows(atlas, k):
+    """The norms add every row once: relative error at most n 2^-53 (n <= 1e6), so 1e-9."""
+    b, x = vectors(atlas.n, k)
+    r = b - atlas.apply(x)
+    np.testing.assert_allclose(atlas.residual(b, x), np.sqrt((r * r).sum(0) / (b * b).sum(0)), rtol=1e-9)
