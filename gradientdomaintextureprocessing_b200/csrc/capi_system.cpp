@@ -134,7 +134,7 @@ extern "C" int gdtp_system_array(const gdtp_system* s, const char* cname, int le
     }
     if (name == "profile.setup") return vec(std::vector<double>(s->sys->setupMs, s->sys->setupMs + 14));
     if (name == "levelStats") return vec(s->sys->level_stats());  // 9 per level, see DeviceSystem::level_stats
-    if (name == "levelRoutes") return vec(level ? s->sys->level_routes<double>() : s->sys->level_routes<float>());
+    if (name == "levelRoutes") return vec(s->sys->level_routes(level));  // level: right-hand sides, 0 FP64
     if (name == "levelsUsed") {
       if (count) *count = 1;
       if (out) *static_cast<int32_t*>(out) = s->sys->levelsUsed();

@@ -1322,23 +1322,23 @@ std::vector<double> DeviceSystem::level_stats() const {
 }
 
 template <typename T>
-std::vector<double> DeviceSystem::level_routes() const {
-  const Multigrid<T>* mg = nullptr;
-  if constexpr (sizeof(T) == 4) mg = mg32_.empty() ? nullptr : mg32_.back().get();
-  else mg = mg64_.get();
-  std::vector<double> v;
-  for (size_t l = 0; mg && l + 1 < mg->levels.size(); l++) {
-    const LevelDev<T>& D = mg->levels[l];
-    const int KP = mg->KP, W = KP % 4 == 0 ? 4 : 1;
+void DeviceSystem::append_routes(const Multigrid<T>& mg, std::vector<double>& v) const {
+  for (size_t l = 0; l + 1 < mg.levels.size(); l++) {
+    const LevelDev<T>& D = mg.levels[l];
+    const int KP = mg.KP, W = KP % 4 == 0 ? 4 : 1;
     v.push_back(tiled(D, KP) ? 4 : clustered(D, KP) ? 3 : grouped(D, KP) ? 2 : row_sweeps_on(D, KP, sizeof(T), W) ? 1 : 0);
     const dev::BoundaryDev<T>& B = D.B;
     v.push_back(B.nSubTasks == 0 ? 0 : B.subPart ? 2 : 1);
     v.push_back(B.nS == 0 ? 0 : B.schurPart ? 2 : 1);
   }
+}
+std::vector<double> DeviceSystem::level_routes(int k) const {
+  std::vector<double> v;
+  if (k == 0 && mg64_) append_routes(*mg64_, v);
+  for (const auto& m : mg32_)
+    if (k > 0 && m->KP == kp_for(k)) append_routes(*m, v);
   return v;
 }
-template std::vector<double> DeviceSystem::level_routes<float>() const;
-template std::vector<double> DeviceSystem::level_routes<double>() const;
 
 bool DeviceSystem::cluster_timeline(std::vector<unsigned long long>& out) {
   out.clear();

@@ -282,11 +282,11 @@ class DeviceSystem {
   // texels, subdomain rows, separator rows, subdomain tasks x chunks, Schur tasks
   // x chunks, chart groups, largest chart (deep texels)
   std::vector<double> level_stats() const;
-  // per level but the coarsest of the last built FP32 (or FP64) multigrid, what smooths it:
-  // 0 colour passes, 1 row launches, 2 a block per chart, 3 chart clusters, 4 tiles; and
-  // its subdomains' and its separator's product: 0 none, 1 on clusters, 2 a CTA per chunk
-  template <typename T>
-  std::vector<double> level_routes() const;
+  // per level but the coarsest of the FP32 multigrid for k right-hand sides (k = 0: of the
+  // FP64 one; empty when not built) what smooths it: 0 colour passes, 1 row launches, 2 a
+  // block per chart, 3 chart clusters, 4 tiles; and its subdomains' and its separator's
+  // product: 0 none, 1 on clusters, 2 a CTA per chunk
+  std::vector<double> level_routes(int k) const;
   // last set-up, ms: update (weights, Galerkin coarsening, FP64 operators),
   // boundary solver factorisations, coarsest inverse, other multigrid set-up
   // (device layouts, uploads); the last three when the multigrid is built;
@@ -331,6 +331,8 @@ class DeviceSystem {
   // iterate and right-hand side (padded), and the iterate back: padded and stripped
   // on the device (value by value on the host a V-cycle on 640 x 480 RGB vectors took
   // 21.0 ms, now 0.82)
+  template <typename T>
+  void append_routes(const Multigrid<T>& mg, std::vector<double>& v) const;
   template <typename T>
   bool vectors_in(Multigrid<T>& mg, const T* x, const T* rhs, int k);
   template <typename T>

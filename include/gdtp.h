@@ -123,10 +123,11 @@ void gdtp_system_free(gdtp_system* s);
  *   kernels per step graph, kernels launched by solves, the timed group's smoother:
  *   1 one fused tile-smoother launch, 2 a sweep of two row-smoother launches, 0 a
  *   sweep of four colour passes}; "profile.reset" clears the counts
- *   "levelRoutes": per level but the coarsest of the last built FP32 multigrid (level 1:
- *   of the FP64 one) what smooths it: 0 colour passes, 1 row launches, 2 a block per
- *   chart, 3 a cluster per chart, 4 tiles; then its boundary subdomains' and its
- *   separator's product: 0 none, 1 on clusters, 2 a CTA per chunk (3 per level)
+ *   "levelRoutes": per level but the coarsest of the FP32 multigrid for `level`
+ *   right-hand sides (0: of the FP64 one; empty when not built) what smooths it: 0
+ *   colour passes, 1 row launches, 2 a block per chart, 3 a cluster per chart, 4
+ *   tiles; then its boundary subdomains' and its separator's product: 0 none, 1 on
+ *   clusters, 2 a CTA per chunk (3 per level)
  *   "fault.barrier" (no values): the built multigrids' grid barriers read as timed
  *   out, as after a lost block: the next V-cycle that uses one fails
  *   "profile.setup": ms of the last set-up {update, boundary solver factorisations,

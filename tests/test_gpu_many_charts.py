@@ -56,7 +56,7 @@ def test_charts_smooth_on_clusters(atlas, k, precision):
             atlas.set("chart_cluster", on)
             atlas.set("chart_texels", texels)
             got[on, texels] = atlas.solve(b, tol=1e-30, max_iters=2, check=False, precision=precision)[0]
-            routes = atlas.array("levelRoutes", 1 if precision == "fp64" else 0)[::3]
+            routes = atlas.array("levelRoutes", 0 if precision == "fp64" else k)[::3]
             deep = [atlas.hierarchy.counts(l)["numDeepTexels"] for l in range(min(4, len(routes)))]
             if on and k <= 4:
                 assert all(r == 3 for r, d in zip(routes, deep) if d > 0), routes
@@ -74,11 +74,11 @@ def test_boundary_products_run_where_they_are_faster(atlas):
     """The largest separators, more row groups than there are resident clusters, and the
     subdomains' product of one chunk take a CTA per chunk."""
     b, _ = vectors(atlas.n, 3)
-    for precision, wide in (("mixed", 0), ("fp64", 1)):
+    for precision, width in (("mixed", 3), ("fp64", 0)):
         atlas.set("max_block", atlas.get("max_block"))  # drops the multigrids of other widths
         atlas.solve(b, tol=1e-30, max_iters=1, check=False, precision=precision)
-        routes = atlas.array("levelRoutes", wide).reshape(-1, 3)
-        if not wide:
+        routes = atlas.array("levelRoutes", width).reshape(-1, 3)
+        if width:
             stats = atlas.array("levelStats").reshape(-1, 9)
             for (_, sub, schur), row in zip(routes, stats):
                 rows = row[4]
