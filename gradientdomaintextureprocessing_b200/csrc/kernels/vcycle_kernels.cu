@@ -1322,19 +1322,23 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
 
 // The same for K = KT <= 4 right-hand sides.
 //  * A warp takes a run, its header loaded during the run before.
-//  * Boundary rows come before the deep rows, whose loads hide their trips: a thread per
-//    row, the warps of rows dealt to the blocks in turn, since blocks that are launched
-//    early share few SMs (rows in the first blocks: 42.5 instead of 19 us at 1024^2).  On 8
-//    lanes with the first entries loaded ahead (OrderedRow8) the shuffles cost more than
-//    the trips: 3 right-hand sides of a 256^2 torus 116.5 / 111.6 us per step, of icospheres
-//    of 28 k rows 279 / 277, of 60 k 633.5 / 621.7, 16 x 16 charts of 123 k rows 625 / 593; one
-//    right-hand side 15 k rows 134.2 / 135.5, 29 k 197.9 / 200.5, 123 k 461.7 / 449.2.  The
-//    rows' threads are the same for every KT: so are the norms, whatever is solved together.
+//  * Boundary rows come before the deep rows, whose loads hide their trips.  A warp takes 4
+//    of them (FEW: at most kRawRowsFew, one pass of the chip) or 32, the warps dealt to the
+//    blocks in turn, since blocks that are launched early share few SMs (rows in the first
+//    blocks: 42.5 instead of 19 us at 1024^2).  The threads that add a row to the norms are
+//    the same for every KT: so are the norms, whatever is solved together.  One right-hand
+//    side of few rows takes 8 lanes a row with the first entries loaded ahead; with more,
+//    handing the terms round costs more than the trips it saves.  Per step, 8 lanes always
+//    / now: 3 right-hand sides, 256^2 torus 115.5 / 110 us, 1013 x 1187 genus-2 170.6 / 167,
+//    icospheres of 28 k rows 277.8 / 276.2, of 60 k 632 / 617, 16 x 16 charts of 123 k rows 631
+//    / 591; one, 256^2 torus 85.5 / 83.8, 640 x 480 183.8 / 185.6, 16 x 16 charts 467 / 452 (a
+//    thread per row also where there are few: genus-2 of 15 k rows 134.2 / 135.5, of 29 k
+//    197 / 200.8).
 // What bounds it at 2048^2 (77 us for 203 MB): half the warps (64 registers), each a
 // long-scoreboard wait of 10.6 of 17.9 cycles per issue, and 58 % of the first-level
 // cache's cycles; a lane per value instead of per texel (consecutive addresses, but
 // the coefficients read for every channel) took 85 us.
-template <int KT>
+template <int KT, bool FEW>
 __global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict__ runs, int nRuns, const double* __restrict__ coef,
                                                     int planeStride, const int* __restrict__ bPtr, const int* __restrict__ bCol,
                                                     const double* __restrict__ bVal, const int* __restrict__ bGlobal, int nB,
@@ -1357,19 +1361,49 @@ __global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict_
     if (out32)  // zero the padding channels
       for (int c = KT; c < KP; c++) out32[(long long)g * KP + c] = 0.f;
   };
-  grid_dependency_wait();
-  grid_launch_dependents();
-  for (int row = (blockIdx.x + gridDim.x * (threadIdx.x >> 5)) * 32 + lane; row < nB; row += gridDim.x * blockDim.x) {
-    double acc[KT];
-#pragma unroll
-    for (int ch = 0; ch < KT; ch++) acc[ch] = 0;
-    for (int k = mode == 3 ? bPtr[row + 1] : bPtr[row]; k < bPtr[row + 1]; k++) {
-      const double w = bVal[k];
-      const double* xs = x + (long long)bCol[k] * KT;
-#pragma unroll
-      for (int ch = 0; ch < KT; ch++) acc[ch] = fma(w, xs[ch], acc[ch]);
+  const int rowWarp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+  if constexpr (FEW && KT == 1) {
+    const int lane8 = lane & 7;
+    int row = rowWarp * 4 + (lane >> 3), k0, k1, g;
+    auto range = [&] {
+      const bool valid = row < nB;
+      g = valid ? bGlobal[row] : 0;
+      k0 = valid && mode != 3 ? bPtr[row] : 0;
+      k1 = valid && mode != 3 ? bPtr[row + 1] : 0;
+    };
+    range();
+    OrderedRow8<double, KT, 2> entries(bCol, bVal, k0, k1, lane8);
+    grid_dependency_wait();
+    grid_launch_dependents();
+    for (int first = rowWarp * 4; first < nB; first += warps * 4) {
+      Vec<double, KT> acc;
+      acc.v[0] = 0;
+      entries.add_to(acc, false, bCol, bVal, lane8, [&](int c) {
+        Vec<double, KT> v;
+        v.v[0] = x[c];
+        return v;
+      });
+      if (row < nB && lane8 == 0) finish(g, acc.v);
+      row += warps * 4;
+      range();
+      entries = OrderedRow8<double, KT, 2>(bCol, bVal, k0, k1, lane8);
     }
-    finish(bGlobal[row], acc);
+  } else {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (!FEW || (lane & 7) == 0)
+      for (int row = FEW ? rowWarp * 4 + (lane >> 3) : rowWarp * 32 + lane; row < nB; row += warps * (FEW ? 4 : 32)) {
+        double acc[KT];
+#pragma unroll
+        for (int ch = 0; ch < KT; ch++) acc[ch] = 0;
+        for (int k = mode == 3 ? bPtr[row + 1] : bPtr[row]; k < bPtr[row + 1]; k++) {
+          const double w = bVal[k];
+          const double* xs = x + (long long)bCol[k] * KT;
+#pragma unroll
+          for (int ch = 0; ch < KT; ch++) acc[ch] = fma(w, xs[ch], acc[ch]);
+        }
+        finish(bGlobal[row], acc);
+      }
   }
   ColourRun R;
   R.len = 0;
@@ -1900,6 +1934,7 @@ static bool launch_sums(const SumTarget& t, int blocks, int K, cudaStream_t s, i
 // most 8 per SM).  K <= 4 against the kernel for any K, per step: LIC on a 1024^2
 // genus-2 134 -> 129 us, its filtering at 1013 x 1187 140 -> 134, 1024^2 icosphere 307
 // -> 303; half the blocks (one wave) 127, 136 and 306.
+constexpr int kRawRowsFew = 32000;
 static int launch_raw(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
                       const double* bVal, const int* bGlobal, int nB, const double* b, const double* x, double* out, int K, int mode,
                       double* partials, float* out32, int KP, cudaStream_t s) {
@@ -1918,10 +1953,11 @@ static int launch_raw(const ColourRun* runs, int nRuns, const double* coef, int 
   auto go = [&](auto kernel) {
     launch(kernel, dim3(blocks), s, runs, nRuns, coef, planeStride, bPtr, bCol, bVal, bGlobal, nB, b, x, out, mode, partials, out32, KP);
   };
-  if (K == 1) go(k_raw_few<1>);
-  else if (K == 2) go(k_raw_few<2>);
-  else if (K == 3) go(k_raw_few<3>);
-  else go(k_raw_few<4>);
+  const bool few = nB <= kRawRowsFew;
+  if (K == 1) few ? go(k_raw_few<1, true>) : go(k_raw_few<1, false>);
+  else if (K == 2) few ? go(k_raw_few<2, true>) : go(k_raw_few<2, false>);
+  else if (K == 3) few ? go(k_raw_few<3, true>) : go(k_raw_few<3, false>);
+  else few ? go(k_raw_few<4, true>) : go(k_raw_few<4, false>);
   return blocks;
 }
 void launch_raw_operator(const ColourRun* runs, int nRuns, const double* coef, int planeStride, const int* bPtr, const int* bCol,
