@@ -202,6 +202,8 @@ bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& 
     // more pairs per CTA than that, and charts share a cluster's CTAs (largest first)
     int pairs = 0;
     for (const std::vector<Row>& rc : rows) pairs = std::max(pairs, most_pairs(rc, C, cut));
+    cc.threads = std::max(32, (pairs + 31) / 32 * 32);
+    if (cc.threads > (C == 8 ? dev::kClusterLargeThreads : kClusterThreadsGoal)) continue;
     std::vector<std::pair<int, int>> order;  // (-CTAs, chart)
     for (int c = 0; c < nc; c++) {
       if (rows[c].empty()) continue;
@@ -272,12 +274,9 @@ bool build_chart_clusters(const GridLevel& L, const DeepRuns& R, ChartClusters& 
         cc.parts[base + p] = P;
       }
     }
-    cc.threads = std::max(32, (pairs + 31) / 32 * 32);
     cc.slab = (cc.slab + 1) & ~1;  // the kernel may swap the entries of a pair (slab_slot)
-    if (cc.threads <= kClusterThreadsGoal || (C == 8 && cc.threads <= dev::kClusterLargeThreads)) {
-      out = std::move(cc);
-      return !out.parts.empty();
-    }
+    out = std::move(cc);
+    return !out.parts.empty();
   }
   return false;
 }
