@@ -1071,8 +1071,6 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
         D.nGroups = (int)grp.size() / 10;
         D.maxGroupDeep = maxDeep;
         D.maxGroupSpan = maxSpan;
-        for (int gi = 0; gi < D.nGroups; gi++)
-          for (int c = 0; c < 4; c++) D.maxGroupColourRuns = std::max(D.maxGroupColourRuns, grp[10 * gi + 4 + c]);
       }
     }
     // boundary rows (merged BD + BB, global columns)
@@ -1508,10 +1506,10 @@ void DeviceSystem::vcycle(Multigrid<T>& mg, cudaStream_t s, bool zeroStart) {
       // x = 0 on entry (a refinement step's correction, or a level entered
       // through the restriction) unless a boundary solve ran first
       tile_smooth(mg, D, knobs.tilePreSweeps, false, (l > 0 || zeroStart) && !knobs.preBoundary, s, false);
-    } else if (clustered(D, KP) && pre_sweeps(l) > 0) {
-      dev::launch_gs_cluster<T, W>(D, pre_sweeps(l), false, (l > 0 || zeroStart) && !knobs.preBoundary, KP, s);
-    } else if (grouped(D, KP) && pre_sweeps(l) > 0) {
-      dev::launch_gs_groups<T, W>(D, pre_sweeps(l), false, KP, s);
+    } else if (clustered(D, KP) && pre_sweeps(l) > 0 &&
+               dev::launch_gs_cluster<T, W>(D, pre_sweeps(l), false, (l > 0 || zeroStart) && !knobs.preBoundary, KP, s)) {
+      // every sweep in that launch (one that is refused leaves the step to the next kind)
+    } else if (grouped(D, KP) && pre_sweeps(l) > 0 && dev::launch_gs_groups<T, W>(D, pre_sweeps(l), false, KP, s)) {
     } else {
       // timed on level 0: every full sweep (all but a first sweep that skips
       // zeros), here and in the post-smoothing; the sweep average is reported
@@ -1567,11 +1565,9 @@ void DeviceSystem::vcycle(Multigrid<T>& mg, cudaStream_t s, bool zeroStart) {
       // timed on level 0: the post-smoothing rounds (coefficients, rhs, x read
       // and written once each per round)
       tile_smooth(mg, D, knobs.tilePostSweeps, true, false, s, profiling_ && l == 0);
-    } else if (clustered(D, KP) && post_sweeps(l) > 0) {
-      dev::launch_gs_cluster<T, W>(D, post_sweeps(l), true, false, KP, s, true);
-    } else if (grouped(D, KP) && post_sweeps(l) > 0) {
-      // after the prolongation and the boundary solve, which leave the right-hand side alone
-      dev::launch_gs_groups<T, W>(D, post_sweeps(l), true, KP, s, true);
+    } else if (clustered(D, KP) && post_sweeps(l) > 0 && dev::launch_gs_cluster<T, W>(D, post_sweeps(l), true, false, KP, s, true)) {
+      // (after the prolongation and the boundary solve, which leave the right-hand side alone)
+    } else if (grouped(D, KP) && post_sweeps(l) > 0 && dev::launch_gs_groups<T, W>(D, post_sweeps(l), true, KP, s)) {
     } else {
       const bool prof = profiling_ && l == 0 && post_sweeps(l) > 0;
       if (prof) cudaEventRecordWithFlags(profEv_[2], s, cudaEventRecordExternal);
