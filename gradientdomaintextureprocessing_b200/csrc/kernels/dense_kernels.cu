@@ -39,7 +39,7 @@ namespace {
 
 constexpr int kPB = 64;  // pivot block of the blocked Gauss-Jordan elimination
 
-// C (M x N) = alpha op(A) B + beta C over a batch of tasks (blockIdx.z); op(A)
+// C (M x N) = op(A) B over a batch of tasks (blockIdx.z); op(A)
 // is A (M x K, leading dimension lda) or, with transA, the transpose of A
 // stored K x M.  64 x 64 tiles, 256 threads of 4 x 4 outputs each (rows ty +
 // 16 r, columns tx + 16 c), K in chunks of 16 through shared memory.
@@ -108,8 +108,7 @@ __global__ void __launch_bounds__(256) k_gemm(const GemmTask* __restrict__ tasks
     for (int c = 0; c < 4; c++) {
       const int gc = col0 + tx + 16 * c;
       if (gc >= T.N) continue;
-      double* dst = C + T.c + (long long)gr * T.ldc + gc;
-      *dst = T.alpha * acc[r][c] + (T.beta != 0.0 ? T.beta * *dst : 0.0);
+      C[T.c + (long long)gr * T.ldc + gc] = acc[r][c] + 0.0;  // (no negative zeros)
     }
   }
 }
@@ -384,7 +383,7 @@ __global__ void __launch_bounds__(kEThreads, 3) k_bgj_update(const GemmTask* __r
   if (!pivot) return;
   __syncthreads();  // As is free
   invert_block(P, min(kPB, T.M - row0), As, bad);
-  store_inverse(P, Pinv + (long long)T.pad * kPB * kPB);
+  store_inverse(P, Pinv + (long long)T.matrix * kPB * kPB);
 }
 
 // out = (in + in^T) / 2, a 32 x 32 tile per CTA (32 x 8 threads) with its transpose
@@ -490,12 +489,9 @@ bool spd_inverse_layout(const std::vector<int64_t>& offsets, const std::vector<i
       T.c = offsets[q];
       T.M = T.N = m;
       T.K = std::min(kPB, m - kb);
-      T.lda = kPB;
       T.ldb = m;
       T.ldc = m;
-      T.alpha = -1.0;
-      T.beta = 1.0;
-      T.pad = q;
+      T.matrix = q;
       L.tasks.push_back(T);
       L.stepMax[k] = std::max(L.stepMax[k], m);
     }
@@ -592,7 +588,6 @@ void schur_product_tasks(const std::vector<int64_t>& invOff, const std::vector<i
     g.lda = m[p];
     g.ldb = t[p];
     g.ldc = t[p];
-    g.alpha = 1.0;
     gTasks.push_back(g);
     GemmTask l{};  // local = C^T G   (t x t)
     l.a = cOff[p];
@@ -605,7 +600,6 @@ void schur_product_tasks(const std::vector<int64_t>& invOff, const std::vector<i
     l.ldb = t[p];
     l.ldc = t[p];
     l.transA = 1;
-    l.alpha = 1.0;
     lTasks.push_back(l);
     maxM = std::max(maxM, m[p]);
     maxT = std::max(maxT, t[p]);

@@ -1695,7 +1695,7 @@ size_t gs_groups_smem(const LevelDev<T>& D, int KP) {
   return size_t(D.maxGroupSpan) * KP * sizeof(T);
 }
 template <typename T, int W>
-bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s, bool rhsEarly) {
+bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s) {
   if (D.nGroups == 0 || sweeps <= 0) return true;
   const size_t smem = gs_groups_smem<T, W>(D, KP);
   if (smem > kGroupSmemMax) return false;
@@ -2033,7 +2033,7 @@ void launch_add_correction(double* x, T* e, long long n, int K, int KP, cudaStre
   template bool launch_gs_rows<T, W>(const LevelDev<T>&, int, bool, int, cudaStream_t, int, bool);                       \
   template bool gs_rows_available<T, W>(const LevelDev<T>&);                                                             \
   template size_t gs_rows_smem<T, W>(const LevelDev<T>&);                                                                \
-  template bool launch_gs_groups<T, W>(const LevelDev<T>&, int, bool, int, cudaStream_t, bool);                          \
+  template bool launch_gs_groups<T, W>(const LevelDev<T>&, int, bool, int, cudaStream_t);                                \
   template bool bs_dense_on_clusters<T, W>(const BoundaryDev<T>&, int, int);                                              \
   template void launch_residual<T, W>(const ColourRun*, int, const T*, int, const int*, const int*, const T*, const int*, \
                                       int, const T*, const T*, T*, int, cudaStream_t, bool);                             \

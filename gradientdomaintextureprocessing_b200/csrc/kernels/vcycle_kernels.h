@@ -100,7 +100,6 @@ struct LevelDev {
   T *x = nullptr, *b = nullptr, *r = nullptr;
   const int* groups = nullptr;  // per chart: first run of each colour [4], run counts [4], texel span [2]
   int nGroups = 0, maxGroupDeep = 0, maxGroupSpan = 0;
-  int maxGroupColourRuns = 0;   // most runs of one colour in one chart
   // fused tile smoother (launch_tile_smooth): tiles ordered by tile colour
   // (tiles of colour c are [tileStart[c], tileStart[c + 1])), segments, FP32
   // coefficient blocks
@@ -155,9 +154,8 @@ size_t gs_rows_smem(const LevelDev<T>& D);
 // the same updates in the same order as launch_gs_colour per colour.  False
 // (nothing launched) when a chart's span does not fit kGroupSmemMax.
 constexpr size_t kGroupSmemMax = 200 * 1024;
-// rhsEarly: the previous launch does not write the level's right-hand side
 template <typename T, int W>
-bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s, bool rhsEarly = false);
+bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s);
 // The same sweeps, same bits, on a cluster of CTAs per chart (chart_cluster.cu).
 // zeroStart: x = 0 on entry.  gs_cluster_available: the level has its layout, it
 // fits this device, and KP channels of it fill few enough waves.
@@ -326,14 +324,13 @@ void launch_boundary_triangles(int n, const int* btPtr, const int* btTri, const 
 void launch_gather_cells(int n, const int* idx, const double* src, double* dst, cudaStream_t s);
 
 // Dense FP64 set-up products (kernels/dense_kernels.cu).
-// One task of a batched C = alpha op(A) B + beta C (row-major, offsets in
-// doubles into the A, B and C buffers of the launch; op(A) = A (M x K) or,
-// transA, the transpose of A stored K x M); pad: in an elimination step's tasks the
-// matrix's index in the batch.
+// One task of a batched C = op(A) B (row-major, offsets in doubles into the A, B and C
+// buffers of the launch; op(A) = A (M x K) or, transA, the transpose of A stored
+// K x M), or of an elimination step's C -= A B with A 64 wide (lda and transA unused),
+// `matrix` then being the matrix's index in the batch.
 struct GemmTask {
   long long a, b, c;
-  int M, N, K, lda, ldb, ldc, transA, pad;
-  double alpha, beta;
+  int M, N, K, lda, ldb, ldc, transA, matrix;
 };
 void launch_gemm_batch(const GemmTask* dTasks, int nTasks, int maxM, int maxN, const double* A, const double* B, double* C,
                        cudaStream_t s);
