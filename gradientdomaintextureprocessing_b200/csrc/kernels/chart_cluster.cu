@@ -325,7 +325,7 @@ int cluster_ready() {
   });
 }
 
-// Most CTAs of one launch with several channel groups, each of which loads the
+// Most CTAs per SM of one launch with several channel groups, each of which loads the
 // coefficients again, or with FP64 charts of more than one CTA: beyond a few waves the
 // colour passes keep up (64 right-hand sides at 1024^2, level 1: 92 us against 80; 256
 // charts of a 1024^2 atlas in FP64 270 against 261).  FP32 values of up to 4 channels and
@@ -333,7 +333,7 @@ int cluster_ready() {
 // charts 72 us with clusters, 143 with a block per chart (3 channels; FP64 178 and 247), in
 // 576 charts 89 against 134 with the row launches, in 256 106 against 132.  Per refinement
 // step of 3 channels: 1024 charts 2853 -> 2740 us, 576 1629 -> 1558, 256 806 -> 756.
-constexpr int kClusterMaxCtas = 4 * 148;
+constexpr int kClusterMaxCtasPerSm = 4;
 
 template <typename T, int W, int MAXT, int MINB, bool CREG, bool BREG>
 bool cluster_fits(const LevelDev<T>& D) {
@@ -373,7 +373,7 @@ template <typename T, int W>
 bool gs_cluster_available(const LevelDev<T>& D, int KP) {
   if (D.clusterThreads == 0) return false;
   const bool limited = KP / W > 1 || (sizeof(T) == 8 && D.clusterSize > 1);
-  if (limited && (long long)D.nClusterParts * (KP / W) > kClusterMaxCtas) return false;
+  if (limited && (long long)D.nClusterParts * (KP / W) > (long long)kClusterMaxCtasPerSm * device_sms()) return false;
   if constexpr (std::is_same<T, float>::value)
     return cluster_fits<T, W, 320, 2, true, false>(D) || cluster_fits<T, W, 512, 1, true, true>(D) || large_in_one_wave<T, W>(D, KP);
   else

@@ -1608,6 +1608,22 @@ static inline int nblk(long long threads) { return int((threads + 255) / 256); }
 static bool g_programmatic = true;
 void set_programmatic_launch(bool on) { g_programmatic = on; }
 bool programmatic_launch() { return g_programmatic; }
+int device_sms() {
+  static std::atomic<int> slots[kMaxDevices];
+  static const bool init = [] {
+    for (auto& a : slots) a.store(kUnset);
+    return true;
+  }();
+  (void)init;
+  return per_device_once(slots, [] {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return sms;
+  });
+}
 
 // Every V-cycle kernel is launched with programmatic stream serialization:
 // inside a captured graph consecutive kernels get programmatic edges, so a
@@ -1895,9 +1911,9 @@ void launch_coarse_solve(int n, const double* ainv, const double* scale, const T
     if (G % 4 == 0) return go(k_coarse_solve<T, W, 4, 4, 1>, 4, 4);
     if (G % 2 == 0) return go(k_coarse_solve<T, W, 2, 2, 4>, 2, 2);
   }
-  constexpr int kWave = 2 * 148;
-  if (n <= 2 * kWave) return go(k_coarse_solve<T, W, 1, 1, 4>, 1, 1);
-  if (n <= 4 * kWave) return go(k_coarse_solve<T, W, 2, 1, 4>, 2, 1);
+  const int wave = 2 * device_sms();
+  if (n <= 2 * wave) return go(k_coarse_solve<T, W, 1, 1, 4>, 1, 1);
+  if (n <= 4 * wave) return go(k_coarse_solve<T, W, 2, 1, 4>, 2, 1);
   go(k_coarse_solve<T, W, 4, 1, 4>, 4, 1);
 }
 
@@ -1907,19 +1923,8 @@ static inline int raw_groups(int K) { int G = 1; while (4 * G < K) G *= 2; retur
 // device (its partial sums are added in block order, so one device always gives
 // the same bits), at most kRawMaxBlocks.
 static int raw_blocks() {
-  static std::atomic<int> slots[kMaxDevices];
-  static const bool init = [] {
-    for (auto& a : slots) a.store(kUnset);
-    return true;
-  }();
-  (void)init;
-  return per_device_once(slots, [] {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        sms <= 0)
-      return kRawMaxBlocks;
-    return std::min(kRawMaxBlocks, 8 * sms);
-  });
+  const int sms = device_sms();
+  return sms > 0 ? std::min(kRawMaxBlocks, 8 * sms) : kRawMaxBlocks;
 }
 // The 2K sums of a launch of `blocks` blocks; scalar: true when the reduction
 // evaluated it too (it holds every sum in one block)
@@ -2023,8 +2028,8 @@ template <typename T>
 void launch_add_correction(double* x, T* e, long long n, int K, int KP, cudaStream_t s, const int* frozen) {
   const long long total = n * K;
   const int small = total <= 0xffffffffLL ? 1 : 0;
-  // one value per thread up to two waves of threads (148 SMs of 2048)
-  if (total <= 2 * 148 * 2048LL) launch(k_add_correction<T, 1>, dim3(nblk(total)), s, x, e, n, K, KP, frozen, small);
+  // one value per thread up to two waves of threads (2048 an SM)
+  if (total <= 2 * 2048LL * device_sms()) launch(k_add_correction<T, 1>, dim3(nblk(total)), s, x, e, n, K, KP, frozen, small);
   else launch(k_add_correction<T, 4>, dim3(nblk((total + 3) / 4)), s, x, e, n, K, KP, frozen, small);
 }
 

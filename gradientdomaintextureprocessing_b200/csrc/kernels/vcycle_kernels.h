@@ -309,6 +309,8 @@ int per_device_once(std::atomic<int> (&slots)[kMaxDevices], F compute) {
   }
   return v;
 }
+// SMs of the current device (0: no answer)
+int device_sms();
 // Programmatic dependent launch of the V-cycle kernels (process-wide, default on)
 void set_programmatic_launch(bool on);
 bool programmatic_launch();

@@ -1125,8 +1125,8 @@ bool DeviceSystem::build_multigrid(Multigrid<T>& mg, int KP) {
         B.inv = static_cast<T*>(A.alloc(std::max<size_t>(1, size_t(off[bs.nSub])) * sizeof(T)));
       }
       // blocks per row group: enough chunks for one wave of bsBlocksPerSm
-      // resident blocks on each of the 148 SMs, each warp still taking >= 4 j steps
-      const int target = knobs.bsBlocksPerSm * 148;
+      // resident blocks on each SM, each warp still taking >= 4 j steps
+      const int target = knobs.bsBlocksPerSm * std::max(1, dev::device_sms());
       auto chunks_for = [target](int tasks, int m, int minChunks) {
         int c = (target + std::max(1, tasks) - 1) / std::max(1, tasks);
         c = std::min(c, std::max(1, m / 32));
