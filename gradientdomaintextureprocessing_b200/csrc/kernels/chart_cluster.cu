@@ -85,23 +85,13 @@ __device__ __forceinline__ PairPos load_pair(const ClusterItem& it, int lo, int 
   return p;
 }
 
-// Asynchronous copies into shared memory (each at its own size, so aligned as the
-// value is); a thread's copies are complete after async_wait()
-template <int BYTES>
-__device__ __forceinline__ void async_copy(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
-}
+// an asynchronous copy of a texel's values
 template <typename T, int W>
 __device__ __forceinline__ void async_vec(Vec<T, W>* dst, const T* src) {
   constexpr int kBytes = sizeof(Vec<T, W>), kStep = kBytes < 16 ? kBytes : 16;
 #pragma unroll
-  for (int b = 0; b < kBytes; b += kStep) async_copy<kStep>(reinterpret_cast<char*>(dst) + b, reinterpret_cast<const char*>(src) + b);
+  for (int b = 0; b < kBytes; b += kStep) copy_async<kStep>(reinterpret_cast<char*>(dst) + b, reinterpret_cast<const char*>(src) + b);
 }
-__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename T, int W>
 struct Slab {
@@ -239,8 +229,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_gs_cluster(const ClusterPart* __
           if (pos[h].flags & 1) wr[h][k] = cA[(long long)k * planeStride];
           if (pos[h].flags & 2) wr[h][9 + k] = cB[(long long)k * planeStride];
         } else {
-          if (pos[h].flags & 1) async_copy<sizeof(T)>(&sw[(18 * h + k) * nt + tid], cA + (long long)k * planeStride);
-          if (pos[h].flags & 2) async_copy<sizeof(T)>(&sw[(18 * h + 9 + k) * nt + tid], cB + (long long)k * planeStride);
+          if (pos[h].flags & 1) copy_async<sizeof(T)>(&sw[(18 * h + k) * nt + tid], cA + (long long)k * planeStride);
+          if (pos[h].flags & 2) copy_async<sizeof(T)>(&sw[(18 * h + 9 + k) * nt + tid], cB + (long long)k * planeStride);
         }
       }
       if (rhsEarly) load_rhs(h);
@@ -260,7 +250,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_gs_cluster(const ClusterPart* __
     load_rhs(0);
     load_rhs(1);
   }
-  async_wait();  // this thread's copies; the barrier then orders every thread's
+  copies_wait_all();  // this thread's copies; the barrier then orders every thread's
   if (C > 1) cluster.sync(); else __syncthreads();
 
   auto half = [&](auto hc, bool push) {

@@ -31,6 +31,7 @@
 #include <string>
 #include <vector>
 
+#include "vcycle.cuh"
 #include "vcycle_kernels.h"
 
 namespace gdtp {
@@ -141,30 +142,19 @@ __device__ __forceinline__ void tile_product(double (&acc)[8][4], const double* 
   }
 }
 
-// asynchronous copies to shared memory, zeros where !in
-__device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void copy16(double* dst, const double* src, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // queue the inner part [K0, K0 + 32) of the tiles: A rows [0, rows) (64 wide, 16-byte
 // aligned) and B rows below K, columns [0, cols) (leading dimension ldb)
 __device__ __forceinline__ void queue_half(double* As, double* Bs, const double* A, int rows, const double* B, int ldb, int K, int cols, int K0) {
 #pragma unroll
   for (int q = 0; q < 8; q++) {
     const int e = threadIdx.x + kEThreads * q, r = e >> 4, c = K0 + 2 * (e & 15);
-    copy16(As + r * kPitchA + c, r < rows ? A + r * kPB + c : A, r < rows);
+    copy_async_or_zero<16>(As + r * kPitchA + c, r < rows ? A + r * kPB + c : A, r < rows);
   }
 #pragma unroll
   for (int q = 0; q < 16; q++) {
     const int e = threadIdx.x + kEThreads * q, r = K0 + (e >> 6), c = e & 63;
     const bool in = r < K && c < cols;
-    copy8(Bs + r * kPB + c, in ? B + (long long)r * ldb + c : B, in);
+    copy_async_or_zero<8>(Bs + r * kPB + c, in ? B + (long long)r * ldb + c : B, in);
   }
   copies_commit();
 }

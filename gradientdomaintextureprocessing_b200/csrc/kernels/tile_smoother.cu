@@ -100,20 +100,6 @@ __device__ __forceinline__ void pass(float* xs, const float* bs, const float (&c
   __syncthreads();
 }
 
-// global -> shared copies that bypass registers (completion: cp_async_wait_all)
-template <int KP>
-__device__ __forceinline__ void cp_async(float* smem, const float* gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  if constexpr (KP == 4)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
 // ring-and-tile elements per thread (a tile with its ring has at most
 // (kTileW + 2) x (kTileH + 2) active texels)
 constexpr int kElemsPerThread = ((kTileW + 2) * (kTileH + 2) + kPerColour - 1) / kPerColour;
@@ -224,7 +210,7 @@ __global__ void __launch_bounds__(kPerColour, 3) k_tile_smooth(TileRound a, floa
         so = (sub * kSub + (V >> 1) * kSubW + (U >> 1)) * KP;
         if (u >= 1 && u <= kTileW && r >= 1 && r <= kTileH) {
           slot = sub * kPerColour + ((V >> 1) - 1) * kHalfW + ((U >> 1) - 1);
-          cp_async<KP>(bs + slot * KP, a.rhs + (long long)g * KP);
+          copy_async<4 * KP>(bs + slot * KP, a.rhs + (long long)g * KP);
         }
       }
       gE[m] = g;
@@ -254,7 +240,7 @@ __global__ void __launch_bounds__(kPerColour, 3) k_tile_smooth(TileRound a, floa
       for (int m = 0; m < kElemsPerThread; m++)
         if (gE[m] >= 0) tstore<KP>(xs + sE[m], tload_l2<KP>(x + (long long)gE[m] * KP));
     }
-    cp_async_wait_all();
+    copies_wait_all();
     __syncthreads();
     for (int sw = 0; sw < a.sweeps; sw++) {
       if (a.reverse) {

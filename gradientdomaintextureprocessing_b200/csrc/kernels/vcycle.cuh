@@ -80,5 +80,33 @@ __device__ __forceinline__ void vstore(T* p, const Vec<T, W>& v) {
   *reinterpret_cast<Vec<T, W>*>(p) = v;
 }
 
+#ifdef __CUDACC__  // (host files include the types above)
+// Asynchronous copies of BYTES (both sides aligned to it) from global into shared
+// memory, past the registers: 16 bytes through L2 only unless L1, smaller ones always
+// through L1.  copy_async_or_zero writes zeros where !in (src is not read then).  A
+// thread's copies are complete, for itself, after copies_wait.
+template <int BYTES, bool L1 = BYTES != 16>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (L1)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+  else
+    asm volatile("cp.async.cg.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void copy_async_or_zero(void* dst, const void* src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(in ? BYTES : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the N last committed groups
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void copies_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+#endif
+
 }  // namespace dev
 }  // namespace gdtp

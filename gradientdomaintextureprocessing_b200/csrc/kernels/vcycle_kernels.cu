@@ -1000,12 +1000,10 @@ __global__ void __launch_bounds__(256, Q == 1 ? 2 : 1) k_coarse_solve(int n, con
       for (int u = 0; u < kPieces; u++) {
         const int e = lane + 32 * u, row = e / kPieces, piece = e % kPieces;
         if (j + row < j1)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
-                           (unsigned)__cvta_generic_to_shared(&stage[warp][buf][row * kPitch + piece * 16])),
-                       "l"(reinterpret_cast<const char*>(rhs + (long long)(j + row) * KP + c0) + piece * 16)
-                       : "memory");
+          copy_async<16, true>(&stage[warp][buf][row * kPitch + piece * 16],
+                               reinterpret_cast<const char*>(rhs + (long long)(j + row) * KP + c0) + piece * 16);
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      copies_commit();
     };
     double wn[R], scn = 0;
     auto fetch = [&](int j) {
@@ -1025,9 +1023,9 @@ __global__ void __launch_bounds__(256, Q == 1 ? 2 : 1) k_coarse_solve(int n, con
       if (jb + 32 < j1) {
         queue(jb + 32, buf ^ 1);
         fetch(j + 32);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        copies_wait<1>();
       } else {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        copies_wait<0>();
       }
       __syncwarp();
       if (j < j1)
