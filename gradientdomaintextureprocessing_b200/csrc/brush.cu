@@ -56,9 +56,11 @@ struct BrushRows {  // per channel the boundary x cells matrix
 // boundary texels, 8 lanes per row and channel (a chain of loads that the deep
 // texels hide): out = row times m.  The others a deep texel per thread: out = c0
 // m[prev i] + c1 m[prev i+1] + c2 m[next i] + c3 m[next i+1], its 4 K coefficients
-// read as pairs.  The bytes (140 per deep texel at K = 3) take 8 us at 1024^2; as a
-// launch for the deep values, with a division per value, and a launch per channel of
-// one thread per row a call took 34.8 us, now 18.3 with the host's share.
+// read as pairs.  The bytes (140 per deep texel at K = 3) take 8 us at 1024^2 from HBM.
+// Between events on the stream a stroke takes 22.6 us when its buffers have left L2, 14.5
+// when the last stroke left them there.  Strokes one after another (so from L2), with the
+// host's share: 34.8 us as a launch for the deep values, with a division per value, and a
+// launch per channel of one thread per row, now 18.3.
 template <int K>
 __global__ void __launch_bounds__(256) k_brush_apply(int rowBlocks, int nB, const int* __restrict__ bGlobal, BrushRows rows, int nDeep,
                                                      const int* __restrict__ deepGlobal, const int4* __restrict__ cells,

@@ -1,10 +1,10 @@
 // Chart smoother on a thread-block cluster: every sweep of one smoothing step
 // (IterativeSolvers.inl:174-395 restated as 4-colour Gauss-Seidel) in one launch,
-// a cluster of C CTAs per chart.
+// a chart on the CTAs of a cluster (charts that need few of them share one).
 //
 // Deep texels of different charts never neighbour each other and the sweeps do
 // not change boundary texels, so a chart is independent of the others.  The
-// chart's rows are dealt to the cluster's CTAs (contiguous rows, balanced by
+// chart's rows are dealt to its CTAs (contiguous rows, balanced by
 // texels); a CTA keeps its rows' x, with the row above and the row below, in
 // shared memory (the slab), and its coefficients and right-hand side in
 // registers or shared memory, for all sweeps.  One half sweep updates the rows of
@@ -23,7 +23,7 @@
 // passes', bit for bit.
 //
 // What bounds it: on the levels below the finest, and on whole problems up to about
-// 512^2, a sweep is a chain of latencies, not bytes.  As two row launches it took
+// 1024^2, a sweep is a chain of latencies, not bytes.  As two row launches it took
 // 5.5 us (launch, x through L2, two block barriers, each time); a sweep more in here
 // takes 1.9 us (256^2 torus, 8 CTAs a chart), and a smoothing step of 3 sweeps 12
 // instead of 22 us.  Per refinement step: 256^2 torus 187 -> 134 us, 1024^2 genus-2

@@ -116,7 +116,8 @@ struct LevelDev {
   const int* rowLineOf[2] = {nullptr, nullptr};
   int nRowBins[2] = {0, 0};
   int rowBlock = 0, rowSlots = 0;
-  // chart smoother on clusters (launch_gs_cluster): clusterSize parts per chart
+  // chart smoother on clusters (launch_gs_cluster): clusters of clusterSize parts (CTAs),
+  // a chart on one or more parts of one cluster
   const ClusterPart* clusterParts = nullptr;
   const ClusterItem* clusterItems = nullptr;
   int nClusterParts = 0, clusterSize = 0, clusterThreads = 0, clusterSlab = 0;
@@ -156,9 +157,9 @@ size_t gs_rows_smem(const LevelDev<T>& D);
 constexpr size_t kGroupSmemMax = 200 * 1024;
 template <typename T, int W>
 bool launch_gs_groups(const LevelDev<T>& D, int sweeps, bool reverse, int KP, cudaStream_t s);
-// The same sweeps, same bits, on a cluster of CTAs per chart (chart_cluster.cu).
-// zeroStart: x = 0 on entry.  gs_cluster_available: the level has its layout, it
-// fits this device, and KP channels of it fill few enough waves.
+// The same sweeps, same bits, a chart on the CTAs of a cluster (chart_cluster.cu).
+// zeroStart: x = 0 on entry.  gs_cluster_available: the level has its layout, it fits
+// this device, and, where that is limited, KP channels of it fill few enough waves.
 template <typename T, int W>
 bool gs_cluster_available(const LevelDev<T>& D, int KP);
 template <typename T, int W>

@@ -79,8 +79,8 @@ struct RowBins {
 };
 bool build_row_bins(const GridLevel& L, const DeepRuns& R, RowBins& out);
 
-// Rows of every chart dealt to the CTAs of its cluster (dev::launch_gs_cluster):
-// `size` parts per chart; threads: the most items of one row parity in a part, in
+// Rows of every chart dealt to CTAs of one cluster (dev::launch_gs_cluster): clusters of
+// `size` parts (CTAs), which charts may share; threads: the most items of one row parity in a part, in
 // warps; slab: the most texels a part touches
 struct ChartClusters {
   std::vector<dev::ClusterPart> parts;
@@ -327,12 +327,12 @@ class DeviceSystem {
   bool raw_apply_dev(const RawOperator& op, const double* b, const double* x, double* out, int k, int mode, cudaStream_t s,
                      double* sumsHost);
   bool check(cudaError_t e, const char* what);
+  template <typename T>
+  void append_routes(const Multigrid<T>& mg, std::vector<double>& v) const;
   // host vectors of a V-cycle or a smoothing step (tight n x k) to the level-0
   // iterate and right-hand side (padded), and the iterate back: padded and stripped
   // on the device (value by value on the host a V-cycle on 640 x 480 RGB vectors took
-  // 21.0 ms, now 0.82)
-  template <typename T>
-  void append_routes(const Multigrid<T>& mg, std::vector<double>& v) const;
+  // 21.0 ms, now 0.88)
   template <typename T>
   bool vectors_in(Multigrid<T>& mg, const T* x, const T* rhs, int k);
   template <typename T>
