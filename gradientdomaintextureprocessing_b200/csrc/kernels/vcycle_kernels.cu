@@ -1332,10 +1332,10 @@ __global__ void __launch_bounds__(256) k_raw_operator(const ColourRun* __restric
 //    / 591; one, 256^2 torus 85.5 / 83.8, 640 x 480 183.8 / 185.6, 16 x 16 charts 467 / 452 (a
 //    thread per row also where there are few: genus-2 of 15 k rows 134.2 / 135.5, of 29 k
 //    197 / 200.8).
-// What bounds it at 2048^2 (77 us for 203 MB): half the warps (64 registers), each a
-// long-scoreboard wait of 10.6 of 17.9 cycles per issue, and 58 % of the first-level
-// cache's cycles; a lane per value instead of per texel (consecutive addresses, but
-// the coefficients read for every channel) took 85 us.
+// What bounds it at 2048^2 (65 us for 203 MB; read when every row ran on 8 lanes, 77 us):
+// half the warps (64 registers), each a long-scoreboard wait of 10.6 of 17.9 cycles per
+// issue, and 58 % of the first-level cache's cycles; a lane per value instead of per texel
+// (consecutive addresses, but the coefficients read for every channel) took 85 us.
 template <int KT, bool FEW>
 __global__ void __launch_bounds__(256, 4) k_raw_few(const ColourRun* __restrict__ runs, int nRuns, const double* __restrict__ coef,
                                                     int planeStride, const int* __restrict__ bPtr, const int* __restrict__ bCol,
